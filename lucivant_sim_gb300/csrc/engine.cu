@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "jit.cuh"
 #include "kernels.cuh"
+#include "lower.cuh"
 #include "program.cuh"
 #include "tile.cuh"
 
@@ -449,10 +450,16 @@ Plan plan_ops(const lsg_op* ops, int nops, int nbits, int K, int L, const int* p
     return plan;
 }
 
-// Widest register block: 16 elements per thread for 4- and 8-byte elements, 8 complex128.
-int block_bits_for(int precision) {
-    const int top = lsg_elem_bytes(precision) == 16 ? 3 : 4;
+// Widest register block: 16 elements per thread. A complex register of 2^10 amplitudes or fewer is
+// one tile on one SM: narrower blocks keep more of its lanes at work (8 qubits, complex128, 4
+// layers: 82 us in 4-bit blocks, 56 in 3-bit, 36 in 2-bit ones; 10 qubits: 105, 69, 75; 11: 114,
+// 130, 138). Trajectory segments (not lowered) of complex128 take 8 amplitudes per thread, as many
+// groups as the kernel has threads.
+int block_bits_for(int precision, int nbits, bool lowered) {
+    const int top = 4;
     int u = top;
+    if (!lsg_precision_real(precision)) u = std::max(2, std::min(top, nbits - 7));
+    if (precision == LSG_C128 && !lowered) u = std::min(u, 3);
     if (const char* env = getenv("LSG_BLOCK_BITS")) u = atoi(env);
     return std::max(0, std::min(u, top));
 }
@@ -572,6 +579,7 @@ struct lsg_program_s {
     size_t smem = 0;
     int K = 0;
     std::vector<cudaEvent_t> events;
+    std::vector<char> swz;  // per pass: how the interpreter runs it (tile.cuh kPlain, kSwz, kRounds, kMixed)
     std::shared_ptr<lsg::JitPasses> jit;  // specialized passes, when the program could be specialized
     // runs from a basis state: the passes restricted to tiles that can be nonzero (uploaded after
     // the block descriptors, for the basis index `basis_index`)
@@ -586,6 +594,7 @@ struct lsg_program_s {
     // plan without planning again (lsg_program_set_data)
     std::vector<lsg_op> src_ops;
     lsg::Plan raw_plan;
+    lsg::Plan core_plan;  // the plan with its operators' codes, before blocks were fused or lowered
     // the template's CUDA graph: set basis state + every pass, captured for one register and index
     cudaGraphExec_t graph = nullptr;
     uint64_t graph_uid = 0;
@@ -647,22 +656,45 @@ static int launch_passes(lsg_program_s* p, lsg_state_s* s, cudaEvent_t* marks, c
     }
     if (pipe) {
         // each pass gets the shared memory its own operators need: short passes fit more CTAs per SM
-        const void* kern = PassKernels<T>::pipe();
-        LSG_CHECK(allow_smem(kern));
+        const bool swizzle = swizzle_enabled();
+        LSG_CHECK(allow_smem(PassKernels<T>::pipe()));
+        for (int mode : {kSwz, kRounds, kMixed}) LSG_CHECK(allow_smem(PassKernels<T>::swz(mode)));
         size_t last_smem = 0;
+        const void* last_kern = nullptr;
         int64_t grid = 1;
+        std::vector<std::pair<uint32_t, Tmap>> maps;
         for (size_t i = 0; i < p->plan.passes.size(); ++i) {
             const PassDesc& pd = p->plan.passes[i];
             const int64_t total = tpm[i] * s->batch;
-            const size_t smem = 2 * tile_bytes + (size_t)pd.nops * (sizeof(TileOp) + 16) + (size_t)pd.nblocks * sizeof(BlockDesc);
-            if (smem != last_smem) {
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPipeThreads, smem);
+            const bool swz = swizzle && p->swz[i];
+            const int mode = swz ? p->swz[i] : kPlain;
+            const bool rounds = mode == kRounds;
+            const void* kern = swz ? PassKernels<T>::swz(mode) : PassKernels<T>::pipe();
+            const size_t smem = 2 * tile_bytes + (swz ? 1024 : 0) + (size_t)pd.nops * (sizeof(TileOp) + 16) +
+                                (size_t)pd.nblocks * sizeof(BlockDesc) +
+                                (rounds ? (size_t)pd.rounds * 16 * round_words<T>() : 0);
+            if (smem != last_smem || kern != last_kern) {
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, rounds ? compute_threads<kRounds>() + 32 : kPipeThreads, smem);
                 last_smem = smem;
+                last_kern = kern;
             }
             grid = std::max<int64_t>(1, std::min<int64_t>(total, (int64_t)sms * std::max(per_sm, 1)));
             if (marks) LSG_CUDA(cudaEventRecord(marks[i], s->stream));
-            PassKernels<T>::launch_pipe((unsigned)grid, smem, s->stream, state, s->elems, pd_dev + i, ops_dev, blk_dev,
-                                        pool_dev, tpm[i], total, status, ctx);
+            if (!swz) {
+                PassKernels<T>::launch_pipe((unsigned)grid, smem, s->stream, state, s->elems, pd_dev + i, ops_dev, blk_dev,
+                                            pool_dev, tpm[i], total, status, ctx);
+                continue;
+            }
+            const uint32_t key = tile_map_key(pd, sizeof(T));
+            auto map = std::find_if(maps.begin(), maps.end(), [&](const auto& m) { return m.first == key; });
+            if (map == maps.end()) {
+                Tmap m{};
+                LSG_CHECK(encode_tile_map(state, s->elems * s->batch * (int64_t)sizeof(T), sizeof(T), pd, &m));
+                maps.emplace_back(key, m);
+                map = maps.end() - 1;
+            }
+            PassKernels<T>::launch_swz(mode, (unsigned)grid, smem, s->stream, state, s->elems, pd_dev + i, ops_dev, blk_dev,
+                                       pool_dev, tpm[i], total, status, ctx, map->second);
         }
     } else {
         const void* kern = PassKernels<T>::pass();
@@ -716,6 +748,102 @@ static std::vector<PassDesc> basis_passes(const Plan& plan, int nbits, int preci
         }
     }
     return out;
+}
+
+// ---- register blocks on swizzled tiles
+
+// The block's GF(2) address maps (program.cuh BlockDesc). The 128-byte swizzle stores tile element x
+// at S(x) = x ^ (((x >> row) & 7) << unit), linear over GF(2), so the byte address of a group's
+// element is a XOR of one constant per index bit. Two choices are free: which of the group
+// index's bits each of a warp's lanes drives, and the order of the block's elements. The lanes of
+// one shared-memory phase (128 bytes) take tile bits whose addresses fall into different banks
+// (independent over GF(2) within the 128 bytes) as far as the block leaves them; renames at the
+// block's ends permute its elements, so they are folded into the load and store maps.
+static int block_layout(const PassDesc& pd, BlockDesc& b, const TileOp* ops, size_t eb) {
+    int lg = 0;
+    while (((size_t)1 << lg) < eb) ++lg;
+    const int unit = 4 - lg, row = 7 - lg, U = b.u, K = pd.K;
+    auto bytes = [&](uint32_t x) { return (x ^ (((x >> row) & 7u) << unit)) << lg; };
+    auto bit = [&](int P) { return 1u << (U - 1 - P); };
+    auto rename = [&](int code, uint32_t e) -> uint32_t {
+        if (code < kT_CX) return e ^ bit(code - kT_X1);
+        if (code < kT_SWAP) return (e & bit((code - kT_CX) / 4)) ? e ^ bit((code - kT_CX) % 4) : e;
+        const uint32_t x = bit((code - kT_SWAP) / 4), y = bit((code - kT_SWAP) % 4);
+        return ((e & x) != 0) != ((e & y) != 0) ? e ^ x ^ y : e;
+    };
+    // (a rename under a branch's predicate is a member's own: executed)
+    auto is_rename = [&](int o) { return ops[o].pred == 0 && ops[o].tmpl >= kT_X1 && ops[o].tmpl < kT_SWAP + 16; };
+    int lead = 0, end = b.nops;
+    while (lead < end && is_rename(lead)) ++lead;
+    while (end > lead && is_rename(end - 1)) --end;
+    b.lead = (short)lead;
+    b.nexec = (short)(end - lead);
+    auto offset = [&](uint32_t e) {
+        uint32_t x = 0;
+        for (int j = 0; j < U; ++j)
+            if (e & bit(j)) x ^= bytes(1u << b.bits[j]);
+        return x;
+    };
+    auto from = [&](uint32_t e) {  // a rename's new element e is the old rename(e): the last one acts first
+        for (int o = lead - 1; o >= 0; --o) e = rename(ops[o].tmpl, e);
+        return e;
+    };
+    auto to = [&](uint32_t e) {
+        for (int o = end; o < b.nops; ++o) e = rename(ops[o].tmpl, e);
+        return e;
+    };
+    b.lconst = (unsigned short)offset(from(0));
+    b.sconst = (unsigned short)offset(to(0));
+    for (int j = 0; j < 4; ++j) {
+        b.lob[j] = j < U ? (unsigned short)(offset(from(bit(j))) ^ b.lconst) : 0;
+        b.sob[j] = j < U ? (unsigned short)(offset(to(bit(j))) ^ b.sconst) : 0;
+    }
+    // runs of `vec` elements per access: the last positions' steps are the run, nothing else moves inside it
+    auto width = [&](const unsigned short* ob, unsigned short c) {
+        for (int vec = (int)std::min<size_t>((size_t)b.vec, 16 / eb); vec > 1; vec /= 2) {
+            const int k = vec == 4 ? 2 : 1;
+            const uint32_t inside = (uint32_t)(vec - 1) * (uint32_t)eb;
+            bool ok = U >= k && !(c & inside);
+            for (int j = 0; j < U && ok; ++j)
+                ok = j >= U - k ? ob[j] == eb << (U - 1 - j) : !(ob[j] & inside);
+            if (ok) return vec;
+        }
+        return 1;
+    };
+    b.lvec = (short)width(b.lob, b.lconst);
+    b.svec = (short)width(b.sob, b.sconst);
+    // lanes: bits of the group index in order; the first ones reach different banks of a phase
+    int access = 0;
+    while ((1 << access) < (int)(b.lvec * (int)eb)) ++access;
+    std::vector<int> rest, order;
+    for (int t = 0; t < K; ++t)
+        if (std::find(b.bits, b.bits + U, t) == b.bits + U) rest.push_back(t);
+    std::vector<uint32_t> span;  // reduced projections chosen so far
+    for (int t : rest) {
+        if ((int)span.size() == 7 - access) break;
+        uint32_t v = (bytes(1u << t) & 127u) >> access;
+        for (uint32_t s : span) v = std::min(v, v ^ s);
+        if (!v) continue;
+        span.push_back(v);
+        order.push_back(t);
+    }
+    for (int t : rest)
+        if (std::find(order.begin(), order.end(), t) == order.end()) order.push_back(t);
+    std::fill(b.gb, b.gb + 16, (unsigned short)0);
+    if ((int)order.size() > 16) return fail(LSG_E_ARG, "internal planning error: a tile of 2^%d elements", K);
+    for (size_t i = 0; i < order.size(); ++i) b.gb[i] = (unsigned short)bytes(1u << order[i]);
+    // the maps reach every element of the tile once: K independent addresses below the tile's size
+    for (const unsigned short* ob : {b.lob, b.sob}) {
+        std::vector<uint32_t> basis;
+        for (int i = 0; i < K; ++i) {
+            uint32_t v = i < U ? ob[i] : b.gb[i - U];
+            if (v >= (uint32_t)(eb << K) || (v & (eb - 1))) return fail(LSG_E_ARG, "internal planning error: block address");
+            for (uint32_t s : basis) v = std::min(v, v ^ s);
+            if (!v) return fail(LSG_E_ARG, "internal planning error: block addresses collide");
+            basis.push_back(v);
+        }
+    }
+    return LSG_OK;
 }
 
 // ---- whole-block fusion (complex registers): a register block whose operators cost more than one
@@ -798,7 +926,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     p->K = tile_bits_for(nbits, precision);
     const int L = std::min(p->K, low_bits_for(nbits, precision));
     if (nops > 0) {
-        p->plan = preplanned ? *preplanned : plan_ops(ops, nops, nbits, p->K, L, pred, draw, count, block_bits_for(precision));
+        p->plan = preplanned ? *preplanned : plan_ops(ops, nops, nbits, p->K, L, pred, draw, count, block_bits_for(precision, nbits, !pred && !draw && !count));
         if (upload && !pred && !draw && !count) {
             p->src_ops.assign(ops, ops + nops);
             p->raw_plan = p->plan;
@@ -847,6 +975,21 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
             else if (src[0] == 0 && src[1] == 2 && src[2] == 1 && src[3] == 3) t.tmpl = kT_SWAP + 4 * P0 + P1;
         }
     }
+    if (!pred && !draw && !count) p->core_plan = p->plan;
+    // Complex programs: outer factors of one-bit operators move on to the next ones, so that blocks
+    // lower to rounds (lower.cu). Trajectory segments keep their operators: each has its own
+    // predicate and draws.
+    const char* fuse_env = getenv("LSG_FUSE_BLOCKS");
+    const bool fuse = !lsg_precision_real(precision) && !(fuse_env && fuse_env[0] == '0');
+    const bool rounds = fuse && !pred && !draw && !count;
+    std::vector<double> grown;
+    std::vector<char> moved;
+    if (rounds && nops > 0) {
+        grown.assign(pool, pool + 2 * pool_entries);
+        moved = move_outer_factors(p->plan, batch, grown);
+        pool = grown.data();
+        pool_entries = (int64_t)grown.size() / 2;
+    }
     // Register-block operator data, copied once here into an extension of the pool: diagonals
     // re-indexed in block order (the kernel multiplies v[e] by m[e] with no index arithmetic), and
     // dense matrices, diagonals and mixture matrices placed on 16-byte boundaries (the kernel reads
@@ -861,12 +1004,65 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
             ext.push_back(0.0);
         }
     };
-    const char* fuse_env = getenv("LSG_FUSE_BLOCKS");
-    const bool fuse = !lsg_precision_real(precision) && !(fuse_env && fuse_env[0] == '0');
     for (const PassDesc& pd : p->plan.passes)
         for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks; ++bi) {
             BlockDesc& blk = p->plan.blocks[bi];
             if (blk.generic) continue;
+            if (rounds && blk.nops > 1) {
+                const double overhead = precision == LSG_C64 ? 0.5 : 0.1;
+                double cost = 0.0;
+                bool dense = blk.u >= 2;
+                for (int o = blk.first; o < blk.first + blk.nops; ++o) {
+                    const TileOp& t = p->plan.ops[pd.first_op + o];
+                    cost += block_op_cost(t, overhead);
+                    dense = dense && block_fusable_op(t);
+                }
+                if (dense) cost = std::min(cost, 1.1 * ((double)(1 << blk.u) + overhead + (double)(1 << blk.u) / 16.0));
+                LoweredBlock low;
+                if (lower_block(p->plan, pd, blk, moved, batch, pool, overhead, precision == LSG_C64, &low) && low.cost < cost) {
+                    const int D = 1 << blk.u;
+                    std::vector<TileOp> made;
+                    for (const LoweredItem& it : low.items) {
+                        if (it.code == kKeepOp) {
+                            made.push_back(p->plan.ops[it.op]);
+                            made.back().tmpl = it.tmpl;
+                            continue;
+                        }
+                        // complex64 diagonals as (re, re, -im, im): the operands of packed products
+                        const int64_t len = (precision == LSG_C64 ? 2 * D : D) + blk.u;
+                        const int64_t stride = round_up(len);
+                        pad_ext(0);
+                        TileOp f{};
+                        f.kind = LSG_OP_MATRIX;
+                        f.k = blk.u;
+                        for (int i = 0; i < blk.u; ++i) {
+                            f.lb[i] = blk.bits[i];
+                            f.sorted[i] = blk.sorted[i];
+                            f.pos[i] = i;
+                        }
+                        f.data = pool_entries + (int64_t)ext.size() / 2;
+                        f.stride = low.members > 1 ? stride : 0;
+                        f.tmpl = it.code;
+                        f.zmask = it.mask;
+                        for (int64_t b = 0; b < low.members; ++b) {
+                            const size_t end = ext.size() + 2 * (size_t)stride;
+                            for (int e = 0; e < D; ++e) {
+                                const std::complex<double> v = it.diag.empty() ? 1.0 : it.diag[(size_t)(b * D + e)];
+                                if (precision == LSG_C64) ext.insert(ext.end(), {v.real(), v.real(), -v.imag(), v.imag()});
+                                else ext.insert(ext.end(), {v.real(), v.imag()});
+                            }
+                            for (int i = 0; i < blk.u; ++i) {
+                                ext.push_back(it.t.empty() ? 0.0 : it.t[(size_t)(b * blk.u + i)]);
+                                ext.push_back(it.t.empty() ? 0.0 : it.second[(size_t)(b * blk.u + i)]);
+                            }
+                            ext.resize(end, 0.0);
+                        }
+                        made.push_back(f);
+                    }
+                    std::copy(made.begin(), made.end(), p->plan.ops.begin() + pd.first_op + blk.first);
+                    blk.nops = (int)made.size();
+                }
+            }
             if (fuse && blk.u >= 2 && blk.nops > 1) {
                 const int U = blk.u, D = 1 << U;
                 const double overhead = precision == LSG_C64 ? 0.5 : 0.1;
@@ -975,6 +1171,40 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 }
             }
         }
+    {  // which passes move swizzled tiles, and their blocks' address maps
+        const size_t eb = lsg_elem_bytes(precision);
+        p->swz.assign(p->plan.passes.size(), 0);
+        for (size_t i = 0; i < p->plan.passes.size(); ++i) {
+            PassDesc& pd = p->plan.passes[i];
+            bool fits = pass_swizzle_fits(pd, eb, ((int64_t)eb << nbits) * batch) && (eb << pd.K) <= 65536;
+            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks && fits; ++bi)
+                fits = !p->plan.blocks[bi].generic;
+            if (!fits) continue;
+            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks; ++bi) {
+                BlockDesc& b = p->plan.blocks[bi];
+                if (block_layout(pd, b, &p->plan.ops[pd.first_op + b.first], eb) != LSG_OK) {
+                    delete p;
+                    return LSG_E_ARG;
+                }
+            }
+            bool lowered = !lsg_precision_real(precision), any = false;
+            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks; ++bi) {
+                const BlockDesc& b = p->plan.blocks[bi];
+                for (int o = pd.first_op + b.first; o < pd.first_op + b.first + b.nops; ++o) {
+                    const TileOp& t = p->plan.ops[o];
+                    any = any || t.tmpl == kT_ROUND;
+                    lowered = lowered && t.pred == 0 && (t.tmpl == kT_ROUND || (t.tmpl >= kT_X1 && t.tmpl < kT_SWAP + 16));
+                }
+            }
+            p->swz[i] = (char)(lowered ? kRounds : any ? kMixed : kSwz);
+            for (int o = pd.first_op; lowered && o < pd.first_op + pd.nops; ++o) p->plan.ops[o].count = 0;
+            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks && lowered; ++bi) {
+                const BlockDesc& b = p->plan.blocks[bi];
+                for (int o = pd.first_op + b.first; o < pd.first_op + b.first + b.nops; ++o)
+                    if (p->plan.ops[o].tmpl == kT_ROUND) p->plan.ops[o].count = pd.rounds++;
+            }
+        }
+    }
     const int64_t base_entries = pool_entries;  // the caller's pool, then the relocated data
     pool_entries = base_entries + (int64_t)ext.size() / 2;
     size_t max_meta = 0;
@@ -1096,6 +1326,32 @@ void program_destroy(lsg_program_s* p) {
     if (p->graph) cudaGraphExecDestroy(p->graph);
     release(p->dev);
     delete p;
+}
+
+// Put a program made anew from `ops` (its plan choices, its kind of passes) in the place of `p`'s
+// content. The old device memory is released with cudaFree, which waits for runs that still read
+// it; the graph is captured again by the next graph run.
+static int program_remake(lsg_program_s* p, const lsg_op* ops, int32_t nops, const double* pool, int64_t pool_entries) {
+    lsg_program_s* q = nullptr;
+    const PlanChoice keep = t_choice;
+    t_choice = p->choice;
+    const Plan raw = p->raw_plan;
+    int rc = program_build(p->nbits, p->precision, p->batch, ops, nops, pool, pool_entries, nullptr, nullptr, nullptr,
+                           &q, nullptr, true, &raw);
+    if (rc == LSG_OK && p->jit) {
+        const size_t eb = lsg_elem_bytes(p->precision);
+        q->jit = jit_build(q->plan, p->precision, jit_ctas(p->precision),
+                           jit_swizzle_fits(q->plan, eb, ((int64_t)eb << p->nbits) * p->batch), jit_packed(p->precision));
+    }
+    t_choice = keep;
+    LSG_CHECK(rc);
+    std::swap(*p, *q);
+    std::swap(p->events, q->events);
+    if (p->graph) cudaGraphExecDestroy(p->graph);
+    p->graph = nullptr;
+    p->graph_uid = 0;
+    program_destroy(q);
+    return LSG_OK;
 }
 
 static int program_launch(lsg_program_s* p, lsg_state_s* s, cudaEvent_t* marks, const TrajCtx& ctx, bool from_basis) {
@@ -1743,13 +1999,19 @@ int lsg_program_set_data(lsg_program p, lsg_state s, const lsg_op* ops, int32_t 
     auto same_bytes = [](const auto& a, const auto& b) {
         return a.size() == b.size() && (a.empty() || std::memcmp(a.data(), b.data(), a.size() * sizeof(a[0])) == 0);
     };
-    const bool same = q->K == p->K && same_bytes(q->plan.passes, p->plan.passes) && same_bytes(q->plan.ops, p->plan.ops) &&
-                      same_bytes(q->plan.blocks, p->plan.blocks) &&
-                      p->head_aligned + q->pool_bytes.size() <= p->dev.bytes;
-    if (!same) {
+    auto same_plan = [&](const Plan& a, const Plan& b) {
+        return same_bytes(a.passes, b.passes) && same_bytes(a.ops, b.ops) && same_bytes(a.blocks, b.blocks);
+    };
+    if (q->K != p->K || !same_plan(q->core_plan, p->core_plan)) {
         program_destroy(q);
         return fail(LSG_E_STATE, "lsg_program_set_data: the operators plan differently from the program's (another "
                                  "structure): build a new program");
+    }
+    if (!same_plan(q->plan, p->plan) || p->head_aligned + q->pool_bytes.size() > p->dev.bytes) {
+        // the same operators, but their values lower to other blocks (a rotation whose phase is
+        // exactly one needs no diagonal): the program is made again with the new values
+        program_destroy(q);
+        return program_remake(p, ops, nops, pool, pool_entries);
     }
     // after the register's earlier work (a run may still read the old data); pageable source:
     // staged before the call returns
@@ -1806,7 +2068,7 @@ int lsg_program_basis_info(lsg_program p, int64_t* bytes_per_run, int64_t* tiles
 // Floating-point operations per register element that one operator of a pass executes (a
 // multiply or add counts 1, a fused multiply-add 2), as the register-block functions and the
 // shared-memory operators compute them.
-static double op_flops_per_element(const lsg::TileOp& op, bool complex_elems) {
+static double op_flops_per_element(const lsg::TileOp& op, bool complex_elems, bool whole) {
     using namespace lsg;
     const int c = op.tmpl;
     const double mul = complex_elems ? 6.0 : 1.0;  // one (complex) product per element
@@ -1822,6 +2084,8 @@ static double op_flops_per_element(const lsg::TileOp& op, bool complex_elems) {
     }
     if ((c >= kT_PERM1 && c < kT_PERM1 + 4) || (c >= kT_PERM2 && c < kT_PERM2 + 16)) return mul;
     if (c == kT_DIAGB || c == kT_SCALE || c == kT_DIAG) return mul;
+    if (c == kT_ROUND)
+        return (op.zmask & 16 ? 6.0 : 0.0) + (whole ? 6.0 : 4.0) * __builtin_popcount((unsigned)op.zmask & 15u);
     if (c == kT_DENSEB) return (complex_elems ? 8.0 : 2.0) * (double)(1 << op.k);
     if ((c >= kT_DEPOL1 && c < kT_DEPOL1 + 16) || c == kT_DEPOL2) return 4.0;
     if ((c >= kT_X1 && c < kT_X1 + 4) || (c >= kT_CX && c < kT_CX + 16) || (c >= kT_SWAP && c < kT_SWAP + 16)) return 0.0;
@@ -1848,7 +2112,11 @@ int lsg_program_pass_info(lsg_program p, int32_t cap, int64_t* bytes, double* fl
         if (blocks) blocks[i] = pd.nblocks;
         if (flops_per_element) {
             double f = 0.0;
-            for (int k = 0; k < pd.nops; ++k) f += op_flops_per_element(p->plan.ops[(size_t)(pd.first_op + k)], cx);
+            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks; ++bi) {
+                const lsg::BlockDesc& b = p->plan.blocks[(size_t)bi];
+                for (int k = b.first; k < b.first + b.nops; ++k)
+                    f += op_flops_per_element(p->plan.ops[(size_t)(pd.first_op + k)], cx, p->precision == LSG_C64);
+            }
             flops_per_element[i] = f;
         }
     }
@@ -1907,7 +2175,7 @@ int lsg_plan(int nbits, int precision, const lsg_op* ops, int32_t nops, int32_t*
         if (!op_bits_ok(ops[i], nbits)) return fail(LSG_E_ARG, "operator %d has a bad kind or bits", i);
     const int K = tile_bits_for(nbits, precision);
     const int L = std::min(K, low_bits_for(nbits, precision));
-    Plan plan = plan_passes(ops, nops, nbits, K, L, block_bits_for(precision));
+    Plan plan = plan_passes(ops, nops, nbits, K, L, block_bits_for(precision, nbits, true));
     if (nops > 0 && plan.passes.empty()) return fail(LSG_E_ARG, "an operator does not fit a tile of %d bits", K);
     LSG_CHECK(check_plan(plan));
     *passes = (int32_t)plan.passes.size();

@@ -142,12 +142,15 @@ bool op_call(std::ostringstream& o, const TileOp& t, int U, const char* T, int a
     else if (c == kT_DIAGB) name("diagb", true), o << ">";
     else if (c == kT_SCALE) name("scale", true), o << ">";
     else if (c == kT_DENSEB && !packed) name("denseb", true), o << ">";
+    else if (c == kT_ROUND && !packed) name("round", true), o << ">";
     else if (c >= kT_X1 && c < kT_X1 + 4) one("x", kT_X1, false), data = false;
     else if (c >= kT_CX && c < kT_CX + 16) two("cx", kT_CX, false), data = false;
     else if (c >= kT_SWAP && c < kT_SWAP + 16) two("swap", kT_SWAP, false), data = false;
     else return false;
     const std::string v = at ? "v + " + std::to_string(at) : std::string("v");
-    if (data) o << "(" << v << ", data + " << t.data << "LL + member * " << t.stride << "LL);\n";
+    if (data)
+        o << "(" << v << ", data + " << t.data << "LL + member * " << t.stride << "LL"
+          << (c == kT_ROUND ? ", " + std::to_string(t.zmask) : std::string()) << ");\n";
     else o << "(" << v << ");\n";
     return true;
 }
@@ -638,18 +641,60 @@ int jit_compile_check(const std::string& source) {
     return LSG_OK;
 }
 
+bool pass_swizzle_fits(const PassDesc& pd, size_t elem_bytes, int64_t register_bytes) {
+    if (register_bytes <= 0 || register_bytes % 1024 != 0 || (register_bytes >> 7) >= (1ll << 31)) return false;
+    // chunks of 512 bytes move in pairs (1 KB boxes), larger ones in whole 1 KB swizzle atoms
+    const size_t chunk = elem_bytes << pd.L;
+    if (chunk < 512) return false;
+    if (chunk > 512) return true;
+    return pd.K > pd.L && (elem_bytes << pd.hi[0]) % 1024 == 0 &&
+           register_bytes / (int64_t)(elem_bytes << pd.hi[0]) < (1ll << 31);
+}
+
+uint32_t tile_map_key(const PassDesc& pd, size_t elem_bytes) {
+    const uint64_t chunk = (uint64_t)elem_bytes << pd.L;
+    return chunk == 512 ? (0x80000000u | (uint32_t)pd.hi[0]) : (uint32_t)(std::min<uint64_t>(chunk, 16384) >> 7);
+}
+
+// The register as rows of 128 bytes, copied in boxes with the 128-byte swizzle (tile.cuh pipe_run):
+// 2-D boxes of min(chunk, 16 KB) for chunks of 1 KB and more, one map per box height; 3-D boxes
+// pairing two 512-byte chunks that differ in register bit h = hi[0], one map per h (rows of 128
+// bytes, blocks of 2^h elements).
+int encode_tile_map(void* state, int64_t register_bytes, size_t elem_bytes, const PassDesc& pd, Tmap* out) {
+    static_assert(sizeof(Tmap) == sizeof(CUtensorMap), "a tensor map");
+    const Driver& drv = driver();
+    const uint64_t bytes = (uint64_t)register_bytes, chunk = (uint64_t)elem_bytes << pd.L;
+    const bool pair = chunk == 512;
+    const uint64_t block = pair ? (uint64_t)elem_bytes << pd.hi[0] : 0;
+    if (!drv.encode) return fail(LSG_E_STATE, "cuTensorMapEncodeTiled is not available");
+    if (bytes % 1024 != 0 || (bytes >> 7) >= (1ull << 31) || (pair && (block % 1024 != 0 || bytes % block != 0)))
+        return fail(LSG_E_STATE, "a register of %llu bytes does not fit the swizzled tensor copies",
+                    (unsigned long long)bytes);
+    CUtensorMap m;
+    std::memset(&m, 0, sizeof(m));
+    cuuint64_t dims[3] = {32, pair ? block >> 7 : bytes >> 7, pair ? bytes / block : 1};
+    cuuint64_t strides[2] = {128, block};
+    cuuint32_t box[3] = {32, pair ? 4u : (uint32_t)(std::min<uint64_t>(chunk, 16384) >> 7), 2};
+    cuuint32_t estr[3] = {1, 1, 1};
+    if (drv.encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT32, pair ? 3 : 2, state, dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return fail(LSG_E_CUDA, "encoding the register's tensor map failed");
+    std::memcpy(out, &m, sizeof(m));
+    return LSG_OK;
+}
+
+bool swizzle_enabled() {
+    const char* env = getenv("LSG_SWIZZLE");
+    return !(env && env[0] == '0') && driver().encode;
+}
+
 bool jit_swizzle_fits(const Plan& plan, size_t elem_bytes, int64_t register_bytes) {
     const char* env = getenv("LSG_SWIZZLE");
     if (env && env[0] == '0') return false;
-    if (register_bytes <= 0 || register_bytes % 1024 != 0 || (register_bytes >> 7) >= (1ll << 31)) return false;
-    for (const PassDesc& pd : plan.passes) {
-        // chunks of 512 bytes move in pairs (1 KB boxes), larger ones in whole 1 KB swizzle atoms
-        const size_t chunk = elem_bytes << pd.L;
-        if (chunk < 512 || chunk % 512 != 0 || pd.K <= pd.L) return false;
-        if (chunk == 512 && ((elem_bytes << pd.hi[0]) % 1024 != 0 || (register_bytes / (elem_bytes << pd.hi[0])) >= (1ll << 31)))
-            return false;
-    }
-    return true;
+    for (const PassDesc& pd : plan.passes)
+        if (pd.K <= pd.L || !pass_swizzle_fits(pd, elem_bytes, register_bytes)) return false;
+    return !plan.passes.empty() || (register_bytes > 0 && register_bytes % 1024 == 0 && (register_bytes >> 7) < (1ll << 31));
 }
 
 std::string jit_source(const Plan& plan, int precision, int ctas, bool swz, bool packed) {
@@ -810,43 +855,22 @@ int jit_launch(const JitPasses& jp, const Plan& plan, void* state, int64_t membe
     LSG_CUDA(cudaGetDevice(&dev));
     LSG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const size_t smem = 2 * tile_bytes + (jp.swz ? 1024 : 0);
-    // the register as rows of 128 bytes, copied in boxes with the 128-byte swizzle (tile.cuh
-    // pipe_run): 2-D boxes of min(chunk, 16 KB) for chunks of 1 KB and more, one map per box
-    // height; 3-D boxes pairing two 512-byte chunks that differ in register bit h = hi[0], one map
-    // per h (rows of 128 bytes, blocks of 2^h elements). Unused without swizzle.
-    const uint64_t eb = (uint64_t)(tile_bytes >> plan.passes[0].K);
-    const uint64_t bytes = (uint64_t)member_elems * (uint64_t)batch * eb;
-    std::map<uint32_t, CUtensorMap> maps;
-    auto map_for = [&](const PassDesc& pd, CUtensorMap** out) -> int {
-        const uint64_t chunk = eb << pd.L;
-        const bool pair = chunk == 512;
-        const uint32_t key = pair ? (0x80000000u | (uint32_t)pd.hi[0]) : (uint32_t)(std::min<uint64_t>(chunk, 16384) >> 7);
+    const size_t eb = tile_bytes >> plan.passes[0].K;
+    const int64_t bytes = member_elems * batch * (int64_t)eb;
+    std::map<uint32_t, Tmap> maps;  // unused without swizzle
+    auto map_for = [&](const PassDesc& pd, Tmap** out) -> int {
+        const uint32_t key = tile_map_key(pd, eb);
         auto it = maps.find(key);
         if (it == maps.end()) {
-            CUtensorMap m;
-            std::memset(&m, 0, sizeof(m));
-            if (jp.swz) {
-                if (!drv.encode) return fail(LSG_E_STATE, "cuTensorMapEncodeTiled is not available");
-                const uint64_t block = pair ? eb << pd.hi[0] : 0;
-                if (bytes % 1024 != 0 || (bytes >> 7) >= (1ull << 31) || (pair && (block % 1024 != 0 || bytes % block != 0)))
-                    return fail(LSG_E_STATE, "a register of %llu bytes does not fit the swizzled tensor copies",
-                                (unsigned long long)bytes);
-                cuuint64_t dims[3] = {32, pair ? block >> 7 : bytes >> 7, pair ? bytes / block : 1};
-                cuuint64_t strides[2] = {128, block};
-                cuuint32_t box[3] = {32, pair ? 4u : key, 2};
-                cuuint32_t estr[3] = {1, 1, 1};
-                if (drv.encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT32, pair ? 3 : 2, state, dims, strides, box, estr,
-                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-                    return fail(LSG_E_CUDA, "encoding the register's tensor map failed");
-            }
+            Tmap m{};
+            if (jp.swz) LSG_CHECK(encode_tile_map(state, bytes, eb, pd, &m));
             it = maps.emplace(key, m).first;
         }
         *out = &it->second;
         return LSG_OK;
     };
     for (size_t i = 0; i < plan.passes.size(); ++i) {
-        CUtensorMap* map = nullptr;
+        Tmap* map = nullptr;
         LSG_CHECK(map_for(plan.passes[i], &map));
         CUfunction f = reinterpret_cast<CUfunction>(jp.fns[i]);
         const int64_t total = tiles_per_member[i] * batch;

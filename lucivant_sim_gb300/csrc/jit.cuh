@@ -46,6 +46,14 @@ int jit_compile_check(const std::string& source);
 // 1 KB swizzle atoms, and the register's 128-byte rows fit 31-bit coordinates.
 bool jit_swizzle_fits(const Plan& plan, size_t elem_bytes, int64_t register_bytes);
 
+// Whether interpreted passes may use them (LSG_SWIZZLE, the driver's encoder).
+bool swizzle_enabled();
+// Whether one pass can (chunks as above, or a tile that is one contiguous run).
+bool pass_swizzle_fits(const PassDesc& pd, size_t elem_bytes, int64_t register_bytes);
+// The tensor map a pass's swizzled copies go through (passes of equal keys share it).
+uint32_t tile_map_key(const PassDesc& pd, size_t elem_bytes);
+int encode_tile_map(void* state, int64_t register_bytes, size_t elem_bytes, const PassDesc& pd, Tmap* out);
+
 // Specialize a planned gate program (no trajectory operators, no shared-memory operators), or
 // nullptr when it can't be (unsupported operators, no NVRTC, compilation failure): the
 // interpreter then runs it. `ctas` is the launch bound's CTAs per SM. Passes compile in parallel

@@ -4,6 +4,8 @@
 #include <stdint.h>
 
 #ifndef __CUDACC_RTC__
+#include <cstddef>
+
 #include <vector>
 #endif
 
@@ -13,7 +15,8 @@ namespace lsg {
 // (one contiguous run per chunk), local bit L+j is register bit hi[j]. Register bits outside the
 // tile (outer[]) enumerate the tiles.
 struct PassDesc {
-    int K, L, nouter, nops, first_op, pad;
+    int K, L, nouter, nops, first_op;
+    int rounds;  // lowered passes: their rounds, whose data the kernel stages (TileOp::count numbers them)
     int first_block, nblocks;
     int hi[32];
     int outer[32];
@@ -36,7 +39,18 @@ struct BlockDesc {
     int vec;  // 1, 2 or 4: the block's last positions are tile bits (1,) 0, so each group holds
               // runs of `vec` consecutive elements (vector shared-memory accesses)
     unsigned dep[5];  // group index g -> tile position of its first element: OR of (g << i) & dep[i]
+    // The block in a tile moved by swizzled tensor copies (engine.cu block_layout): every address is
+    // linear over GF(2) in the bits of the group index g and of the element index e, so element e of
+    // group g lies at byte XOR(gb[i], bits i of g) ^ XOR(lob[j], positions j of e) ^ lconst, and is
+    // stored at the same with sob and sconst. Renames (X, cx, swap) at the block's two ends are part
+    // of these maps and not executed: operators first + lead .. first + lead + nexec - 1 are.
     int pad[2];
+    unsigned short gb[16];  // (16-byte aligned: read as words)
+    unsigned short lob[4], sob[4];
+    unsigned short lconst, sconst;
+    short lead, nexec;
+    short lvec, svec;  // elements per shared-memory access
+    int pad2;
 };
 
 // Operator kinds beyond the public LSG_OP_* set, used by trajectory programs.
@@ -55,7 +69,7 @@ struct TileOp {
     int tmpl;       // register-block code: kind and positions (see tile.cuh)
     int pos[8];     // positions of the operator's bits within its block (0 = block MSB)
     int zmask;      // trace-preserving 4x4 operators: coefficients zero for every member
-                    // (bit 4 * (row - 1) + column), left out by specialized passes
+                    // (bit 4 * (row - 1) + column), left out by specialized passes; rounds: their parts
     int pad;
 };
 
@@ -64,6 +78,9 @@ struct TileOp {
 static_assert(sizeof(PassDesc) % 16 == 0, "PassDesc keeps 16-byte alignment");
 static_assert(sizeof(TileOp) % 16 == 0, "TileOp keeps 16-byte alignment");
 static_assert(sizeof(BlockDesc) % 16 == 0, "BlockDesc keeps 16-byte alignment");
+#ifndef __CUDACC_RTC__
+static_assert(offsetof(BlockDesc, gb) % 16 == 0, "a block's address maps are read as 16-byte words");
+#endif
 
 #ifndef __CUDACC_RTC__
 struct Plan {
@@ -87,12 +104,14 @@ constexpr int kT_X1 = 75;       // + P: unit-phase X (register swap)
 constexpr int kT_CX = 79;       // + 4 * Pcontrol + Ptarget: unit-phase CX (register swap)
 constexpr int kT_SWAP = 95;     // + 4 * P0 + P1
 constexpr int kT_DENSEB = 111;  // a whole register block as one dense 2^u x 2^u complex matrix (block order)
-constexpr int kT_CODES = 112;   // the kernel's codes are exactly 0 .. kT_CODES-1 (a dense switch)
+constexpr int kT_ROUND = 112;   // a diagonal over the block, then real rotations on its bits (complex; rb_round);
+                                // zmask: bit P a rotation on position P, bit 4 the diagonal
+constexpr int kT_CODES = 113;   // the kernel's codes are exactly 0 .. kT_CODES-1 (a dense switch)
 // host-side markers, rewritten before upload: mixtures become dense codes per member in the kernel,
 // diagonals become kT_DIAGB
-constexpr int kT_MIX1 = 112;    // + P
-constexpr int kT_MIX2 = 116;    // + 4 * P0 + P1
-constexpr int kT_DIAG = 132;
+constexpr int kT_MIX1 = 113;    // + P
+constexpr int kT_MIX2 = 117;    // + 4 * P0 + P1
+constexpr int kT_DIAG = 133;
 constexpr int kT_GENERIC = -1;
 // The greedy fusion planner (csrc/engine.cu): lsg_op list -> passes of tile-local operators.
 // pred/draw/count (may be null) give trajectory operators their predicate bit, uniform offset and

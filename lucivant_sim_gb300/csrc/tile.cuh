@@ -23,18 +23,22 @@ constexpr int kCompute = 256;
 
 // Barrier over the 256 compute threads only (named barrier 1): the pipelined kernel's producer
 // warp never joins it. In the 256-thread kernel it spans the whole CTA.
-__device__ __forceinline__ void cbar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+template <int NC = kCompute>
+__device__ __forceinline__ void cbar() {
+    asm volatile("bar.sync 1, %0;" ::"n"(NC) : "memory");
+}
 
 // The same barrier, returning whether any compute thread passed true.
+template <int NC = kCompute>
 __device__ __forceinline__ bool cbar_or(bool v) {
     uint32_t out;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, 256, p;\n\t"
+        "bar.red.or.pred q, 1, %2, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(out)
-        : "r"((uint32_t)v)
+        : "r"((uint32_t)v), "n"(NC)
         : "memory");
     return out != 0;
 }
@@ -412,10 +416,199 @@ __device__ __forceinline__ void rb_denseb(T* v, const T* m) {
     for (int e = 0; e < D; ++e) v[e] = out[e];
 }
 
+// Two FP32 values in one 64-bit register pair, each lane of an operation rounded as the scalar
+// mul / fma (sm_100 and later).
+struct F2 {
+    unsigned long long r;
+};
+__device__ __forceinline__ F2 f2_bcast(float c) {
+    F2 o;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(o.r) : "f"(c));
+    return o;
+}
+__device__ __forceinline__ F2 f2_mul(float c, F2 a) {
+    F2 o;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(o.r) : "l"(f2_bcast(c).r), "l"(a.r));
+    return o;
+}
+__device__ __forceinline__ F2 f2_fma(float c, F2 a, F2 acc) {
+    F2 o;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(o.r) : "l"(f2_bcast(c).r), "l"(a.r), "l"(acc.r));
+    return o;
+}
+// the pair at p (8-byte aligned): p[0] to lane 0, p[1] to lane 1
+__device__ __forceinline__ F2 ld_f2(const float* p) {
+    F2 o;
+    o.r = *reinterpret_cast<const unsigned long long*>(p);
+    return o;
+}
+__device__ __forceinline__ void st_f2(float* p, F2 v) { *reinterpret_cast<unsigned long long*>(p) = v.r; }
+
+// A round of a lowered complex block (lower.cu): the block's diagonal (mask bit 4), then a real plane
+// rotation on every position P with mask bit P. Data: the 2^U diagonal entries (complex64: as (re,
+// re, -im, im), the operands of packed products), then U rotations.
+//
+// complex128 is bound by FP64 issue: a rotation (t, flip) is [[1, -t], [t, 1]] (flip: [[t, -1],
+// [1, t]]), two multiply-adds an amplitude, its cosine (flip: sine) left to the diagonal.
+// complex64 takes the whole rotation (c, s), both components of an amplitude in one packed
+// instruction and both amplitudes updated in place (an update that needs both old values costs
+// copies, as dear as the multiplication it saves). Each result is rounded once at its own size: c *
+// x is added last. Fewer roundings show: expectations of 40-layer circuits are off by 0.8e-6 rms
+// where dense 2x2 matrices give 1.5e-6 and three shears, at three quarters of the arithmetic, 1.2e-6.
+// A dense 2x2 complex matrix takes eight multiply-adds an amplitude.
+__device__ __forceinline__ void rb_turn(unsigned long long& x, unsigned long long& y, F2 c, F2 s, F2 ns) {
+    asm("{\n\t.reg .b64 p, q;\n\t"
+        "mul.rn.f32x2 p, %4, %1;\n\tmul.rn.f32x2 q, %3, %0;\n\t"
+        "fma.rn.f32x2 %0, %2, %0, p;\n\tfma.rn.f32x2 %1, %2, %1, q;\n\t}"
+        : "+l"(x), "+l"(y)
+        : "l"(c.r), "l"(s.r), "l"(ns.r));
+}
+__device__ __forceinline__ void rb_rotate(Cx<float>& x, Cx<float>& y, Cx<float> rot) {
+    unsigned long long a, b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "f"(x.re), "f"(x.im));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(y.re), "f"(y.im));
+    rb_turn(a, b, f2_bcast(rot.re), f2_bcast(rot.im), f2_bcast(-rot.im));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x.re), "=f"(x.im) : "l"(a));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(y.re), "=f"(y.im) : "l"(b));
+}
+__device__ __forceinline__ void rb_rotate(Cx<double>& x, Cx<double>& y, double t) {
+    const Cx<double> a = x, b = y;
+    x = Cx<double>(fma(-t, b.re, a.re), fma(-t, b.im, a.im));
+    y = Cx<double>(fma(t, a.re, b.re), fma(t, a.im, b.im));
+}
+__device__ __forceinline__ void rb_rotate_flip(Cx<double>& x, Cx<double>& y, double t) {
+    const Cx<double> a = x, b = y;
+    x = Cx<double>(fma(t, a.re, -b.re), fma(t, a.im, -b.im));
+    y = Cx<double>(fma(t, b.re, a.re), fma(t, b.im, a.im));
+}
+
+template <typename T, int U>
+__device__ __forceinline__ void rb_round(T* v, const T* m, int mask) {
+    if constexpr (Elem<T>::complex) {
+        constexpr int D = 1 << U, ND = sizeof(T) == 8 ? 2 * D : D;
+        T rot[U];  // read ahead of the diagonal's arithmetic (a diagonal alone has none)
+#pragma unroll
+        for (int P = 0; P < U; ++P) rot[P] = (mask & 15) ? m[ND + P] : T();
+        if (mask & 16) {
+#pragma unroll
+            for (int e = 0; e < D; ++e) {
+                if constexpr (sizeof(T) == 8) {
+                    T mm[2];
+                    ldv<T, 2>(m + 2 * e, mm);
+                    v[e] = cmul(T(mm[0].re, mm[1].im), v[e]);
+                } else {
+                    v[e] = cmul(m[e], v[e]);
+                }
+            }
+        }
+#pragma unroll
+        for (int P = 0; P < U; ++P) {
+            if (!((mask >> P) & 1)) continue;
+            const int B = 1 << (U - 1 - P);
+            if constexpr (sizeof(T) == 8) {
+#pragma unroll
+                for (int e = 0; e < D; ++e)
+                    if (!(e & B)) rb_rotate(v[e], v[e | B], rot[P]);
+            } else if (rot[P].im == 0) {
+#pragma unroll
+                for (int e = 0; e < D; ++e)
+                    if (!(e & B)) rb_rotate(v[e], v[e | B], rot[P].re);
+            } else {
+#pragma unroll
+                for (int e = 0; e < D; ++e)
+                    if (!(e & B)) rb_rotate_flip(v[e], v[e | B], rot[P].re);
+            }
+        }
+    }
+}
+
+// Lowered complex64 groups stay in 64-bit register pairs, updated in place: as separate floats every
+// packed instruction would first collect its operands into pairs, and where branches merge each
+// operator's results would be copied back (half of the pass's instructions).
+template <typename T>
+struct Held {
+    using W = T;
+};
+template <>
+struct Held<Cx<float>> {
+    using W = unsigned long long;
+};
+
+__device__ __forceinline__ ulonglong2 lds_pair(uint32_t a) {
+    ulonglong2 d;
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(d.x), "=l"(d.y) : "r"(a));
+    return d;
+}
+
+// rb_round on NG held groups, its data at shared-memory address `m`: the same operations.
+template <int U, int NG>
+__device__ __forceinline__ void held_round(unsigned long long (*w)[1 << U], uint32_t m, int mask) {
+    constexpr int D = 1 << U;
+    if (mask & 16) {
+#pragma unroll
+        for (int e = 0; e < D; ++e) {
+            const ulonglong2 d = lds_pair(m + 16 * e);  // (re, re), (-im, im)
+#pragma unroll
+            for (int k = 0; k < NG; ++k)
+                asm("{\n\t.reg .b32 a, b;\n\t.reg .b64 t;\n\t"
+                    "mov.b64 {a, b}, %0;\n\tmov.b64 t, {b, a};\n\t"
+                    "mul.rn.f32x2 t, %2, t;\n\tfma.rn.f32x2 %0, %1, %0, t;\n\t}"
+                    : "+l"(w[k][e])
+                    : "l"(d.x), "l"(d.y));
+        }
+    }
+#pragma unroll
+    for (int P = 0; P < U; ++P) {
+        if (!((mask >> P) & 1)) continue;
+        float c, s;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(c), "=f"(s) : "r"(m + 16 * D + 8 * P));
+        const int B = 1 << (U - 1 - P);
+        const F2 cc = f2_bcast(c), ss = f2_bcast(s), ns = f2_bcast(-s);
+#pragma unroll
+        for (int k = 0; k < NG; ++k)
+#pragma unroll
+            for (int e = 0; e < D; ++e)
+                if (!(e & B)) rb_turn(w[k][e], w[k][e | B], cc, ss, ns);
+    }
+}
+template <int U, int NG>
+__device__ __forceinline__ void held_round(Cx<double> (*v)[1 << U], uint32_t m, int mask) {
+    constexpr int D = 1 << U;
+    if (mask & 16) {
+#pragma unroll
+        for (int e = 0; e < D; ++e) {
+            Cx<double> d;
+            asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(d.re), "=d"(d.im) : "r"(m + 16 * e));
+#pragma unroll
+            for (int k = 0; k < NG; ++k) v[k][e] = cmul(d, v[k][e]);
+        }
+    }
+#pragma unroll
+    for (int P = 0; P < U; ++P) {
+        if (!((mask >> P) & 1)) continue;
+        double t, flip;
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(t), "=d"(flip) : "r"(m + 16 * (D + P)));
+        const int B = 1 << (U - 1 - P);
+        if (flip == 0.0) {
+#pragma unroll
+            for (int k = 0; k < NG; ++k)
+#pragma unroll
+                for (int e = 0; e < D; ++e)
+                    if (!(e & B)) rb_rotate(v[k][e], v[k][e | B], t);
+        } else {
+#pragma unroll
+            for (int k = 0; k < NG; ++k)
+#pragma unroll
+                for (int e = 0; e < D; ++e)
+                    if (!(e & B)) rb_rotate_flip(v[k][e], v[k][e | B], t);
+        }
+    }
+}
+
 // The interpreter's form of rb_denseb: the group is in registers, each output row is stored to
 // the tile as soon as it is formed (the group's elements belong to this thread alone).
 template <typename T, int U>
-__device__ __forceinline__ void rb_denseb_store(T* tile, uint32_t base, const uint32_t* off, const T* v, const T* m) {
+__device__ __forceinline__ void rb_denseb_xor(T* tile, uint32_t base, const uint32_t* off, const T* v, const T* m) {
     constexpr int D = 1 << U;
 #pragma unroll
     for (int r = 0; r < D; ++r) {
@@ -427,21 +620,26 @@ __device__ __forceinline__ void rb_denseb_store(T* tile, uint32_t base, const ui
             if ((c & 3) == 0) ldv<T, 4>(m + r * D + c, row);
             acc = cfma(row[c & 3], v[c], acc);
         }
-        tile[base | off[r]] = acc;
+        tile[base ^ off[r]] = acc;
     }
 }
 
 // Unit-phase permutations are register renames: no arithmetic at all.
+template <typename T>
+__device__ __forceinline__ void rb_exchange(T& a, T& b) {
+    const T t = a;
+    a = b;
+    b = t;
+}
+__device__ __forceinline__ void rb_exchange(unsigned long long& a, unsigned long long& b) {
+    asm("{\n\t.reg .b64 t;\n\tmov.b64 t, %0;\n\tmov.b64 %0, %1;\n\tmov.b64 %1, t;\n\t}" : "+l"(a), "+l"(b));
+}
 template <typename T, int U, int P>
 __device__ __forceinline__ void rb_x(T* v) {
     constexpr int B = 1 << (U - 1 - P);
 #pragma unroll
     for (int e = 0; e < (1 << U); ++e)
-        if (!(e & B)) {
-            const T t = v[e];
-            v[e] = v[e | B];
-            v[e | B] = t;
-        }
+        if (!(e & B)) rb_exchange(v[e], v[e | B]);
 }
 
 // controlled X: control at position PC, target at PT
@@ -450,11 +648,7 @@ __device__ __forceinline__ void rb_cx(T* v) {
     constexpr int BC = 1 << (U - 1 - PC), BT = 1 << (U - 1 - PT);
 #pragma unroll
     for (int e = 0; e < (1 << U); ++e)
-        if ((e & BC) && !(e & BT)) {
-            const T t = v[e];
-            v[e] = v[e | BT];
-            v[e | BT] = t;
-        }
+        if ((e & BC) && !(e & BT)) rb_exchange(v[e], v[e | BT]);
 }
 
 template <typename T, int U, int P0, int P1>
@@ -462,11 +656,7 @@ __device__ __forceinline__ void rb_swap(T* v) {
     constexpr int B0 = 1 << (U - 1 - P0), B1 = 1 << (U - 1 - P1);
 #pragma unroll
     for (int e = 0; e < (1 << U); ++e)
-        if ((e & B0) && !(e & B1)) {
-            const T t = v[e];
-            v[e] = v[(e & ~B0) | B1];
-            v[(e & ~B0) | B1] = t;
-        }
+        if ((e & B0) && !(e & B1)) rb_exchange(v[e], v[(e & ~B0) | B1]);
 }
 
 // (1-p) rho + (p/2) I Tr on one row bit (position PR) and its column bit (PC)
@@ -543,32 +733,6 @@ __device__ __forceinline__ void rb_scale(T* v, const T* m) {
 // fma.rn.f32x2, sm_100 and later): lane 0 is the group with tile bit 0 clear. Each lane is
 // rounded exactly as the scalar mul / fma of the unpacked form, in the same order, so results
 // are identical bit for bit; the coefficient is broadcast to both lanes.
-struct F2 {
-    unsigned long long r;
-};
-__device__ __forceinline__ F2 f2_bcast(float c) {
-    F2 o;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(o.r) : "f"(c));
-    return o;
-}
-__device__ __forceinline__ F2 f2_mul(float c, F2 a) {
-    F2 o;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(o.r) : "l"(f2_bcast(c).r), "l"(a.r));
-    return o;
-}
-__device__ __forceinline__ F2 f2_fma(float c, F2 a, F2 acc) {
-    F2 o;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(o.r) : "l"(f2_bcast(c).r), "l"(a.r), "l"(acc.r));
-    return o;
-}
-// the pair at p (8-byte aligned): p[0] to lane 0, p[1] to lane 1
-__device__ __forceinline__ F2 ld_f2(const float* p) {
-    F2 o;
-    o.r = *reinterpret_cast<const unsigned long long*>(p);
-    return o;
-}
-__device__ __forceinline__ void st_f2(float* p, F2 v) { *reinterpret_cast<unsigned long long*>(p) = v.r; }
-
 template <int U, int P>
 __device__ __forceinline__ void rp_dense1(F2* v, const float* m) {
     constexpr int B = 1 << (U - 1 - P);
@@ -735,8 +899,8 @@ __device__ __forceinline__ const T* mixture_pick(const TileOp& op, const T* m, d
     LSG_P2ONE(X, BASE, 2, 3) LSG_P2ONE(X, BASE, 3, 0) LSG_P2ONE(X, BASE, 3, 1) LSG_P2ONE(X, BASE, 3, 2) \
     LSG_SAME(BASE)
 
-template <typename T, int U>
-__device__ __forceinline__ void rb_apply(T* v, int code, const T* m) {
+template <typename T, int U, bool ROUNDS = true>
+__device__ __forceinline__ void rb_apply(T* v, int code, int mask, const T* m) {
     switch (code) {
         LSG_P1(rb_dense1, kT_DENSE1)
         LSG_P2(rb_dense2, kT_DENSE2)
@@ -752,7 +916,20 @@ __device__ __forceinline__ void rb_apply(T* v, int code, const T* m) {
         LSG_R2(rb_swap, kT_SWAP)
         case kT_DIAGB: rb_diagb<T, U>(v, m); break;
         case kT_SCALE: rb_scale<T, U>(v, m); break;
+        case kT_ROUND:
+            if constexpr (ROUNDS) rb_round<T, U>(v, m, mask);
+            break;
+        default: break;
+    }
+}
 
+// The renames on a held group.
+template <int U, typename T>
+__device__ __forceinline__ void held_rename(T* v, int code) {
+    switch (code) {
+        LSG_R1(rb_x, kT_X1)
+        LSG_R2(rb_cx, kT_CX)
+        LSG_R2(rb_swap, kT_SWAP)
         default: break;
     }
 }
@@ -835,7 +1012,7 @@ __device__ __forceinline__ void store_group(T* tile, uint32_t base, const uint32
 // A register-block operator resolved for the tile's member: its code and data pointer (built
 // once per tile in shared memory, so the inner loop reads one 16-byte record per operator).
 struct OpRec {
-    int code, pad;
+    int code, mask;  // mask: a round's parts (TileOp::zmask)
     const void* m;
 };
 
@@ -864,16 +1041,243 @@ __device__ void run_block(T* tile, int tbits, const BlockDesc& blk, const OpRec*
         load_group<T, U>(tile, base, off, blk.vec, v);
         if constexpr (Elem<T>::complex) {
             if (dense) {  // a fused block: each output row straight back to its place in the tile
-                rb_denseb_store<T, U>(tile, base, off, v, static_cast<const T*>(recs[blk.first].m));
+                rb_denseb_xor<T, U>(tile, base, off, v, static_cast<const T*>(recs[blk.first].m));
                 continue;
             }
         }
         for (int o = 0; o < blk.nops; ++o) {
             const OpRec r = recs[blk.first + o];
-            rb_apply<T, U>(v, r.code, static_cast<const T*>(r.m));
+            rb_apply<T, U>(v, r.code, r.mask, static_cast<const T*>(r.m));
         }
         store_group<T, U>(tile, base, off, blk.vec, v);
     }
+}
+
+// Shared-memory words by 32-bit address.
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
+    uint4 w;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(a) : "memory");
+    return w;
+}
+__device__ __forceinline__ uint2 lds8(uint32_t a) {
+    uint2 w;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w.x), "=r"(w.y) : "r"(a) : "memory");
+    return w;
+}
+__device__ __forceinline__ uint32_t lds4(uint32_t a) {
+    uint32_t w;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(a) : "memory");
+    return w;
+}
+__device__ __forceinline__ uint32_t lds2(uint32_t a) {
+    uint16_t w;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(w) : "r"(a) : "memory");
+    return w;
+}
+__device__ __forceinline__ void sts16(uint32_t a, uint4 w) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+}
+__device__ __forceinline__ void sts8(uint32_t a, uint2 w) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(w.x), "r"(w.y) : "memory");
+}
+__device__ __forceinline__ void sts4(uint32_t a, uint32_t w) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(w) : "memory");
+}
+
+// BYTES of consecutive elements between shared memory and registers.
+template <typename T, int BYTES>
+__device__ __forceinline__ void lds_elems(uint32_t a, T* v) {
+    if constexpr (BYTES == 16) {
+        const uint4 w = lds16(a);
+        memcpy(v, &w, 16);
+    } else if constexpr (BYTES == 8) {
+        const uint2 w = lds8(a);
+        memcpy(v, &w, 8);
+    } else {
+        const uint32_t w = lds4(a);
+        memcpy(v, &w, 4);
+    }
+}
+template <typename T, int BYTES>
+__device__ __forceinline__ void sts_elems(uint32_t a, const T* v) {
+    if constexpr (BYTES == 16) {
+        uint4 w;
+        memcpy(&w, v, 16);
+        sts16(a, w);
+    } else if constexpr (BYTES == 8) {
+        uint2 w;
+        memcpy(&w, v, 8);
+        sts8(a, w);
+    } else {
+        uint32_t w;
+        memcpy(&w, v, 4);
+        sts4(a, w);
+    }
+}
+
+// Element e of a group at byte `at` ^ the XOR of ob over its set positions, VEC elements per access,
+// in Gray-code order: one XOR steps from each access to the next. `tile` is the tile's
+// shared-memory address.
+template <typename T, int U, int VEC, bool STORE>
+__device__ __forceinline__ void move_group(uint32_t tile, uint32_t at, const uint32_t* ob, T* v) {
+    constexpr int LV = VEC == 4 ? 2 : VEC == 2 ? 1 : 0, N = 1 << (U - LV);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int e = (i ^ (i >> 1)) << LV;
+#pragma unroll
+        for (int k = 0; k < U - LV; ++k)  // the step's bit: i's lowest one
+            if ((i & (2 * (1 << k) - 1)) == (1 << k)) at ^= ob[U - 1 - LV - k];
+        if constexpr (STORE) sts_elems<T, VEC * (int)sizeof(T)>(tile + at, v + e);
+        else lds_elems<T, VEC * (int)sizeof(T)>(tile + at, v + e);
+    }
+}
+template <typename T, int U, bool STORE>
+__device__ __forceinline__ void move_swz(uint32_t tile, uint32_t at, const uint32_t* ob, int vec, T* v) {
+    if constexpr (sizeof(T) == 4 && U >= 2) {
+        if (vec == 4) {
+            move_group<T, U, 4, STORE>(tile, at, ob, v);
+            return;
+        }
+    }
+    if constexpr (sizeof(T) <= 8) {
+        if (vec >= 2) {
+            move_group<T, U, 2, STORE>(tile, at, ob, v);
+            return;
+        }
+    }
+    move_group<T, U, 1, STORE>(tile, at, ob, v);
+}
+
+// Byte offsets of a staged block descriptor's fields.
+constexpr uint32_t kDescGb = 80, kDescOb = 112, kDescConst = 128;
+
+// A block's GF(2) address maps (BlockDesc gb, lob, sob) as this thread needs them.
+template <int U, int NC = kCompute>
+struct BlockMaps {
+    uint32_t desc, own;  // the descriptor (shared memory); this thread's part of the group address (g below NC)
+    // `blk` is staged in shared memory: read by its 32-bit address (generic loads wait longer)
+    __device__ __forceinline__ explicit BlockMaps(const BlockDesc& blk) {
+        desc = smem_u32(&blk);
+        const uint4 gb = lds16(desc + kDescGb);  // two bits' addresses per word
+        const uint32_t t = threadIdx.x;
+        auto both = [&](int i) { return ((0u - ((t >> i) & 1u)) & 0xffffu) | (0u - ((t >> (i + 1)) & 1u)) << 16; };
+        const uint32_t a = (gb.x & both(0)) ^ (gb.y & both(2)) ^ (gb.z & both(4)) ^ (gb.w & both(6));
+        own = (a ^ (a >> 16)) & 0xffffu;
+    }
+    // group g's base address (g = this thread's index plus a multiple of the compute threads)
+    __device__ __forceinline__ uint32_t base(int g) const {
+        uint32_t a = own;
+        for (uint32_t at = desc + kDescGb + (NC == 128 ? 14 : 16), h = (uint32_t)g / NC; h; at += 2, h >>= 1)
+            a ^= (h & 1) ? lds2(at) : 0u;
+        return a;
+    }
+    __device__ __forceinline__ int lead() const { return (int)lds2(desc + kDescConst + 4); }
+    __device__ __forceinline__ int nexec() const { return (int)lds2(desc + kDescConst + 6); }
+    // The load (STORE: store) map: steps per position, constant, elements per access. Read where it is
+    // used, so that the operators between have its registers.
+    template <bool STORE>
+    __device__ __forceinline__ uint32_t map(uint32_t* ob, int* vec) const {
+        const uint2 w = lds8(desc + kDescOb + (STORE ? 8 : 0));
+#pragma unroll
+        for (int j = 0; j < U; ++j) ob[j] = ((j & 2 ? w.y : w.x) >> (16 * (j & 1))) & 0xffffu;
+        *vec = (int)lds2(desc + kDescConst + 8 + (STORE ? 2 : 0));
+        return lds2(desc + kDescConst + (STORE ? 2 : 0));
+    }
+    // one group's elements, base address `at`
+    template <typename W, bool STORE>
+    __device__ __forceinline__ void move(uint32_t tile, uint32_t at, W* v) const {
+        uint32_t ob[U];
+        int vec;
+        const uint32_t c = map<STORE>(ob, &vec);
+        move_swz<W, U, STORE>(tile, at ^ c, ob, vec, v);
+    }
+};
+
+// run_block on a swizzled tile.
+template <typename T, int U, bool ROUNDS>
+__device__ __forceinline__ void run_block_swz(T* tile, int tbits, const BlockDesc& blk, const OpRec* __restrict__ recs) {
+    const uint32_t t32 = smem_u32(tile);
+    const BlockMaps<U> maps(blk);
+    const int groups = 1 << (tbits - U);
+    const int first = blk.first + maps.lead(), nops = maps.nexec();
+    const bool dense = nops == 1 && recs[first].code == kT_DENSEB;
+    for (int g = threadIdx.x; g < groups; g += kCompute) {
+        const uint32_t base = maps.base(g);
+        T v[1 << U];
+        maps.template move<T, false>(t32, base, v);
+        if constexpr (Elem<T>::complex) {
+            if (dense) {  // a fused block: each output row straight to its place in the tile
+                uint32_t at[1 << U], ob[U];
+                int vec;
+                const uint32_t c = maps.template map<true>(ob, &vec);
+#pragma unroll
+                for (int e = 0; e < (1 << U); ++e) {
+                    at[e] = 0;
+#pragma unroll
+                    for (int j = 0; j < U; ++j)
+                        if ((e >> (U - 1 - j)) & 1) at[e] ^= ob[j] / (uint32_t)sizeof(T);
+                }
+                rb_denseb_xor<T, U>(tile, (base ^ c) / (uint32_t)sizeof(T), at, v, static_cast<const T*>(recs[first].m));
+                continue;
+            }
+        }
+        for (int o = 0; o < nops; ++o) {
+            const OpRec r = recs[first + o];
+            rb_apply<T, U, ROUNDS>(v, r.code, r.mask, static_cast<const T*>(r.m));
+        }
+        maps.template move<T, true>(t32, base, v);
+    }
+}
+
+// The staged data of one round: its diagonal and rotations at block width 4, in 16-byte words.
+template <typename T>
+constexpr int round_words() {
+    return (int)(((sizeof(T) == 8 ? 32 : 16) + 4) * sizeof(T) / 16);
+}
+
+// A block of rounds and renames only (a lowered one) on a swizzled tile; the operators' records hold
+// their data's shared-memory addresses. Each thread takes NG groups at a time: every coefficient and
+// record read, every dispatch serves them all (a 16-byte read costs four wavefronts even when a
+// whole warp reads one address).
+template <typename T, int U, int NG, int NC>
+__device__ __forceinline__ void run_groups(uint32_t t32, const BlockDesc& blk, const BlockMaps<U, NC>& maps,
+                                           const OpRec* __restrict__ recs, int groups) {
+    using W = typename Held<T>::W;
+    const uint32_t ops = smem_u32(recs) + (uint32_t)sizeof(OpRec) * (uint32_t)(blk.first + maps.lead());
+    const int nops = maps.nexec();
+    for (int g = threadIdx.x; g < groups; g += NG * NC) {
+        uint32_t base[NG];
+        W w[NG][1 << U];
+#pragma unroll
+        for (int k = 0; k < NG; ++k) {
+            base[k] = maps.base(g + k * NC);
+            maps.template move<W, false>(t32, base[k], w[k]);
+        }
+        for (int o = 0; o < nops; ++o) {
+            const uint4 r = lds16(ops + (uint32_t)sizeof(OpRec) * o);  // code, mask, address
+            if ((int)r.x == kT_ROUND) {
+                held_round<U, NG>(w, r.z, (int)r.y);
+            } else {
+#pragma unroll
+                for (int k = 0; k < NG; ++k) held_rename<U>(w[k], (int)r.x);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < NG; ++k) maps.template move<W, true>(t32, base[k], w[k]);
+    }
+}
+template <typename T, int U, int NC>
+__device__ __forceinline__ void run_block_rounds(T* tile, int tbits, const BlockDesc& blk, const OpRec* __restrict__ recs) {
+    const uint32_t t32 = smem_u32(tile);
+    const BlockMaps<U, NC> maps(blk);
+    const int groups = 1 << (tbits - U);
+    if constexpr (sizeof(T) == 8) {
+        if (groups >= 2 * NC) {
+            run_groups<T, U, 2, NC>(t32, blk, maps, recs, groups);
+            return;
+        }
+    }
+    run_groups<T, U, 1, NC>(t32, blk, maps, recs, groups);
 }
 
 template <typename T>
@@ -912,10 +1316,48 @@ __device__ void run_ops(T* tile, int tbits, const TileOp* __restrict__ ops, int 
 }
 
 // All blocks of a pass on one tile (the 256 compute threads).
-template <typename T>
+// MODE: how the pass's blocks run.
+constexpr int kPlain = 0;   // plain tiles, any block
+constexpr int kSwz = 1;     // swizzled tiles, register blocks without rounds (fewer registers)
+constexpr int kMixed = 3;   // swizzled tiles, register blocks, rounds among their operators
+constexpr int kRounds = 2;  // swizzled tiles, lowered complex blocks (rounds and renames)
+template <typename T, int MODE = kPlain>
 __device__ __forceinline__ void compute_tile(T* tile, int K, const PassDesc& pd, const BlockDesc* sblk,
                                              const TileOp* sops, OpRec* recs, const T* __restrict__ data,
-                                             int64_t member, const TrajCtx& ctx) {
+                                             int64_t member, const TrajCtx& ctx, uint4* staged = nullptr,
+                                             int64_t* staged_member = nullptr) {
+    if constexpr (MODE == kRounds) {
+        constexpr int NC = 128;
+        // The rounds' data and the records of this tile's member, once for consecutive tiles of one
+        // member. Read from global memory by every warp and block they took more of the L1's
+        // data path than the tile itself: 65% of it busy, loads the first stall reason.
+        if (member != *staged_member) {
+            for (int o = threadIdx.x; o < pd.nops; o += NC)
+                recs[o] = OpRec{sops[o].tmpl, sops[o].zmask,
+                                reinterpret_cast<const void*>((uintptr_t)smem_u32(staged + sops[o].count * round_words<T>()))};
+            for (int i = threadIdx.x; i < pd.nops * round_words<T>(); i += NC) {
+                const TileOp& op = sops[i / round_words<T>()];
+                const int w = i % round_words<T>();
+                const int have = (int)((((sizeof(T) == 8 ? 2 : 1) << op.k) + op.k) * sizeof(T) + 15) / 16;
+                if (op.tmpl == kT_ROUND && w < have)
+                    staged[op.count * round_words<T>() + w] =
+                        __ldg(reinterpret_cast<const uint4*>(data + op.data + member * op.stride) + w);
+            }
+            *staged_member = member;
+        }
+        for (int bi = 0; bi < pd.nblocks; ++bi) {
+            const BlockDesc& blk = sblk[bi];
+            cbar<NC>();
+            switch (blk.u) {
+                case 1: run_block_rounds<T, 1, NC>(tile, K, blk, recs); break;
+                case 2: run_block_rounds<T, 2, NC>(tile, K, blk, recs); break;
+                case 3: run_block_rounds<T, 3, NC>(tile, K, blk, recs); break;
+                default: run_block_rounds<T, 4, NC>(tile, K, blk, recs); break;
+            }
+        }
+        cbar<NC>();
+        return;
+    }
     const bool plain = ctx.u == nullptr;
     const uint64_t pred = plain ? ~0ull : ctx.pred[member];
     const int64_t cur = plain ? 0 : ctx.cursor[member];
@@ -934,25 +1376,25 @@ __device__ __forceinline__ void compute_tile(T* tile, int K, const PassDesc& pd,
                 code = m ? (op.k == 1 ? kT_DENSE1 : kT_DENSE2) + (code - (op.k == 1 ? kT_MIX1 : kT_MIX2)) : -1;
             }
         }
-        recs[o] = OpRec{code, 0, m};
+        recs[o] = OpRec{code, op.zmask, m};
     }
     for (int bi = 0; bi < pd.nblocks; ++bi) {
         const BlockDesc& blk = sblk[bi];
         cbar();
-        if (blk.generic) {
-            run_ops<T>(tile, K, sops + blk.first, blk.nops, data, member, ctx);
-            continue;
+        if constexpr (MODE == kPlain) {  // passes with such blocks are launched on plain tiles
+            if (blk.generic) {
+                run_ops<T>(tile, K, sops + blk.first, blk.nops, data, member, ctx);
+                continue;
+            }
         }
-#define LSG_RUN(UU) run_block<T, UU>(tile, K, blk, recs);
+#define LSG_RUN(UU)                                                   \
+    if constexpr (MODE != kPlain) run_block_swz<T, UU, MODE == kMixed>(tile, K, blk, recs); \
+    else run_block<T, UU>(tile, K, blk, recs);
         switch (blk.u) {
             case 1: LSG_RUN(1) break;
             case 2: LSG_RUN(2) break;
             case 3: LSG_RUN(3) break;
-            default:
-                if constexpr (sizeof(T) <= 8) {
-                    LSG_RUN(4)
-                }
-                break;
+            default: LSG_RUN(4) break;
         }
 #undef LSG_RUN
     }
@@ -1001,7 +1443,7 @@ constexpr int pipe_ctas() {
 // compute side addresses the tile through the same swizzle): a pass whose chunks are 512 bytes
 // pairs chunks 2q and 2q+1 (they differ in register bit hi[0]) in one 3-D box of 1 KB; larger
 // chunks move as 2-D boxes of min(chunk, 16 KB). Otherwise one plain bulk copy per chunk.
-template <typename T, bool Swz = false, typename F>
+template <typename T, bool Swz = false, int NC = kCompute, typename F>
 __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_elems, const PassDesc& pd, T* buf0,
                                          T* buf1, uint64_t* full, uint64_t* empty, int64_t tiles_per_member,
                                          int64_t total_tiles, int* status, F&& compute, const Tmap* tmap = nullptr,
@@ -1020,9 +1462,9 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
     const int box_shift = (Swz && !pair) ? (__ffs((int)(chunk_bytes / box_bytes)) - 1) : 0;  // boxes per chunk
     const int nboxes = pair ? nchunks / 2 : nchunks << box_shift;
     const int h = pd.hi[0];  // the register bit between the two chunks of a pair
-    if (threadIdx.x >= 256) {
+    if (threadIdx.x >= NC) {
         // ---------------- producer warp
-        const int lane = threadIdx.x - 256;
+        const int lane = threadIdx.x - NC;
         auto tile_at = [&](int64_t t, T** mem, uint64_t* base) {
             const int64_t member = t / tiles_per_member;
             const uint64_t tt = (uint64_t)(t - member * tiles_per_member);
@@ -1107,21 +1549,22 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
         const int b = (int)(it & 1);
         T* tile = b ? buf1 : buf0;
         const bool ok = mbar_wait_bounded(&full[b], (uint32_t)((it >> 1) & 1), status);
-        if (cbar_or(!ok)) return;  // every compute thread leaves together on a timeout
+        if (cbar_or<NC>(!ok)) return;  // every compute thread leaves together on a timeout
         compute(tile, t / tiles_per_member);
         fence_proxy_async_smem();  // this thread's writes, before the producer's bulk store reads them
         mbar_arrive(&empty[b]);
     }
 }
 
-// Barriers of the two-buffer ring: `full` completes on the bulk loads, `empty` when all 256
-// compute threads are done with the buffer.
+// Barriers of the two-buffer ring: `full` completes on the bulk loads, `empty` when all compute
+// threads are done with the buffer.
+template <int NC = kCompute>
 __device__ __forceinline__ void pipe_init(uint64_t* full, uint64_t* empty) {
     if (threadIdx.x == 0) {
         mbar_init(&full[0], 1);
         mbar_init(&full[1], 1);
-        mbar_init(&empty[0], 256);
-        mbar_init(&empty[1], 256);
+        mbar_init(&empty[0], NC);
+        mbar_init(&empty[1], NC);
         fence_mbar_init();
     }
 }
@@ -1148,6 +1591,51 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_ctas<T>()) k_tile_pipe(T* _
     __syncthreads();
     pipe_run<T>(state, member_elems, pd, buf0, buf1, full, empty, tiles_per_member, total_tiles, status,
                 [&](T* tile, int64_t member) { compute_tile<T>(tile, pd.K, pd, sblk, sops, recs, data, member, ctx); });
+}
+
+// The same pass on tiles moved by swizzled tensor copies, the register blocks addressing them through
+// their GF(2) maps. Plain tiles of 512-byte chunks put every group of a block on low register bits
+// into the same banks (8-way conflicts: 9,700 cycles a block, where the arithmetic takes a
+// tenth); the swizzle, with the lanes driving bits that reach different banks, leaves one or two.
+template <int MODE>
+constexpr int compute_threads() {
+    return MODE == kRounds ? 128 : kCompute;
+}
+// CTAs per SM the swizzled kernels are compiled for. Lowered passes run 128 threads with 16
+// (complex128) or 32 (complex64) amplitudes each: their registers leave room for two and three CTAs.
+template <typename T, int MODE>
+constexpr int swz_ctas() {
+    return MODE == kRounds ? (sizeof(T) == 8 ? 3 : 2) : pipe_ctas<T>();
+}
+template <typename T, int MODE>
+__global__ void __launch_bounds__(compute_threads<MODE>() + 32, (swz_ctas<T, MODE>())) k_tile_pipe_swz(T* __restrict__ state, int64_t member_elems,
+                                                                   const PassDesc* __restrict__ pass_g,
+                                                                   const TileOp* __restrict__ ops,
+                                                                   const BlockDesc* __restrict__ blocks,
+                                                                   const T* __restrict__ data, int64_t tiles_per_member,
+                                                                   int64_t total_tiles, int* status, TrajCtx ctx,
+                                                                   const __grid_constant__ Tmap tmap) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ uint64_t full[2], empty[2];
+    __shared__ PassDesc pd;
+    const size_t tile_bytes = sizeof(T) << pass_g->K;
+    unsigned char* tiles = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // a swizzle atom's boundary
+    T* buf0 = reinterpret_cast<T*>(tiles);
+    T* buf1 = reinterpret_cast<T*>(tiles + tile_bytes);
+    TileOp* sops = reinterpret_cast<TileOp*>(tiles + 2 * tile_bytes);
+    BlockDesc* sblk = reinterpret_cast<BlockDesc*>(sops + pass_g->nops);
+    OpRec* recs = reinterpret_cast<OpRec*>(sblk + pass_g->nblocks);
+    if (threadIdx.x == 0) pd = *pass_g;
+    stage_pass<T>(pass_g, ops, blocks, sops, sblk);
+    uint4* staged = reinterpret_cast<uint4*>(recs + pass_g->nops);
+    pipe_init<compute_threads<MODE>()>(full, empty);
+    __syncthreads();
+    int64_t staged_member = -1;
+    pipe_run<T, true, compute_threads<MODE>()>(state, member_elems, pd, buf0, buf1, full, empty, tiles_per_member, total_tiles, status,
+                      [&](T* tile, int64_t member) {
+                          compute_tile<T, MODE>(tile, pd.K, pd, sblk, sops, recs, data, member, ctx, staged, &staged_member);
+                      },
+                      &tmap);
 }
 
 // One program's pass in a launch over several registers (circuits of uneven widths): the
