@@ -49,9 +49,23 @@ Mat mul(const Mat& x, const Mat& y) {
     return Mat{x.a * y.a + x.b * y.c, x.a * y.b + x.b * y.d, x.c * y.a + x.d * y.c, x.c * y.b + x.d * y.d};
 }
 
+// 1 / sqrt(x + y * y + z * z) with the rounding of the result beside it (one Newton step on the exact
+// residual).
+struct Exact {
+    double v, err;
+};
+Exact inverse_length(double x, double y, double z) {
+    const double yy = y * y, ye = std::fma(y, y, -yy), zz = z * z, ze = std::fma(z, z, -zz);
+    const double a = x + yy, at = a - x, ae = (x - (a - at)) + (yy - at);
+    const double h = a + zz, ht = h - a, he = (a - (h - ht)) + (zz - ht) + ae + ye + ze;
+    const double r = 1.0 / std::sqrt(h);
+    const double q = r * r, qe = std::fma(r, r, -q);
+    return Exact{r, 0.5 * r * (std::fma(-h, q, 1.0) - h * qe - he * q)};
+}
+
 // s * R * diag(1, e), R = [[1, -t], [t, 1]] or, with flip, [[t, -1], [1, t]]
 struct Rotation {
-    cd s, e;
+    cd s, s_err{0.0}, e;
     double t = 0.0, sine = 0.0;
     bool flip = false;
 };
@@ -77,6 +91,16 @@ bool rotation(const Mat& m, Rotation* out) {
     out->t = r.real();
     if (!(std::abs(r.imag()) <= kUnitary) || !(std::abs(miss) <= kUnitary * big)) return false;
     if (!(std::abs(std::abs(out->e) - 1.0) <= 1e-9)) return false;
+    // A unitary's factor s has modulus 1 / sqrt(1 + t^2): set to it beyond double precision. (Its own
+    // rounding is common to all amplitudes and the norm would drift by it: 1.6e-15 over 20 layers of
+    // 12 qubits, 4e-16 with it set.)
+    if (std::abs(std::norm(out->s) * (1.0 + out->t * out->t) - 1.0) <= 2.0 * kUnitary) {
+        const Exact u = inverse_length(0.0, out->s.real(), out->s.imag()), w = inverse_length(1.0, out->t, 0.0);
+        const double k = u.v * w.v, ke = std::fma(u.v, w.v, -k) + u.v * w.err + u.err * w.v;
+        const double re = out->s.real() * k, im = out->s.imag() * k;
+        out->s_err = cd(std::fma(out->s.real(), k, -re) + out->s.real() * ke, std::fma(out->s.imag(), k, -im) + out->s.imag() * ke);
+        out->s = cd(re, im);
+    }
     if (std::abs(out->e - 1.0) < kResidue) out->e = 1.0;
     return true;
 }
@@ -147,7 +171,7 @@ int rename_of(const TileOp& t, const double* pool, int64_t members) {
 // common to all amplitudes, so its errors would add up over the program.
 struct Factor {
     cd v{1.0}, err{0.0};
-    void operator*=(cd x) {
+    void times(cd x, cd x_err) {
         auto prod = [](double a, double b, double* e) {
             const double p = a * b;
             *e = std::fma(a, b, -p);
@@ -161,7 +185,7 @@ struct Factor {
         double e1, e2, e3, e4, e5, e6;
         const double re = sum(prod(v.real(), x.real(), &e1), -prod(v.imag(), x.imag(), &e2), &e3);
         const double im = sum(prod(v.real(), x.imag(), &e4), prod(v.imag(), x.real(), &e5), &e6);
-        err = err * x + cd(e1 - e2 + e3, e4 + e5 + e6);
+        err = err * x + v * x_err + cd(e1 - e2 + e3, e4 + e5 + e6);
         v = cd(re, im);
     }
     cd value() const { return v + err; }
@@ -346,6 +370,7 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
                     // the FP32 pair's length is not one to rounding, the same for every amplitude: a
                     // drift of the norm that the diagonal can take back
                     x.s *= h / std::hypot((double)(float)c, (double)(float)sn);
+                    x.s_err = 0.0;
                 }
             if (ok) {
                 if (open < 0 || ((in_round | touched | pend.dep) & bits)) {
@@ -369,7 +394,7 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
                     const Rotation& x = r[(size_t)b];
                     it.t[(size_t)(b * U + P)] = x.t;
                     it.second[(size_t)(b * U + P)] = whole ? x.sine : x.flip;
-                    gain[(size_t)b] *= x.s;
+                    gain[(size_t)b].times(x.s, x.s_err);
                     for (int e = 0; e < D; ++e)
                         if (e & bit(P)) {
                             if (x.e != cd(1.0)) pre.v[(size_t)(b * D + e)] *= x.e;
