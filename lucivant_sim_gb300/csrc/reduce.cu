@@ -210,61 +210,119 @@ __global__ void k_readout_flip(double* __restrict__ e, int64_t ne, int j, double
     }
 }
 
-// Re(i^ny * conj(a[i ^ x]) * a[i]) * (-1)^|i & z|: one Pauli string's summand at index i, in R
-template <typename R>
-__device__ __forceinline__ R pauli_summand(const Cx<R>* __restrict__ s, uint64_t i, uint64_t x, uint64_t z, int ny) {
-    const Cx<R> va = s[i], vb = s[i ^ x];
-    const R wr = vb.re * va.re + vb.im * va.im;  // conj(b) * a
-    const R wi = vb.re * va.im - vb.im * va.re;
-    R term = ny == 0 ? wr : ny == 1 ? -wi : ny == 2 ? -wr : wi;
-    return (__popcll(i & z) & 1) ? -term : term;
+// A block's sum by shuffles and one exchange between its warps, in a fixed order; valid in thread 0.
+__device__ __forceinline__ double block_sum_shfl(double v) {
+    __shared__ double warp[kThreads / 32];
+#pragma unroll
+    for (int off = 16; off; off >>= 1) v += __shfl_down_sync(~0u, v, off);
+    if ((threadIdx.x & 31) == 0) warp[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < kThreads / 32; ++w) v += warp[w];
+    }
+    __syncthreads();
+    return v;
 }
 
-// <P> partial sums for every member (grid.y) and term: partials[(member * nterms + t) * gridDim.x + block].
+__device__ __forceinline__ float negate_if(float v, uint32_t neg) { return __uint_as_float(__float_as_uint(v) ^ (neg << 31)); }
+__device__ __forceinline__ double negate_if(double v, uint32_t neg) {
+    return __hiloint2double(__double2hiint(v) ^ (int)(neg << 31), __double2loint(v));
+}
+
+// One Pauli string P: the summand at index i is Re(i^ny * conj(a[i ^ x]) * a[i]) * (-1)^|i & z|, the
+// real or the imaginary part of the product and a sign.
+struct PauliTerm {
+    uint64_t x, z;
+    uint32_t odd, neg;  // the imaginary part; negated
+    __device__ __forceinline__ PauliTerm(uint64_t x_, uint64_t z_) : x(x_), z(z_) {
+        const int ny = __popcll(x & z) & 3;
+        odd = ny & 1;
+        neg = ny == 1 || ny == 2;
+    }
+    __device__ __forceinline__ uint32_t sign(uint64_t i) const { return neg ^ (uint32_t)(__popcll(i & z) & 1); }
+    // two products: acc = vb.re * p + vb.im * q + acc
+    template <typename R>
+    __device__ __forceinline__ R add(Cx<R> va, Cx<R> vb, uint32_t negate, R acc) const {
+        const R p = odd ? va.im : va.re, q = odd ? -va.re : va.im;
+        acc = fma(negate_if(vb.re, negate), p, acc);
+        return fma(negate_if(vb.im, negate), q, acc);
+    }
+};
+
+// <P> partial sums, one block per (chunk of indices, member, term):
+// partials[(member * nterms + t) * gridDim.x + block].
 // Statevectors: P is Hermitian, so the summands at i and i ^ x are equal; each pair is read once,
 // from the half of the indices with x's top bit clear, and counted twice (x = 0 sums every
-// index once). Summands are formed in the register's precision and added four at a time before
-// the FP64 accumulation. Density matrices (dm_n > 0): the summands are the diagonal-block
-// entries rho[i, i ^ x], in FP64.
+// index once). complex128 takes the two FP64 operations a pair needs (both parts of the product,
+// their choice and the sum were five, the bound: 22 qubits x 20 terms 730 us). complex64 reads 16
+// bytes at a time, forms summands in FP32 and adds four before the FP64 accumulation. A block takes
+// one term: looping over the terms, each with its block-wide sum, left small registers waiting at
+// barriers (8 members of 17 qubits x 20 terms: 407 us for 8 MB).
+// Density matrices (dm_n > 0): the summands are the diagonal-block entries rho[i, i ^ x], in FP64.
+// The masks come with the launch when they are few (no copy to wait for), else from xm and zm.
+constexpr int kTermsWithLaunch = 64;
+struct TermMasks {
+    uint64_t x[kTermsWithLaunch], z[kTermsWithLaunch];
+};
+
 template <typename R>
-__global__ void k_expect(const Cx<R>* __restrict__ a, int64_t elems, int dm_n, const uint64_t* __restrict__ xm,
-                         const uint64_t* __restrict__ zm, int nterms, double* __restrict__ partials) {
+__global__ void k_expect(const Cx<R>* __restrict__ a, int64_t elems, int dm_n, const __grid_constant__ TermMasks few,
+                         const uint64_t* __restrict__ xm, const uint64_t* __restrict__ zm, int nterms,
+                         double* __restrict__ partials) {
     const int64_t member = blockIdx.y;
     const Cx<R>* s = a + member * elems;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    for (int t = 0; t < nterms; ++t) {
-        const uint64_t x = xm[t], z = zm[t];
-        const int ny = __popcll(x & z) & 3;
+    for (int t = blockIdx.z; t < nterms; t += gridDim.z) {
+        const PauliTerm term(xm ? xm[t] : few.x[t], xm ? zm[t] : few.z[t]);
         double acc = 0.0;
         if (dm_n) {
             const int64_t count = 1ll << dm_n;
             for (int64_t i = first; i < count; i += stride) {
-                const Cx<R> r = s[((uint64_t)i << dm_n) | ((uint64_t)i ^ x)];
-                const double wr = r.re, wi = r.im;
-                double term = ny == 0 ? wr : ny == 1 ? -wi : ny == 2 ? -wr : wi;
-                if (__popcll((uint64_t)i & z) & 1) term = -term;
-                acc += term;
+                const Cx<R> r = s[((uint64_t)i << dm_n) | ((uint64_t)i ^ term.x)];
+                acc += negate_if(term.odd ? (double)r.im : (double)r.re, term.sign((uint64_t)i));
             }
         } else {
-            const int h = x ? 63 - __clzll((long long)x) : 64;  // x's top bit (none for x = 0)
+            const int h = term.x ? 63 - __clzll((long long)term.x) : 64;  // x's top bit (none for x = 0)
             const uint64_t low = h < 64 ? (1ull << h) - 1 : ~0ull;
-            const int64_t count = x ? elems >> 1 : elems;
+            const int64_t count = term.x ? elems >> 1 : elems;
             auto index = [&](int64_t j) -> uint64_t {  // the j-th index with bit h clear
                 return h < 64 ? ((((uint64_t)j & ~low) << 1) | ((uint64_t)j & low)) : (uint64_t)j;
             };
-            int64_t j = first;
-            for (; j + 3 * stride < count; j += 4 * stride) {
-                R part = pauli_summand(s, index(j), x, z, ny);
-                part += pauli_summand(s, index(j + stride), x, z, ny);
-                part += pauli_summand(s, index(j + 2 * stride), x, z, ny);
-                part += pauli_summand(s, index(j + 3 * stride), x, z, ny);
-                acc += (double)part;
+            bool scalar = true;
+            // else: indices 2k, 2k + 1 and their partners in 16-byte accesses
+            if constexpr (sizeof(R) == 4) scalar = h == 0 || count < 2 || (reinterpret_cast<uintptr_t>(s) & 15) != 0;
+            if (scalar) {
+                for (int64_t j = first; j < count; j += stride) {
+                    const uint64_t i = index(j);
+                    if constexpr (sizeof(R) == 8) acc = term.add(s[i], s[i ^ term.x], term.sign(i), acc);
+                    else acc += (double)term.add(s[i], s[i ^ term.x], term.sign(i), R(0));
+                }
+            } else if constexpr (sizeof(R) == 4) {
+                const uint64_t swap = term.x & 1, xe = term.x & ~1ull;
+                const uint32_t zlow = (uint32_t)(term.z & 1);
+                auto two = [&](int64_t k, R part) -> R {
+                    const uint64_t i = index(2 * k);
+                    const float4 va = *reinterpret_cast<const float4*>(s + i);
+                    float4 vb = *reinterpret_cast<const float4*>(s + (i ^ xe));
+                    if (swap) vb = make_float4(vb.z, vb.w, vb.x, vb.y);
+                    const uint32_t neg = term.sign(i);
+                    part = term.add(Cx<R>(va.x, va.y), Cx<R>(vb.x, vb.y), neg, part);
+                    return term.add(Cx<R>(va.z, va.w), Cx<R>(vb.z, vb.w), neg ^ zlow, part);
+                };
+                const int64_t quads = count >> 1;
+                int64_t k = first;
+                for (; k + 3 * stride < quads; k += 4 * stride) {
+                    const R p0 = two(k + stride, two(k, R(0))), p1 = two(k + 3 * stride, two(k + 2 * stride, R(0)));
+                    acc += (double)p0;
+                    acc += (double)p1;
+                }
+                for (; k < quads; k += stride) acc += (double)two(k, R(0));
             }
-            for (; j < count; j += stride) acc += (double)pauli_summand(s, index(j), x, z, ny);
-            if (x) acc *= 2.0;
+            if (term.x) acc *= 2.0;
         }
-        double tot = block_sum(acc);
+        const double tot = block_sum_shfl(acc);
         if (threadIdx.x == 0) partials[(member * nterms + t) * gridDim.x + blockIdx.x] = tot;
     }
 }
@@ -638,43 +696,62 @@ int lsg_expect_pauli(lsg_state s, int dm_qubits, const uint64_t* xmask, const ui
     const int64_t member_bytes = s->elems * (s->precision == LSG_C128 ? 16 : 8);
     const int64_t chunk = dm_qubits ? kMaxGridY
                                     : std::min<int64_t>(kMaxGridY, std::max<int64_t>(1, kExpectL2Bytes / member_bytes));
-    const unsigned grid = std::max(1u, std::min(reduce_grid(count),
-                                                (unsigned)std::max<int64_t>(1, 4096 / std::min(chunk, s->batch))));
+    // A complex64 statevector made by unitary operators alone has norm one; FP32 rounding lets it drift
+    // (1e-6 over 40 layers), most of the error of an expectation. Its own norm, one more term, is
+    // divided out.
+    const bool normalise = !dm_qubits && s->precision == LSG_C64 && s->unit_norm;
+    const int terms = nterms + (normalise ? 1 : 0);
+    TermMasks few{};
+    std::vector<uint64_t> many;
+    const bool inline_masks = terms <= kTermsWithLaunch;
+    if (inline_masks) {
+        std::copy(xmask, xmask + nterms, few.x);
+        std::copy(zmask, zmask + nterms, few.z);
+    } else {
+        many.assign(2 * (size_t)terms, 0);
+        std::copy(xmask, xmask + nterms, many.begin());
+        std::copy(zmask, zmask + nterms, many.begin() + terms);
+    }
     size_t off = 0;
     auto take = [&](size_t bytes) {
         size_t at = off;
         off += (bytes + 255) & ~size_t(255);
         return at;
     };
-    const int64_t rows = (int64_t)nterms * s->batch;
-    const size_t o_x = take(nterms * 8), o_z = take(nterms * 8), o_part = take((size_t)rows * grid * 8),
-                 o_out = take((size_t)rows * 8);
+    // blocks per term and member: eight indices per thread, within a launch of some 64k blocks
+    const int64_t at_once = (int64_t)terms * std::min(chunk, s->batch);
+    const unsigned grid = (unsigned)std::max<int64_t>(
+        1, std::min<int64_t>({(count + 8 * kThreads - 1) / (8 * kThreads), 152 * 8, std::max<int64_t>(1, 65536 / at_once)}));
+    const int64_t rows = (int64_t)terms * s->batch;
+    const size_t o_m = take(many.size() * 8), o_part = take((size_t)rows * grid * 8), o_out = take((size_t)rows * 8);
     LSG_CHECK(ensure(s->scratch, off));
     char* base = (char*)s->scratch.ptr;
-    LSG_CUDA(cudaMemcpyAsync(base + o_x, xmask, nterms * 8, cudaMemcpyHostToDevice, s->stream));
-    LSG_CUDA(cudaMemcpyAsync(base + o_z, zmask, nterms * 8, cudaMemcpyHostToDevice, s->stream));
+    const uint64_t* xm = inline_masks ? nullptr : (const uint64_t*)(base + o_m);
+    if (!inline_masks)
+        LSG_CUDA(cudaMemcpyAsync(base + o_m, many.data(), many.size() * 8, cudaMemcpyHostToDevice, s->stream));
     // members go on grid y, at most 65,535 (or one L2-sized group) per launch
     for (int64_t b0 = 0; b0 < s->batch; b0 += chunk) {
         const int64_t nb = std::min<int64_t>(chunk, s->batch - b0);
-        const dim3 g2(grid, (unsigned)nb);
-        double* part = (double*)(base + o_part) + b0 * nterms * (int64_t)grid;
+        const dim3 g3(grid, (unsigned)nb, (unsigned)std::min<int64_t>(terms, kMaxGridY));
+        double* part = (double*)(base + o_part) + b0 * terms * (int64_t)grid;
         if (s->precision == LSG_C128)
-            k_expect<double><<<g2, kThreads, 0, s->stream>>>((const Cx<double>*)s->data + b0 * s->elems, s->elems,
-                                                            dm_qubits, (const uint64_t*)(base + o_x),
-                                                            (const uint64_t*)(base + o_z), nterms, part);
+            k_expect<double><<<g3, kThreads, 0, s->stream>>>((const Cx<double>*)s->data + b0 * s->elems, s->elems, dm_qubits,
+                                                            few, xm, xm ? xm + terms : nullptr, terms, part);
         else
-            k_expect<float><<<g2, kThreads, 0, s->stream>>>((const Cx<float>*)s->data + b0 * s->elems, s->elems,
-                                                           dm_qubits, (const uint64_t*)(base + o_x),
-                                                           (const uint64_t*)(base + o_z), nterms, part);
+            k_expect<float><<<g3, kThreads, 0, s->stream>>>((const Cx<float>*)s->data + b0 * s->elems, s->elems, dm_qubits,
+                                                           few, xm, xm ? xm + terms : nullptr, terms, part);
     }
-    k_sum_rows<<<(unsigned)std::min<int64_t>(rows, 152 * 16), kThreads, 0, s->stream>>>((const double*)(base + o_part), grid,
-                                                                                      rows, (double*)(base + o_out));
+    if (grid > 1)
+        k_sum_rows<<<(unsigned)std::min<int64_t>(rows, 152 * 16), kThreads, 0, s->stream>>>((const double*)(base + o_part), grid,
+                                                                                          rows, (double*)(base + o_out));
     LSG_CUDA(cudaGetLastError());
     std::vector<double> tmp((size_t)rows);
-    LSG_CUDA(cudaMemcpyAsync(tmp.data(), base + o_out, tmp.size() * 8, cudaMemcpyDeviceToHost, s->stream));
+    LSG_CUDA(cudaMemcpyAsync(tmp.data(), base + (grid > 1 ? o_out : o_part), tmp.size() * 8, cudaMemcpyDeviceToHost, s->stream));
     LSG_CUDA(cudaStreamSynchronize(s->stream));
-    for (int64_t b = 0; b < s->batch; ++b)
-        for (int t = 0; t < nterms; ++t) out[(int64_t)t * s->batch + b] = tmp[b * nterms + t];
+    for (int64_t b = 0; b < s->batch; ++b) {
+        const double norm = normalise ? tmp[b * terms + nterms] : 1.0;
+        for (int t = 0; t < nterms; ++t) out[(int64_t)t * s->batch + b] = norm > 0.0 ? tmp[b * terms + t] / norm : tmp[b * terms + t];
+    }
     return LSG_OK;
 }
 
@@ -704,6 +781,7 @@ int lsg_collapse(lsg_state s, int qubit, int outcome, double probability, int64_
     if (!s) return fail(LSG_E_ARG, "null register");
     if (qubit < 0 || qubit >= s->nbits || (outcome != 0 && outcome != 1)) return fail(LSG_E_ARG, "bad qubit or outcome");
     if (member < 0 || member >= s->batch) return fail(LSG_E_ARG, "member out of range");
+    s->unit_norm = false;
     const double div = probability > 0 ? sqrt(probability) : 1.0;
     const int do_scale = probability > 0 ? 1 : 0;
     if (s->precision == LSG_C128)
@@ -827,14 +905,14 @@ extern "C" int lsg_expect_pauli_noalloc(const void* amplitudes, int precision, i
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     LSG_CUDA(cudaMemcpyAsync(dx, xmask, (size_t)nterms * 8, cudaMemcpyHostToDevice, st));
     LSG_CUDA(cudaMemcpyAsync(dz, zmask, (size_t)nterms * 8, cudaMemcpyHostToDevice, st));
-    const dim3 g2(grid, (unsigned)batch);
+    const dim3 g2(grid, (unsigned)batch, (unsigned)std::min<int64_t>(nterms, kMaxGridY));
     const int64_t elems = 1ll << nbits;
     if (precision == LSG_C128)
-        k_expect<double><<<g2, kThreads, 0, st>>>(static_cast<const Cx<double>*>(amplitudes), elems, dm_qubits, dx, dz,
-                                                 nterms, part);
+        k_expect<double><<<g2, kThreads, 0, st>>>(static_cast<const Cx<double>*>(amplitudes), elems, dm_qubits, TermMasks{},
+                                                 dx, dz, nterms, part);
     else
-        k_expect<float><<<g2, kThreads, 0, st>>>(static_cast<const Cx<float>*>(amplitudes), elems, dm_qubits, dx, dz,
-                                                nterms, part);
+        k_expect<float><<<g2, kThreads, 0, st>>>(static_cast<const Cx<float>*>(amplitudes), elems, dm_qubits, TermMasks{},
+                                                dx, dz, nterms, part);
     k_sum_rows_to_terms<<<(unsigned)std::min<int64_t>(rows, 152 * 16), kThreads, 0, st>>>(part, grid, nterms, batch,
                                                                                         out_device);
     LSG_CUDA(cudaGetLastError());
