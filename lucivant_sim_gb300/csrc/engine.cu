@@ -970,6 +970,11 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
         delete p;
         return LSG_E_ARG;
     }
+    for (PassDesc& pd : p->plan.passes) {  // a predicate shared by the whole pass
+        pd.slot = pd.nops ? p->plan.ops[pd.first_op].pred : 0;
+        for (int o = pd.first_op; o < pd.first_op + pd.nops; ++o)
+            if (p->plan.ops[o].pred != pd.slot) pd.slot = 0;
+    }
     // real (Pauli-transfer) 4x4 operators whose first row is (1,0,0,0) for every member: trace
     // preserving; the kernel skips that row
     if (lsg_precision_real(precision))

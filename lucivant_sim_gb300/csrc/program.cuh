@@ -24,7 +24,9 @@ struct PassDesc {
     // outer[] then lists only the register bits the earlier passes can have changed, and `fix`
     // holds the basis state's values of the others.
     unsigned long long fix;
-    unsigned long long pad2;
+    // A trajectory pass whose operators all stand under one predicate (bit `slot` of a member's, not
+    // 0): tiles of members without it are not touched.
+    int slot, pad2;
 };
 
 // A register block: consecutive operators of a pass whose bits together span u <= 4 tile bits.

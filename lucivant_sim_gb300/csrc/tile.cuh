@@ -1443,11 +1443,12 @@ constexpr int pipe_ctas() {
 // compute side addresses the tile through the same swizzle): a pass whose chunks are 512 bytes
 // pairs chunks 2q and 2q+1 (they differ in register bit hi[0]) in one 3-D box of 1 KB; larger
 // chunks move as 2-D boxes of min(chunk, 16 KB). Otherwise one plain bulk copy per chunk.
+// `pred` (trajectories): members without predicate bit pd.slot are passed over by both sides.
 template <typename T, bool Swz = false, int NC = kCompute, typename F>
 __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_elems, const PassDesc& pd, T* buf0,
                                          T* buf1, uint64_t* full, uint64_t* empty, int64_t tiles_per_member,
                                          int64_t total_tiles, int* status, F&& compute, const Tmap* tmap = nullptr,
-                                         int64_t first = -1, int64_t stride = 0) {
+                                         int64_t first = -1, int64_t stride = 0, const uint64_t* pred = nullptr) {
     const int K = pd.K, L = pd.L;
     const int nchunks = 1 << (K - L);
     const uint32_t chunk_bytes = (uint32_t)(sizeof(T) << L);
@@ -1462,6 +1463,8 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
     const int box_shift = (Swz && !pair) ? (__ffs((int)(chunk_bytes / box_bytes)) - 1) : 0;  // boxes per chunk
     const int nboxes = pair ? nchunks / 2 : nchunks << box_shift;
     const int h = pd.hi[0];  // the register bit between the two chunks of a pair
+    const int slot = pred ? pd.slot : 0;
+    auto skip = [&](int64_t t) { return slot && !((pred[t / tiles_per_member] >> slot) & 1); };
     if (threadIdx.x >= NC) {
         // ---------------- producer warp
         const int lane = threadIdx.x - NC;
@@ -1505,7 +1508,9 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
             __syncwarp();
         };
         int64_t it = 0;
-        for (int64_t t = first; t < total_tiles; t += stride, ++it) {
+        int64_t held[2] = {0, 0};  // the tiles in the two buffers
+        for (int64_t t = first; t < total_tiles; t += stride) {
+            if (skip(t)) continue;
             const int b = (int)(it & 1);
             T* buf = b ? buf1 : buf0;
             if (it >= 2) {  // buffer b still holds tile it-2: wait for its compute, store it
@@ -1514,8 +1519,10 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
                     bulk_wait_all();  // our own stores in flight, then leave
                     return;
                 }
-                store(t - 2 * stride, buf);
+                store(b ? held[1] : held[0], buf);
             }
+            if (b) held[1] = t;
+            else held[0] = t;
             T* mem;
             uint64_t base;
             tile_at(t, &mem, &base);
@@ -1528,6 +1535,7 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
                     bulk_g2s(buf + ((size_t)c << L), mem + (base | deposit((uint64_t)c, pd.hi, K - L)), chunk_bytes,
                              &full[b]);
             }
+            ++it;
         }
         // the last one or two tiles
         const int64_t n_it = it;
@@ -1538,14 +1546,15 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
                 bulk_wait_all();
                 return;
             }
-            store(first + j * stride, b ? buf1 : buf0);
+            store(b ? held[1] : held[0], b ? buf1 : buf0);
         }
         bulk_wait_all();
         return;
     }
     // ---------------- compute warps
     int64_t it = 0;
-    for (int64_t t = first; t < total_tiles; t += stride, ++it) {
+    for (int64_t t = first; t < total_tiles; t += stride) {
+        if (skip(t)) continue;
         const int b = (int)(it & 1);
         T* tile = b ? buf1 : buf0;
         const bool ok = mbar_wait_bounded(&full[b], (uint32_t)((it >> 1) & 1), status);
@@ -1553,6 +1562,7 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
         compute(tile, t / tiles_per_member);
         fence_proxy_async_smem();  // this thread's writes, before the producer's bulk store reads them
         mbar_arrive(&empty[b]);
+        ++it;
     }
 }
 
@@ -1590,7 +1600,8 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_ctas<T>()) k_tile_pipe(T* _
     pipe_init(full, empty);
     __syncthreads();
     pipe_run<T>(state, member_elems, pd, buf0, buf1, full, empty, tiles_per_member, total_tiles, status,
-                [&](T* tile, int64_t member) { compute_tile<T>(tile, pd.K, pd, sblk, sops, recs, data, member, ctx); });
+                [&](T* tile, int64_t member) { compute_tile<T>(tile, pd.K, pd, sblk, sops, recs, data, member, ctx); },
+                nullptr, -1, 0, ctx.pred);
 }
 
 // The same pass on tiles moved by swizzled tensor copies, the register blocks addressing them through
@@ -1635,7 +1646,7 @@ __global__ void __launch_bounds__(compute_threads<MODE>() + 32, (swz_ctas<T, MOD
                       [&](T* tile, int64_t member) {
                           compute_tile<T, MODE>(tile, pd.K, pd, sblk, sops, recs, data, member, ctx, staged, &staged_member);
                       },
-                      &tmap);
+                      &tmap, -1, 0, ctx.pred);
 }
 
 // One program's pass in a launch over several registers (circuits of uneven widths): the
@@ -1823,6 +1834,7 @@ __global__ void __launch_bounds__(256, 3 - wide_regs<T>()) k_tile_pass(T* __rest
     uint32_t parity = 0;
     for (int64_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
         const int64_t member = t / tiles_per_member;
+        if (ctx.pred && pd.slot && !((ctx.pred[member] >> pd.slot) & 1)) continue;  // (the whole block)
         const uint64_t tt = (uint64_t)(t - member * tiles_per_member);
         T* mem = state + member * member_elems;
         const uint64_t base = deposit(tt, pd.outer, pd.nouter) | pd.fix;

@@ -48,6 +48,7 @@ struct Step {
     int64_t count = 0;  // ADVANCE: uniforms the segment drew
     // MEASURE / RESET
     int q = 0, clbit = -1, readout = 0, is_reset = 0;
+    int known = 0;  // the qubit's value was measured and no operator has changed it since
     double p01 = 0, p10 = 0;
     // KRAUS
     int k = 0, bits[2] = {0, 0}, nkraus = 0;
@@ -81,9 +82,11 @@ __device__ double t_block_sum(double v) {
 
 __device__ __forceinline__ bool has(const uint64_t* pred, int64_t b, int slot) { return (pred[b] >> slot) & 1; }
 
-__global__ void k_t_init(uint64_t* pred, uint64_t* clbits, int64_t* cursor, int64_t batch, int words, int reset_cursor) {
+__global__ void k_t_init(uint64_t* pred, uint64_t* clbits, uint64_t* last, int64_t* cursor, int64_t batch, int words,
+                         int reset_cursor) {
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
         pred[b] = 1;  // slot 0: the main line, always taken
+        last[b] = 0;
         for (int w = 0; w < words; ++w) clbits[b * words + w] = 0;
         if (reset_cursor) cursor[b] = 0;
     }
@@ -138,38 +141,55 @@ __global__ void k_t_p1(const Cx<R>* __restrict__ state, int64_t elems, int q, co
     if (threadIdx.x == 0) partials[b * gridDim.x + blockIdx.x] = tot;
 }
 
-// one thread per member: draw the outcome (and the readout flip), record the classical bit
+// Record a drawn outcome: the readout flip (the member's next uniform), the classical bit.
+__device__ __forceinline__ void record_outcome(int out, int clbit, int readout, double p01, double p10, int64_t* cursor,
+                                               const double* __restrict__ u, uint64_t* clbits) {
+    int seen = out;
+    if (readout) {
+        const double r = u[*cursor];
+        *cursor += 1;
+        if (r < (out ? p10 : p01)) seen ^= 1;
+    }
+    if (clbit >= 0) {
+        uint64_t& w = clbits[clbit >> 6];
+        const uint64_t bit = 1ull << (clbit & 63);
+        w = seen ? (w | bit) : (w & ~bit);
+    }
+}
+
+__device__ __forceinline__ void set_last(uint64_t* last, int q, int v) {
+    *last = (*last & ~(1ull << q)) | ((uint64_t)v << q);
+}
+
+// one warp per member: sum the partials, draw the outcome (and the readout flip), record the classical
+// bit and the qubit's value
 __global__ void k_t_decide(const double* __restrict__ partials, int nparts, int64_t* cursor, const double* __restrict__ u,
-                           int64_t ustride, const uint64_t* pred, int slot, int clbit, int readout, double p01,
-                           double p10, int is_reset, uint64_t* clbits, int words, int* outcome, double* prob,
-                           unsigned long long* near, int64_t batch) {
-    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
+                           int64_t ustride, const uint64_t* pred, int slot, int q, int clbit, int readout, double p01,
+                           double p10, int is_reset, uint64_t* clbits, int words, uint64_t* last, int* outcome,
+                           double* prob, unsigned long long* near, int64_t batch) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; b < batch;
+         b += ((int64_t)gridDim.x * blockDim.x) >> 5) {
         if (!has(pred, b, slot)) {
-            outcome[b] = -1;
+            if (lane == 0) outcome[b] = -1;
             continue;
         }
         double p1 = 0.0;
-        for (int g = 0; g < nparts; ++g) p1 += partials[b * nparts + g];
+        for (int g = lane; g < nparts; g += 32) p1 += partials[b * nparts + g];
+#pragma unroll
+        for (int off = 16; off; off >>= 1) p1 += __shfl_down_sync(~0u, p1, off);
+        if (lane) continue;
         p1 = fmin(fmax(p1, 0.0), 1.0);
-        const double r = u[b * ustride + cursor[b]];
-        cursor[b] += 1;
+        int64_t cur = cursor[b];
+        const double r = u[b * ustride + cur];
+        cur += 1;
         if (fabs(r - p1) < kNear) atomicAdd(near, 1ull);
-        int out = r < p1 ? 1 : 0;
+        const int out = r < p1 ? 1 : 0;
         outcome[b] = out;
         prob[b] = out ? p1 : 1.0 - p1;
-        if (!is_reset) {
-            int seen = out;
-            if (readout) {
-                const double r2 = u[b * ustride + cursor[b]];
-                cursor[b] += 1;
-                if (r2 < (out ? p10 : p01)) seen ^= 1;
-            }
-            if (clbit >= 0) {
-                uint64_t& w = clbits[b * words + (clbit >> 6)];
-                const uint64_t bit = 1ull << (clbit & 63);
-                w = seen ? (w | bit) : (w & ~bit);
-            }
-        }
+        if (!is_reset) record_outcome(out, clbit, readout, p01, p10, &cur, u + b * ustride, clbits + b * words);
+        set_last(last + b, q, is_reset ? 0 : out);
+        cursor[b] = cur;
     }
 }
 
@@ -192,9 +212,16 @@ __global__ void k_t_collapse(Cx<R>* __restrict__ state, int64_t elems, int q, co
     // complex128 divides by the FP64 norm exactly as Orrery does; complex64 multiplies by its
     // FP64 reciprocal rounded once (an FP64 division per element would bind the pass to FP64)
     const R inv = (R)(1.0 / div);
+    // (the quotient from the reciprocal and one correction by its exact remainder, Markstein 1990:
+    // three FP64 operations where the division's own sequence bound the pass)
+    auto quotient = [&](double x, double r) {
+        const double y = x * r;
+        return fma(fma(-y, div, x), r, y);
+    };
+    const double rcp = 1.0 / div;
     auto fix = [&](Cx<R> a) {
         if (!scale) return a;
-        if constexpr (sizeof(R) == 8) return Cx<R>(a.re / div, a.im / div);
+        if constexpr (sizeof(R) == 8) return Cx<R>(quotient(a.re, rcp), quotient(a.im, rcp));
         else return Cx<R>(a.re * inv, a.im * inv);
     };
     const Cx<R> zero(R(0), R(0));
@@ -354,8 +381,8 @@ __global__ void k_t_hist(const Cx<R>* __restrict__ state, int64_t elems, Group g
 // pattern << 8 (-1: not taken), prob[b] = the scale that renormalises the kept slice
 __global__ void k_t_decide_group(const double* __restrict__ partials, int nparts, int64_t* cursor,
                                  const double* __restrict__ u, int64_t ustride, const uint64_t* pred, int slot, Group gr,
-                                 uint64_t* clbits, int words, int* outcome, double* prob, unsigned long long* near,
-                                 int64_t batch) {
+                                 uint64_t* clbits, int words, uint64_t* last, int* outcome, double* prob,
+                                 unsigned long long* near, int64_t batch) {
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
         if (!has(pred, b, slot)) {
             outcome[b] = -1;
@@ -384,22 +411,38 @@ __global__ void k_t_decide_group(const double* __restrict__ partials, int nparts
             const int out = r < p1 ? 1 : 0;
             known |= 1 << i;
             val |= out << i;
+            set_last(last + b, gr.q[i], gr.is_reset[i] ? 0 : out);
             if (gr.is_reset[i]) continue;  // a reset ends with its bit at 0
             fin |= out << i;
-            int seen = out;
-            if (gr.readout[i]) {
-                const double r2 = u[b * ustride + cursor[b]];
-                cursor[b] += 1;
-                if (r2 < (out ? gr.p10[i] : gr.p01[i])) seen ^= 1;
-            }
-            if (gr.clbit[i] >= 0) {
-                uint64_t& w = clbits[b * words + (gr.clbit[i] >> 6)];
-                const uint64_t bit = 1ull << (gr.clbit[i] & 63);
-                w = seen ? (w | bit) : (w & ~bit);
-            }
+            record_outcome(out, gr.clbit[i], gr.readout[i], gr.p01[i], gr.p10[i], cursor + b, u + b * ustride, clbits + b * words);
         }
         outcome[b] = val | (fin << 8);
         prob[b] = bins[val] > 0.0 ? sqrt(total / bins[val]) : 1.0;
+    }
+}
+
+// Measurements and resets of qubits whose values are known (measured, and no operator has changed
+// them since): the outcome has probability one, so no norm is summed; each draws its uniforms as
+// ever. outcome[b] = the values | final pattern << 8, or -1 where nothing moves.
+__global__ void k_t_decide_known(int64_t* cursor, const double* __restrict__ u, int64_t ustride, const uint64_t* pred,
+                                 int slot, Group gr, uint64_t* clbits, int words, uint64_t* last, int* outcome,
+                                 double* prob, unsigned long long* near, int64_t batch) {
+    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
+        outcome[b] = -1;
+        if (!has(pred, b, slot)) continue;
+        int val = 0, fin = 0;
+        for (int i = 0; i < gr.g; ++i) {
+            const int out = (int)((last[b] >> gr.q[i]) & 1);
+            if (fabs(u[b * ustride + cursor[b]] - out) < kNear) atomicAdd(near, 1ull);
+            cursor[b] += 1;
+            val |= out << i;
+            set_last(last + b, gr.q[i], gr.is_reset[i] ? 0 : out);
+            if (gr.is_reset[i]) continue;
+            fin |= out << i;
+            record_outcome(out, gr.clbit[i], gr.readout[i], gr.p01[i], gr.p10[i], cursor + b, u + b * ustride, clbits + b * words);
+        }
+        if (val != fin) outcome[b] = val | (fin << 8);
+        prob[b] = 1.0;
     }
 }
 
@@ -637,6 +680,7 @@ struct Ctl {
     int64_t* cursor;
     uint64_t* pred;
     uint64_t* clbits;
+    uint64_t* last;  // bit q: qubit q's last measured value (0 after a reset and at the start)
     int* outcome;
     double* prob;
     int* apply;
@@ -646,7 +690,7 @@ struct Ctl {
 
 int ctl_setup(lsg_traj_s* t, int64_t batch, Ctl* c) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t need = al(batch * 8) * 2 + al(batch * 8 * t->words) + al(batch * 4) + al(batch * 8) + al(batch * 4) + 512;
+    const size_t need = al(batch * 8) * 3 + al(batch * 8 * t->words) + al(batch * 4) + al(batch * 8) + al(batch * 4) + 512;
     LSG_CHECK(ensure(t->ctl, need));
     char* p = (char*)t->ctl.ptr;
     size_t off = 0;
@@ -658,6 +702,7 @@ int ctl_setup(lsg_traj_s* t, int64_t batch, Ctl* c) {
     c->cursor = (int64_t*)take(batch * 8);
     c->pred = (uint64_t*)take(batch * 8);
     c->clbits = (uint64_t*)take(batch * 8 * t->words);
+    c->last = (uint64_t*)take(batch * 8);
     c->outcome = (int*)take(batch * 4);
     c->prob = (double*)take(batch * 8);
     c->apply = (int*)take(batch * 4);
@@ -675,10 +720,19 @@ int group_length(const std::vector<Step>& steps, size_t si) {
     uint64_t seen = 0;
     for (size_t j = si; j < steps.size() && n < kGroupMax; ++j, ++n) {
         const Step& m = steps[j];
-        if (m.kind != STEP_MEASURE || m.slot != steps[si].slot || ((seen >> m.q) & 1)) break;
+        if (m.kind != STEP_MEASURE || m.slot != steps[si].slot || m.known != steps[si].known || ((seen >> m.q) & 1)) break;
         seen |= 1ull << m.q;
     }
     return std::max(n, 1);
+}
+
+// Blocks per member of the reductions and collapses: four amplitude pairs per thread when there are
+// members enough to fill the device, one for a single shot (13 qubits: 16 blocks in place of 4; its
+// collapse, 15 us of FP64 on 4 SMs, takes 4).
+int64_t reduce_blocks(int64_t batch, int64_t elems) {
+    const int64_t per = batch > 16 ? 4 : 1;
+    return std::max<int64_t>(1, std::min<int64_t>({((elems >> 1) + kT * per - 1) / (kT * per), batch > 16 ? 8192 : 304,
+                                                   std::max<int64_t>(1, 8192 / batch)}));
 }
 
 template <typename R>
@@ -693,8 +747,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
     ctx.ustride = ustride;
     ctx.cursor = c.cursor;
     ctx.pred = c.pred;
-    const unsigned gx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(((elems >> 1) + kT * 4 - 1) / (kT * 4),
-                                                                          std::max<int64_t>(1, 8192 / B)));
+    const unsigned gx = (unsigned)reduce_blocks(B, elems);
     bool p1_ready = false;  // the current step's p(1) partials were accumulated by the previous collapse
     for (size_t si = 0; si < t->steps.size(); ++si) {
         const Step& sp = t->steps[si];
@@ -706,8 +759,8 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                 break;
             case STEP_MEASURE: {
                 double* part = (double*)t->parts.ptr;
-                const int glen = B > 1 ? group_length(t->steps, si) : 1;
-                if (glen > 1) {  // this measurement and the next glen-1 as one group
+                const int glen = B > 1 || sp.known ? group_length(t->steps, si) : 1;
+                if (glen > 1 || sp.known) {  // this measurement and the next glen-1 as one group
                     Group gr;
                     gr.g = glen;
                     for (int i = 0; i < glen; ++i) {
@@ -719,21 +772,32 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                         gr.p01[i] = m.p01;
                         gr.p10[i] = m.p10;
                     }
-                    k_t_hist<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, gr, c.pred, sp.slot, part);
-                    k_t_decide_group<<<t_grid(B), kT, 0, st>>>(part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, gr,
-                                                              c.clbits, t->words, c.outcome, c.prob, c.near, B);
+                    if (sp.known) {
+                        k_t_decide_known<<<t_grid(B), kT, 0, st>>>(c.cursor, u, ustride, c.pred, sp.slot, gr, c.clbits, t->words,
+                                                                  c.last, c.outcome, c.prob, c.near, B);
+                        bool moves = false;  // only a reset of a 1 moves amplitudes
+                        for (int i = 0; i < glen; ++i) moves = moves || gr.is_reset[i];
+                        if (!moves) {
+                            si += glen - 1;
+                            break;
+                        }
+                    } else {
+                        k_t_hist<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, gr, c.pred, sp.slot, part);
+                        k_t_decide_group<<<t_grid(B), kT, 0, st>>>(part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, gr,
+                                                                  c.clbits, t->words, c.last, c.outcome, c.prob, c.near, B);
+                    }
                     k_t_collapse_group<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, gr, c.outcome, c.prob);
                     si += glen - 1;
                     break;
                 }
                 if (!p1_ready)
                     k_t_p1<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.q, c.pred, sp.slot, part);
-                k_t_decide<<<t_grid(B), kT, 0, st>>>(part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.clbit,
-                                                    sp.readout, sp.p01, sp.p10, sp.is_reset, c.clbits, t->words,
-                                                    c.outcome, c.prob, c.near, B);
+                k_t_decide<<<t_grid(B * 32), kT, 0, st>>>(part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.q, sp.clbit,
+                                                         sp.readout, sp.p01, sp.p10, sp.is_reset, c.clbits, t->words, c.last,
+                                                         c.outcome, c.prob, c.near, B);
                 // a measurement right after this one: its p(1) partials come out of this collapse
                 const Step* nx = si + 1 < t->steps.size() ? &t->steps[si + 1] : nullptr;
-                const bool fuse = nx && nx->kind == STEP_MEASURE && (B == 1 || group_length(t->steps, si + 1) == 1);
+                const bool fuse = nx && nx->kind == STEP_MEASURE && !nx->known && (B == 1 || group_length(t->steps, si + 1) == 1);
                 k_t_collapse<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.q, c.outcome, c.prob, sp.is_reset,
                                                                     fuse ? nx->q : -1, c.pred, fuse ? nx->slot : 0, part);
                 next_p1_ready = fuse;
@@ -741,9 +805,11 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
             }
             case STEP_KRAUS: {
                 double* part = (double*)t->parts.ptr;
-                k_t_rdm<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.k, sp.bits[0], sp.bits[1], c.pred,
+                // one thread adds a member's partial matrices: as few as a batch has
+                const unsigned gk = B > 16 ? gx : (gx + 3) / 4;
+                k_t_rdm<R><<<dim3(gk, (unsigned)B), kT, 0, st>>>(state, elems, sp.k, sp.bits[0], sp.bits[1], c.pred,
                                                                sp.slot, part);
-                k_t_kraus_decide<R><<<t_grid(B), kT, 0, st>>>(part, (int)gx, sp.k, (const double*)t->kraus.ptr + 2 * sp.kraus_at,
+                k_t_kraus_decide<R><<<t_grid(B), kT, 0, st>>>(part, (int)gk, sp.k, (const double*)t->kraus.ptr + 2 * sp.kraus_at,
                                                              sp.nkraus, c.cursor, u, ustride, c.pred, sp.slot,
                                                              (Cx<R>*)t->dyn.ptr, c.apply, c.near, B);
                 k_t_apply_dyn<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.k, sp.bits[0], sp.bits[1],
@@ -768,8 +834,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
 }
 
 int parts_setup(lsg_traj_s* t, int64_t batch, int64_t elems) {
-    const int64_t gx = std::max<int64_t>(1, std::min<int64_t>(((elems >> 1) + kT * 4 - 1) / (kT * 4),
-                                                              std::max<int64_t>(1, 8192 / batch)));
+    const int64_t gx = reduce_blocks(batch, elems);
     return ensure(t->parts, (size_t)(batch * gx * 32 + 64) * 8);
 }
 
@@ -805,6 +870,10 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
     std::vector<Frame> stack;
     int slot = 0;
     int64_t draws = 0;  // upper bound along the current path
+    // qubits whose value every member knows (all of them are 0 at the start), on the main line: a
+    // measurement or reset makes one known, an operator that is not diagonal (or a channel) on it,
+    // on any branch, ends that
+    uint64_t known = nbits >= 64 ? ~0ull : (1ull << nbits) - 1;
     auto fail_out = [&](int code) {
         delete t;
         return code;
@@ -858,6 +927,8 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
             else if (o.kind == kOpMixture) need = op.count + op.count * d * d;
             if (op.data < 0 || op.data + need > pool_entries)
                 return fail_out(fail(LSG_E_ARG, "trajectory op %d reads outside the pool", i));
+            if (o.kind != LSG_OP_DIAG)
+                for (int j = 0; j < o.nbits; ++j) known &= ~(1ull << o.bits[j]);
             seg_ops.push_back(o);
             seg_pred.push_back(slot);
             seg_draw.push_back(op.kind == LSG_T_MIXTURE ? (int)seg_draws : 0);
@@ -885,6 +956,10 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
                 sp.readout = op.kind == LSG_T_MEASURE && op.readout;
                 sp.p01 = op.p01;
                 sp.p10 = op.p10;
+                sp.known = slot == 0 && ((known >> sp.q) & 1);
+                // under a branch only some members measure it: what the others hold stays unknown
+                if (slot == 0) known |= 1ull << sp.q;
+                else if (!((known >> sp.q) & 1)) known &= ~(1ull << sp.q);
                 draws += 1 + sp.readout;
                 t->steps.push_back(sp);
                 break;
@@ -893,8 +968,10 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
                 const int64_t d = 1ll << op.nq;
                 if (op.data < 0 || op.data + op.count * d * d > pool_entries)
                     return fail_out(fail(LSG_E_ARG, "op %d reads outside the pool", i));
-                for (int j = 0; j < op.nq; ++j)
+                for (int j = 0; j < op.nq; ++j) {
                     if (op.qubits[j] < 0 || op.qubits[j] >= nbits) return fail_out(fail(LSG_E_ARG, "op %d: bad qubit", i));
+                    known &= ~(1ull << op.qubits[j]);
+                }
                 sp.kind = STEP_KRAUS;
                 sp.k = op.nq;
                 sp.bits[0] = op.qubits[0];
@@ -994,7 +1071,7 @@ int lsg_traj_run_batched(lsg_traj t, lsg_state s, const double* uniforms, int64_
         k_t_basis<double><<<t_grid(n), kT, 0, s->stream>>>((Cx<double>*)s->data, s->elems, n);
     else
         k_t_basis<float><<<t_grid(n), kT, 0, s->stream>>>((Cx<float>*)s->data, s->elems, n);
-    k_t_init<<<t_grid(B), kT, 0, s->stream>>>(c.pred, c.clbits, c.cursor, B, t->words, 1);
+    k_t_init<<<t_grid(B), kT, 0, s->stream>>>(c.pred, c.clbits, c.last, c.cursor, B, t->words, 1);
     LSG_CUDA(cudaGetLastError());
     int rc = s->precision == LSG_C128 ? run_steps<double>(t, s, c, (const double*)t->ubuf.ptr, ustride)
                                       : run_steps<float>(t, s, c, (const double*)t->ubuf.ptr, ustride);
@@ -1038,7 +1115,7 @@ int lsg_traj_run_serial(lsg_traj t, lsg_state s, int64_t shots, const double* un
             k_t_basis<double><<<t_grid(s->elems), kT, 0, s->stream>>>((Cx<double>*)s->data, s->elems, s->elems);
         else
             k_t_basis<float><<<t_grid(s->elems), kT, 0, s->stream>>>((Cx<float>*)s->data, s->elems, s->elems);
-        k_t_init<<<1, 32, 0, s->stream>>>(c.pred, c.clbits, c.cursor, 1, t->words, 0);
+        k_t_init<<<1, 32, 0, s->stream>>>(c.pred, c.clbits, c.last, c.cursor, 1, t->words, 0);
         int rc = s->precision == LSG_C128 ? run_steps<double>(t, s, c, u, 0) : run_steps<float>(t, s, c, u, 0);
         if (rc != LSG_OK) return rc;
         k_t_record<<<1, 32, 0, s->stream>>>(c.clbits, t->words, (uint64_t*)t->results.ptr, c.shot);
