@@ -453,13 +453,14 @@ Plan plan_ops(const lsg_op* ops, int nops, int nbits, int K, int L, const int* p
 // Widest register block: 16 elements per thread. A complex register of 2^10 amplitudes or fewer is
 // one tile on one SM: narrower blocks keep more of its lanes at work (8 qubits, complex128, 4
 // layers: 82 us in 4-bit blocks, 56 in 3-bit, 36 in 2-bit ones; 10 qubits: 105, 69, 75; 11: 114,
-// 130, 138). Trajectory segments (not lowered) of complex128 take 8 amplitudes per thread, as many
-// groups as the kernel has threads.
-int block_bits_for(int precision, int nbits, bool lowered) {
+// 130, 138). Complex128 trajectory segments take 8 amplitudes per thread: on small registers twice the
+// threads at work (13 qubits, 40 serial shots: 31.9 ms in 4-bit blocks, 26.7 in 3-bit ones), equal on
+// large ones.
+int block_bits_for(int precision, int nbits, bool trajectory) {
     const int top = 4;
     int u = top;
     if (!lsg_precision_real(precision)) u = std::max(2, std::min(top, nbits - 7));
-    if (precision == LSG_C128 && !lowered) u = std::min(u, 3);
+    if (precision == LSG_C128 && trajectory) u = std::min(u, 3);
     if (const char* env = getenv("LSG_BLOCK_BITS")) u = atoi(env);
     return std::max(0, std::min(u, top));
 }
@@ -954,16 +955,29 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     p->unitary = precision == LSG_C64 && !pred && !draw && !count && ops_unitary(ops, nops, pool, batch);
     p->dev.stream = stream;
     p->K = tile_bits_for(nbits, precision);
+    // Complex128 trajectory segments on half tiles while every half has an SM to itself: the passes
+    // are bound by one tile's time (20 shots serial x 6 rounds: 13 qubits 15.7 -> 13.4 ms, 16 qubits
+    // 18.8 -> 16.8; 18 qubits, 128 tiles, 23.6 -> 25.4).
+    const int full_bits = p->K;
+    const bool trajectory = pred || draw || count;
+    if (trajectory && precision == LSG_C128 && !t_choice.tile_bits && !getenv("LSG_TILE_BITS") && p->K > 10 &&
+        nbits - p->K < 16 && (batch << (nbits - p->K + 1)) <= 152)
+        --p->K;
     const int L = std::min(p->K, low_bits_for(nbits, precision));
     if (nops > 0) {
-        p->plan = preplanned ? *preplanned : plan_ops(ops, nops, nbits, p->K, L, pred, draw, count, block_bits_for(precision, nbits, !pred && !draw && !count));
+        const int umax = block_bits_for(precision, nbits, trajectory);
+        p->plan = preplanned ? *preplanned : plan_ops(ops, nops, nbits, p->K, L, pred, draw, count, umax);
+        if (p->plan.passes.empty() && p->K < full_bits) {  // an operator wider than the half tile
+            p->K = full_bits;
+            p->plan = plan_ops(ops, nops, nbits, p->K, L, pred, draw, count, umax);
+        }
         if (upload && !pred && !draw && !count) {
             p->src_ops.assign(ops, ops + nops);
             p->raw_plan = p->plan;
         }
         if (p->plan.passes.empty()) {
             delete p;
-            return fail(LSG_E_ARG, "an operator does not fit a tile of %d bits (%d kept low)", tile_bits_for(nbits, precision), L);
+            return fail(LSG_E_ARG, "an operator does not fit a tile of %d bits (%d kept low)", p->K, L);
         }
     }
     if (check_plan(p->plan) != LSG_OK) {
@@ -1012,11 +1026,13 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     }
     if (!pred && !draw && !count) p->core_plan = p->plan;
     // Complex programs: outer factors of one-bit operators move on to the next ones, so that blocks
-    // lower to rounds (lower.cu). Trajectory segments keep their operators: each has its own
-    // predicate and draws.
+    // lower to rounds (lower.cu). So do complex128 trajectory segments, whose operators all stand under
+    // one predicate; complex64 ones, not bound by arithmetic, keep their operators.
     const char* fuse_env = getenv("LSG_FUSE_BLOCKS");
     const bool fuse = !lsg_precision_real(precision) && !(fuse_env && fuse_env[0] == '0');
-    const bool rounds = fuse && !pred && !draw && !count;
+    bool rounds = fuse && ((!pred && !draw && !count) || precision == LSG_C128);
+    const int seg_pred = pred && nops > 0 ? pred[0] : 0;
+    for (int32_t i = 0; pred && i < nops; ++i) rounds = rounds && pred[i] == seg_pred;
     std::vector<double> grown;
     std::vector<char> moved;
     if (rounds && nops > 0) {
@@ -1079,6 +1095,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                         f.stride = low.members > 1 ? stride : 0;
                         f.tmpl = it.code;
                         f.zmask = it.mask;
+                        f.pred = seg_pred;
                         for (int64_t b = 0; b < low.members; ++b) {
                             const size_t end = ext.size() + 2 * (size_t)stride;
                             for (int e = 0; e < D; ++e) {
@@ -2217,7 +2234,7 @@ int lsg_plan(int nbits, int precision, const lsg_op* ops, int32_t nops, int32_t*
         if (!op_bits_ok(ops[i], nbits)) return fail(LSG_E_ARG, "operator %d has a bad kind or bits", i);
     const int K = tile_bits_for(nbits, precision);
     const int L = std::min(K, low_bits_for(nbits, precision));
-    Plan plan = plan_passes(ops, nops, nbits, K, L, block_bits_for(precision, nbits, true));
+    Plan plan = plan_passes(ops, nops, nbits, K, L, block_bits_for(precision, nbits, false));
     if (nops > 0 && plan.passes.empty()) return fail(LSG_E_ARG, "an operator does not fit a tile of %d bits", K);
     LSG_CHECK(check_plan(plan));
     *passes = (int32_t)plan.passes.size();

@@ -330,6 +330,25 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
         }
         open = -1;
     };
+    // Mixtures (a member's branch of a noise channel, nearly always the identity) wait: they commute
+    // with what follows on other bits, so a block's channels share the one diagonal before them.
+    std::vector<int> late;
+    unsigned late_bits = 0;
+    auto keep = [&](int o, int code) {
+        LoweredItem it;
+        it.code = kKeepOp;
+        it.op = o;
+        it.tmpl = code;
+        out->items.push_back(std::move(it));
+    };
+    auto flush_late = [&] {
+        if (late.empty()) return;
+        if (pend.dep & late_bits) emit_diag(pend);
+        for (int o : late) keep(o, plan.ops[(size_t)o].tmpl);
+        touched |= late_bits;
+        late.clear();
+        late_bits = 0;
+    };
     auto permute = [&](int code) {  // the rename moves the diagonal that stands before it
         auto src = [&](int e) {
             if (code < kT_CX) return e ^ bit(code - kT_X1);
@@ -347,6 +366,13 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
         const TileOp& t = plan.ops[(size_t)o];
         unsigned bits = 0;
         for (int i = 0; i < t.k; ++i) bits |= 1u << t.pos[i];
+        if (bits & late_bits) flush_late();
+        if (t.kind == kOpMixture) {
+            late.push_back(o);
+            late_bits |= bits;
+            cost += 0.25 + overhead;
+            continue;
+        }
         if (is_dense1(t)) {
             const int P = t.pos[0];
             std::vector<Rotation> r((size_t)members);
@@ -441,12 +467,9 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
             cost += (t.kind == LSG_OP_PERM ? 1.0 : t.k == 1 ? 2.0 : 4.0) + overhead;
         }
         touched |= bits;
-        LoweredItem it;
-        it.code = kKeepOp;
-        it.op = o;
-        it.tmpl = code >= 0 ? code : t.tmpl;
-        out->items.push_back(std::move(it));
+        keep(o, code >= 0 ? code : t.tmpl);
     }
+    flush_late();
     close(true);
     // A diagonal left over: by structure (whether the block is lowered is the same for every member's
     // data), emitted when some member's is not one.
