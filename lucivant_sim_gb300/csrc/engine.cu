@@ -21,6 +21,7 @@
 #include "jit.cuh"
 #include "kernels.cuh"
 #include "lower.cuh"
+#include "transfer.cuh"
 #include "program.cuh"
 #include "tile.cuh"
 
@@ -1041,6 +1042,16 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
         pool = grown.data();
         pool_entries = (int64_t)grown.size() / 2;
     }
+    // Real64 programs: one-qubit transfer operators as shears (transfer.cu). The other real elements keep
+    // their products: real32 passes are bound by memory, and a double-float shear would renormalise
+    // every coefficient twice where a row of products does once.
+    const bool transfer = precision == LSG_R64 && !pred && !draw && !count && !(fuse_env && fuse_env[0] == '0');
+    if (transfer && nops > 0) {
+        grown.assign(pool, pool + 2 * pool_entries);
+        move_outer_rotations(p->plan, batch, grown);
+        pool = grown.data();
+        pool_entries = (int64_t)grown.size() / 2;
+    }
     // Register-block operator data, copied once here into an extension of the pool: diagonals
     // re-indexed in block order (the kernel multiplies v[e] by m[e] with no index arithmetic), and
     // dense matrices, diagonals and mixture matrices placed on 16-byte boundaries (the kernel reads
@@ -1114,6 +1125,42 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                     std::copy(made.begin(), made.end(), p->plan.ops.begin() + pd.first_op + blk.first);
                     blk.nops = (int)made.size();
                 }
+            }
+            std::vector<TransferItem> shears;
+            int64_t shear_members = 1;
+            if (transfer && lower_transfer_block(p->plan, pd, blk, batch, pool, &shears, &shear_members)) {
+                std::vector<TileOp> made;
+                for (const TransferItem& it : shears) {
+                    if (it.op >= 0) {
+                        made.push_back(p->plan.ops[it.op]);
+                        continue;
+                    }
+                    const bool diag = it.mask < 0;
+                    const int64_t len = diag ? (int64_t)1 << blk.u : kTransferLen, stride = round_up(len);
+                    pad_ext(0);
+                    TileOp f{};
+                    f.kind = diag ? LSG_OP_DIAG : LSG_OP_MATRIX;
+                    f.k = diag ? blk.u : 2;
+                    for (int i = 0; i < f.k; ++i) {
+                        f.pos[i] = diag ? i : it.pos[i];
+                        f.lb[i] = blk.bits[f.pos[i]];
+                        f.sorted[i] = diag ? blk.sorted[i] : 0;
+                    }
+                    if (!diag) f.sorted[0] = std::min(f.lb[0], f.lb[1]), f.sorted[1] = std::max(f.lb[0], f.lb[1]);
+                    f.data = pool_entries + (int64_t)ext.size() / 2;
+                    f.stride = shear_members > 1 ? stride : 0;
+                    f.tmpl = diag ? kT_DIAGB : kT_ROUND;
+                    // (whether a member exchanges a pair stays out of the code: it changes with the angles)
+                    f.zmask = diag ? 0 : it.pos[0] + 4 * it.pos[1] + 16 * (it.mask & ~(kTrFlipV | kTrFlipW | kTrFlipS));
+                    for (int64_t b = 0; b < shear_members; ++b) {
+                        const size_t end = ext.size() + 2 * (size_t)stride;
+                        for (int64_t e = 0; e < len; ++e) ext.insert(ext.end(), {it.v[(size_t)(b * len + e)], 0.0});
+                        ext.resize(end, 0.0);
+                    }
+                    made.push_back(f);
+                }
+                std::copy(made.begin(), made.end(), p->plan.ops.begin() + pd.first_op + blk.first);
+                blk.nops = (int)made.size();
             }
             if (fuse && blk.u >= 2 && blk.nops > 1) {
                 const int U = blk.u, D = 1 << U;
@@ -1244,7 +1291,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 const BlockDesc& b = p->plan.blocks[bi];
                 for (int o = pd.first_op + b.first; o < pd.first_op + b.first + b.nops; ++o) {
                     const TileOp& t = p->plan.ops[o];
-                    any = any || t.tmpl == kT_ROUND;
+                    any = any || (t.tmpl == kT_ROUND && !lsg_precision_real(precision));
                     lowered = lowered && t.pred == 0 && (t.tmpl == kT_ROUND || (t.tmpl >= kT_X1 && t.tmpl < kT_SWAP + 16));
                 }
             }
@@ -2143,6 +2190,11 @@ static double op_flops_per_element(const lsg::TileOp& op, bool complex_elems, bo
     }
     if ((c >= kT_PERM1 && c < kT_PERM1 + 4) || (c >= kT_PERM2 && c < kT_PERM2 + 16)) return mul;
     if (c == kT_DIAGB || c == kT_SCALE || c == kT_DIAG) return mul;
+    if (c == kT_ROUND && !complex_elems) {  // two multiply-adds per pair of four coefficients, a shift one or two
+        const int parts = op.zmask >> 4;
+        return (double)(!!(parts & kTrV) + !!(parts & kTrW) + !!(parts & kTrS)) + (parts & kTrShiftZ ? 0.5 : 0.0) +
+               (parts & kTrShiftXY ? 1.0 : 0.0);
+    }
     if (c == kT_ROUND)
         return (op.zmask & 16 ? 6.0 : 0.0) + (whole ? 6.0 : 4.0) * __builtin_popcount((unsigned)op.zmask & 15u);
     if (c == kT_DENSEB) return (complex_elems ? 8.0 : 2.0) * (double)(1 << op.k);

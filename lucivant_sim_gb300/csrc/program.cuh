@@ -107,8 +107,13 @@ constexpr int kT_CX = 79;       // + 4 * Pcontrol + Ptarget: unit-phase CX (regi
 constexpr int kT_SWAP = 95;     // + 4 * P0 + P1
 constexpr int kT_DENSEB = 111;  // a whole register block as one dense 2^u x 2^u complex matrix (block order)
 constexpr int kT_ROUND = 112;   // a diagonal over the block, then real rotations on its bits (complex; rb_round);
-                                // zmask: bit P a rotation on position P, bit 4 the diagonal
+                                // zmask: bit P a rotation on position P, bit 4 the diagonal.
+                                // real64: a one-qubit transfer operator as shears (rb_transfer); zmask:
+                                // positions P0 + 4 * P1, then 16 * the kTr* parts some member has
 constexpr int kT_CODES = 113;   // the kernel's codes are exactly 0 .. kT_CODES-1 (a dense switch)
+// parts of a transfer operator: the pair maps V, W, S, their exchanges, its shifts, dense rows instead
+constexpr int kTrV = 1, kTrW = 2, kTrS = 4, kTrFlipV = 8, kTrFlipW = 16, kTrFlipS = 32;
+constexpr int kTrShiftZ = 64, kTrShiftXY = 128, kTrDense = 256;
 // host-side markers, rewritten before upload: mixtures become dense codes per member in the kernel,
 // diagonals become kT_DIAGB
 constexpr int kT_MIX1 = 113;    // + P

@@ -482,8 +482,72 @@ __device__ __forceinline__ void rb_rotate_flip(Cx<double>& x, Cx<double>& y, dou
     y = Cx<double>(fma(t, b.re, a.re), fma(t, b.im, a.im));
 }
 
+// One pair map of a transfer operator: (x, y) exchanged when `flip`, then x + p * y and y + q * x.
+template <int U, int B0, int B1, int RX, int RY>
+__device__ __forceinline__ void rb_shears(double* v, double p, double q, bool flip) {
+    if (flip) {
+#pragma unroll
+        for (int e = 0; e < (1 << U); ++e) {
+            if (e & (B0 | B1)) continue;
+            const double x = v[e | RY], y = v[e | RX];
+            v[e | RX] = fma(p, y, x);
+            v[e | RY] = fma(q, x, y);
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < (1 << U); ++e) {
+            if (e & (B0 | B1)) continue;
+            const double x = v[e | RX], y = v[e | RY];
+            v[e | RX] = fma(p, y, x);
+            v[e | RY] = fma(q, x, y);
+        }
+    }
+}
+
+// A trace-preserving transfer operator of one qubit (digits I, Z, X, Y on positions P0, P1) as shears:
+// m = (parts, shift of Y, V, W, S, shifts of Z and X, dense rows 1-3); `all`: the parts some member has.
+template <int U, int P0, int P1>
+__device__ __forceinline__ void rb_transfer(double* v, const double* m, int all) {
+    constexpr int B0 = 1 << (U - 1 - P0), B1 = 1 << (U - 1 - P1);
+    double c[10];
+    ldv<double, 10>(m, c);
+    const int parts = (int)c[0];
+    if ((all & kTrDense) && (parts & kTrDense)) {
+        rb_tpd2<double, U, P0, P1>(v, m + 6);  // (reads its rows from entry 4 on)
+        return;
+    }
+    if (parts & kTrV) rb_shears<U, B0, B1, B0, B0 | B1>(v, c[2], c[3], parts & kTrFlipV);
+    if (parts & kTrW) rb_shears<U, B0, B1, B0, B1>(v, c[4], c[5], parts & kTrFlipW);
+    if ((all & kTrS) && (parts & kTrS)) rb_shears<U, B0, B1, B0, B0 | B1>(v, c[6], c[7], parts & kTrFlipS);
+    if ((all & kTrShiftZ) && (parts & kTrShiftZ)) {
+#pragma unroll
+        for (int e = 0; e < (1 << U); ++e)
+            if (!(e & (B0 | B1))) v[e | B1] = fma(c[8], v[e], v[e | B1]);
+    }
+    if ((all & kTrShiftXY) && (parts & kTrShiftXY)) {
+#pragma unroll
+        for (int e = 0; e < (1 << U); ++e) {
+            if (e & (B0 | B1)) continue;
+            v[e | B0] = fma(c[9], v[e], v[e | B0]);
+            v[e | B0 | B1] = fma(c[1], v[e], v[e | B0 | B1]);
+        }
+    }
+}
+
+template <int U, int P0, int P1>
+__device__ __forceinline__ void rb_transfer_at(double* v, const double* m, int mask) {
+    if constexpr (P0 < U && P1 < U && P0 != P1)
+        if ((mask & 15) == P0 + 4 * P1) rb_transfer<U, P0, P1>(v, m, mask >> 4);
+}
+
 template <typename T, int U>
 __device__ __forceinline__ void rb_round(T* v, const T* m, int mask) {
+    if constexpr (!Elem<T>::complex && !IsDF<T>::value && sizeof(T) == 8) {
+        rb_transfer_at<U, 0, 1>(v, m, mask), rb_transfer_at<U, 0, 2>(v, m, mask), rb_transfer_at<U, 0, 3>(v, m, mask);
+        rb_transfer_at<U, 1, 0>(v, m, mask), rb_transfer_at<U, 1, 2>(v, m, mask), rb_transfer_at<U, 1, 3>(v, m, mask);
+        rb_transfer_at<U, 2, 0>(v, m, mask), rb_transfer_at<U, 2, 1>(v, m, mask), rb_transfer_at<U, 2, 3>(v, m, mask);
+        rb_transfer_at<U, 3, 0>(v, m, mask), rb_transfer_at<U, 3, 1>(v, m, mask), rb_transfer_at<U, 3, 2>(v, m, mask);
+    }
     if constexpr (Elem<T>::complex) {
         constexpr int D = 1 << U, ND = sizeof(T) == 8 ? 2 * D : D;
         T rot[U];  // read ahead of the diagonal's arithmetic (a diagonal alone has none)
@@ -917,7 +981,7 @@ __device__ __forceinline__ void rb_apply(T* v, int code, int mask, const T* m) {
         case kT_DIAGB: rb_diagb<T, U>(v, m); break;
         case kT_SCALE: rb_scale<T, U>(v, m); break;
         case kT_ROUND:
-            if constexpr (ROUNDS) rb_round<T, U>(v, m, mask);
+            if constexpr (ROUNDS || !Elem<T>::complex) rb_round<T, U>(v, m, mask);
             break;
         default: break;
     }
