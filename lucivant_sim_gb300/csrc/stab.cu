@@ -299,248 +299,140 @@ __global__ void k_elim_xor(uint64_t* __restrict__ m, uint8_t* __restrict__ rhs, 
     }
 }
 
-// ---- support() in one launch: a thread-block cluster holds the n stabilizer rows in its CTAs'
-// shared memory (rows split evenly over the CTAs, a contiguous run of rows per warp) and walks
-// the columns with one cluster barrier each. Per column every warp offers its lowest eligible row
-// (atomicMin into its CTA's candidate slot), the cluster's minimum is read from every CTA's slot
-// over distributed shared memory, each warp loads the pivot row from the owning CTA into
-// registers and combines it into its own rows that have the bit. The X phase (pivots with the
-// phase rowsum, stabilizer.py:371-395) is followed by the Z phase on the rows no X pivot took
-// (plain GF(2) elimination with the signs as right-hand side, stabilizer.py:398-422).
+// ---- support() in panels of 64 columns, two launches each. The pivots of a panel depend only on its
+// one word per row and on which rows are taken, so one CTA walks its columns on the rows' words in
+// shared memory, a barrier a column, and notes for every row the set of pivot rows multiplied onto it
+// (64 bits: pivot rows as they stood when the panel began; stabilizer rows commute, so neither a
+// product's words nor its sign depend on the order). Then all SMs form the products, a warp per row.
+// The X phase (pivots with the phase rowsum, stabilizer.py:371-395) is followed by the Z phase on
+// the rows no X pivot took (plain GF(2) elimination with the signs as right-hand side,
+// stabilizer.py:398-422). A column then costs a barrier and a few shared-memory reads of one CTA
+// where a cluster that held the rows exchanged a pivot row per column.
 
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ int cluster_ctarank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return (int)r;
-}
-__device__ __forceinline__ int cluster_nctarank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return (int)r;
-}
-// the address of `p` (this CTA's shared memory) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t dsmem_map(const void* p, int rank) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ uint64_t dsmem_u64(uint32_t a) {
-    uint64_t v;
-    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ int dsmem_s32(uint32_t a) {
-    int v;
-    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ int dsmem_u8(uint32_t a) {
-    unsigned v;
-    asm volatile("ld.shared::cluster.u8 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-    return (int)v;
-}
-
-constexpr int kSupThreads = 1024;
-constexpr int kSupWarps = kSupThreads / 32;
-constexpr int kSupMaxCluster = 8;
-constexpr int kSupRowsPerCta = 256;
+constexpr int kPanelThreads = 1024;
 
 struct SupArgs {
     uint64_t* sx;  // n rows x W words, row-major: in, the stabilizer rows; out, reduced
     uint64_t* sz;
     uint8_t* sr;
-    uint8_t* used;  // out: rows taken as X pivots
-    int* pivots;    // out: the X pivot rows in column order
-    int* zcol;      // out: Z pivots, (column, row) in column order
+    uint8_t* used;   // rows taken as X pivots (zero at the start)
+    uint8_t* zused;  // rows taken as Z pivots (zero at the start)
+    int* pivots;     // out: the X pivot rows in column order
+    int* zcol;       // out: Z pivots, (column, row) in column order
     int* zrow;
-    int* counts;    // out: [number of X pivots, number of Z pivots]
+    int* counts;     // out: number of X pivots, of Z pivots (zero at the start); the panel's
+    uint64_t* comb;  // n: the panel's pivot rows multiplied onto each row
+    uint64_t* px;    // the panel's pivot rows as it began: 64 x W
+    uint64_t* pz;
+    uint8_t* ps;
     int n, W;
 };
 
-// shared memory of one CTA holding R rows of W words
-__host__ __device__ inline size_t sup_smem_bytes(int R, int W) { return (size_t)2 * R * (W | 1) * 8 + 16 + (size_t)3 * R; }
+// shared memory of the panel kernel
+static size_t panel_smem(int n) { return (size_t)17 * n + 15; }
 
-template <int WPL>  // words of a row per lane: W <= 32 * WPL
-__global__ void __launch_bounds__(kSupThreads, 1) k_support_cluster(SupArgs A) {
-    extern __shared__ __align__(16) uint64_t sup_sm[];
-    const int C = cluster_nctarank(), rank = cluster_ctarank();
-    const int n = A.n, W = A.W, S = W | 1;  // odd row stride: the lanes' reads of one word of 32 rows spread over the banks
-    const int R = (n + C - 1) / C;
-    const int RW = (R + kSupWarps - 1) / kSupWarps;
-    uint64_t* lx = sup_sm;
-    uint64_t* lz = lx + (size_t)R * S;
-    int* lmin = (int*)(lz + (size_t)R * S);  // three rotating candidate slots
-    uint8_t* lr = (uint8_t*)(lmin + 4);
-    uint8_t* lu = lr + R;   // taken as an X pivot
-    uint8_t* lzu = lu + R;  // taken as a Z pivot
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = rank * R;
-    const int nloc = max(0, min(R, n - r0));
-    for (int i = threadIdx.x; i < R * W; i += blockDim.x) {
-        const int t = i / W, v = i - t * W;
-        const bool in = t < nloc;
-        lx[t * S + v] = in ? A.sx[(int64_t)(r0 + t) * W + v] : 0;
-        lz[t * S + v] = in ? A.sz[(int64_t)(r0 + t) * W + v] : 0;
+__global__ void __launch_bounds__(kPanelThreads, 1) k_support_panel(SupArgs A, int phase, int w) {
+    extern __shared__ __align__(16) uint64_t panel_sm[];
+    __shared__ int slot[3], prow[64], pcol[64];
+    const int n = A.n, W = A.W, tid = threadIdx.x;
+    uint64_t* word = panel_sm;
+    uint64_t* comb = word + n;
+    uint8_t* taken = (uint8_t*)(comb + n);
+    const uint64_t* M = phase == 0 ? A.sx : A.sz;
+    uint8_t* flags = phase == 0 ? A.used : A.zused;
+    for (int t = tid; t < n; t += blockDim.x) {  // rows of X pivots take no part in the Z phase
+        word[t] = phase == 1 && A.used[t] ? 0 : M[(int64_t)t * W + w];
+        comb[t] = 0;
+        taken[t] = flags[t];
     }
-    for (int t = threadIdx.x; t < R; t += blockDim.x) {
-        lr[t] = t < nloc ? A.sr[r0 + t] : 0;
-        lu[t] = 0;
-        lzu[t] = 0;
+    if (tid < 3) slot[tid] = INT_MAX;
+    const int before = A.counts[phase];
+    __syncthreads();
+    int np = 0;
+    const int cols = min(64, n - 64 * w);
+    for (int j = 0; j < cols; ++j) {
+        int best = INT_MAX;  // the lowest row with the bit that is not taken
+        for (int t = tid; t < n; t += blockDim.x)
+            if (((word[t] >> j) & 1) && !taken[t]) {
+                best = t;
+                break;
+            }
+        best = __reduce_min_sync(0xffffffffu, best);
+        if ((tid & 31) == 0 && best != INT_MAX) atomicMin(&slot[j % 3], best);
+        __syncthreads();
+        // the slot read a column ago is free again: every thread passed this barrier after reading it
+        if (tid == 0) slot[(j + 2) % 3] = INT_MAX;
+        const int p = slot[j % 3];
+        if (p == INT_MAX) continue;
+        // (the pivot's own words change in later columns only, behind the next barrier)
+        const uint64_t wp = word[p], cp = comb[p] ^ (1ull << np);
+        for (int t = tid; t < n; t += blockDim.x) {
+            if (t == p) taken[t] = 1;
+            else if ((word[t] >> j) & 1) {
+                word[t] ^= wp;
+                comb[t] ^= cp;
+            }
+        }
+        if (tid == 0) {
+            prow[np] = p;
+            pcol[np] = 64 * w + j;
+        }
+        ++np;
     }
-    if (threadIdx.x < 3) lmin[threadIdx.x] = INT_MAX;
-    cluster_barrier();  // every CTA of the cluster running and initialised before the first remote read
-    const int w0 = warp * RW, w1 = min(w0 + RW, nloc);
-    const uint32_t slot_base = lane < C ? dsmem_map(lmin, lane) : 0u;
-    int np = 0, nz = 0, k = 0;
-    for (int phase = 0; phase < 2; ++phase) {
-        uint64_t* M = phase == 0 ? lx : lz;
-        for (int q = 0; q < n; ++q, ++k) {
-            const int qw = q >> 6, slot = k % 3;
-            const uint64_t qb = 1ull << (q & 63);
-            for (int base = w0; base < w1; base += 32) {  // this warp's lowest eligible row
-                const int t = base + lane;
-                const bool hit = t < w1 && (M[t * S + qw] & qb) && !lu[t] && (phase == 0 || !lzu[t]);
-                const unsigned m = __ballot_sync(0xffffffffu, hit);
-                if (m) {
-                    if (lane == 0) atomicMin(&lmin[slot], r0 + base + __ffs(m) - 1);
-                    break;
-                }
-            }
-            cluster_barrier();
-            // the slot read two columns ago is free again: every CTA passed this barrier after reading it
-            if (threadIdx.x == 0) lmin[(k + 2) % 3] = INT_MAX;
-            const int p = __reduce_min_sync(0xffffffffu, lane < C ? dsmem_s32(slot_base + 4u * slot) : INT_MAX);
-            if (p == INT_MAX) continue;  // no pivot for this column (the same answer in every CTA)
-            const int owner = p / R, pl = p - owner * R;
-            if (owner == rank && pl >= w0 && pl < w1 && lane == 0) {
-                if (phase == 0) {
-                    lu[pl] = 1;
-                    A.pivots[np] = p;
-                } else {
-                    lzu[pl] = 1;
-                    A.zcol[nz] = q;
-                    A.zrow[nz] = p;
-                }
-            }
-            if (phase == 0) ++np; else ++nz;
-            uint64_t px[WPL], pz[WPL];
-            const uint32_t ax = dsmem_map(lx + (size_t)pl * S, owner), az = dsmem_map(lz + (size_t)pl * S, owner);
-#pragma unroll
-            for (int j = 0; j < WPL; ++j) {
-                const int v = lane + 32 * j;
-                px[j] = (phase == 0 && v < W) ? dsmem_u64(ax + 8u * v) : 0;
-                pz[j] = v < W ? dsmem_u64(az + 8u * v) : 0;
-            }
-            const int psign = dsmem_u8(dsmem_map(lr + pl, owner));
-            for (int base = w0; base < w1; base += 32) {
-                const int t = base + lane;
-                const bool hit = t < w1 && r0 + t != p && (M[t * S + qw] & qb) && (phase == 0 || !lu[t]);
-                unsigned m = __ballot_sync(0xffffffffu, hit);
-                while (m) {
-                    const int tt = base + __ffs(m) - 1;
-                    m &= m - 1;
-                    if (phase == 0) {
-                        int g = 0;
-#pragma unroll
-                        for (int j = 0; j < WPL; ++j) {
-                            const int v = lane + 32 * j;
-                            if (v < W) {
-                                const uint64_t x1 = px[j], z1 = pz[j], x2 = lx[tt * S + v], z2 = lz[tt * S + v];
-                                const uint64_t plus = (x1 & z1 & ~x2 & z2) | (x1 & ~z1 & x2 & z2) | (~x1 & z1 & x2 & ~z2);
-                                const uint64_t minus = (x1 & z1 & x2 & ~z2) | (x1 & ~z1 & ~x2 & z2) | (~x1 & z1 & x2 & z2);
-                                g += __popcll(plus) - __popcll(minus);
-                                lx[tt * S + v] = x2 ^ x1;
-                                lz[tt * S + v] = z2 ^ z1;
-                            }
-                        }
-                        g = __reduce_add_sync(0xffffffffu, g);
-                        if (lane == 0) {
-                            const int total = 2 * lr[tt] + 2 * psign + g;
-                            lr[tt] = (((total % 4) + 4) % 4) == 2 ? 1 : 0;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < WPL; ++j) {
-                            const int v = lane + 32 * j;
-                            if (v < W) lz[tt * S + v] ^= pz[j];
-                        }
-                        if (lane == 0) lr[tt] ^= (uint8_t)psign;
-                    }
-                }
-            }
-            __syncwarp();  // this warp's row and flag updates seen by all its lanes at the next column
+    __syncthreads();
+    for (int t = tid; t < n; t += blockDim.x) {
+        A.comb[t] = comb[t];
+        flags[t] = taken[t];
+    }
+    for (int i = tid; i < np * W; i += blockDim.x) {
+        const int64_t from = (int64_t)prow[i / W] * W + i % W;
+        A.px[i] = A.sx[from];
+        A.pz[i] = A.sz[from];
+    }
+    for (int i = tid; i < np; i += blockDim.x) {
+        A.ps[i] = A.sr[prow[i]];
+        if (phase == 0) {
+            A.pivots[before + i] = prow[i];
+        } else {
+            A.zcol[before + i] = pcol[i];
+            A.zrow[before + i] = prow[i];
         }
     }
-    cluster_barrier();  // no CTA leaves while another may still read its rows
-    for (int i = threadIdx.x; i < nloc * W; i += blockDim.x) {
-        const int t = i / W, v = i - t * W;
-        A.sx[(int64_t)(r0 + t) * W + v] = lx[t * S + v];
-        A.sz[(int64_t)(r0 + t) * W + v] = lz[t * S + v];
-    }
-    for (int t = threadIdx.x; t < nloc; t += blockDim.x) {
-        A.sr[r0 + t] = lr[t];
-        A.used[r0 + t] = lu[t];
-    }
-    if (rank == 0 && threadIdx.x == 0) {
-        A.counts[0] = np;
-        A.counts[1] = nz;
-    }
+    if (tid == 0) A.counts[phase] = before + np;
 }
 
-// cluster size for n rows, or 0 when this device cannot run the one-launch support
-static int support_cluster_size(int n, int W, size_t* smem) {
-    if (getenv("LSG_SUPPORT_STEPS")) return 0;  // diagnostics: the launch-per-column path
-    int C = 1;
-    while (C < kSupMaxCluster && (n + C - 1) / C > kSupRowsPerCta) C *= 2;
-    const int R = (n + C - 1) / C;
-    *smem = sup_smem_bytes(R, W);
-    int dev = 0, optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        (size_t)optin < *smem || W > 64)
-        return 0;
-    auto kern = W <= 32 ? k_support_cluster<1> : k_support_cluster<2>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
+// every row times its panel pivots, with the phase exponent summed mod 4 from popcounts (the Z phase's
+// rows hold no X part: their signs add)
+__global__ void k_support_rows(SupArgs A, int phase) {
+    const int lane = threadIdx.x & 31, W = A.W;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < A.n; t += warps) {
+        const uint64_t set = A.comb[t];
+        if (!set) continue;
+        int g = 0;
+        for (int v = lane; v < W; v += 32) {
+            uint64_t x2 = phase == 0 ? A.sx[(int64_t)t * W + v] : 0, z2 = A.sz[(int64_t)t * W + v];
+            for (uint64_t m = set; m; m &= m - 1) {
+                const int j = __ffsll((long long)m) - 1;
+                const uint64_t z1 = A.pz[j * W + v];
+                if (phase == 0) {
+                    const uint64_t x1 = A.px[j * W + v];
+                    const uint64_t plus = (x1 & z1 & ~x2 & z2) | (x1 & ~z1 & x2 & z2) | (~x1 & z1 & x2 & ~z2);
+                    const uint64_t minus = (x1 & z1 & x2 & ~z2) | (x1 & ~z1 & ~x2 & z2) | (~x1 & z1 & x2 & z2);
+                    g += __popcll(plus) - __popcll(minus);
+                    x2 ^= x1;
+                }
+                z2 ^= z1;
+            }
+            if (phase == 0) A.sx[(int64_t)t * W + v] = x2;
+            A.sz[(int64_t)t * W + v] = z2;
+        }
+        // the pivots' signs, a lane two of them
+        for (int j = lane; j < 64; j += 32)
+            if ((set >> j) & 1) g += 2 * A.ps[j];
+        g = __reduce_add_sync(0xffffffffu, g);
+        if (lane == 0) A.sr[t] = ((2 * A.sr[t] + g) & 3) == 2 ? 1 : 0;
     }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(kSupThreads);
-    cfg.dynamicSmemBytes = *smem;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
-        cudaGetLastError();
-        return 0;
-    }
-    return C;
-}
-
-static cudaError_t launch_support_cluster(const SupArgs& A, int C, size_t smem, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(kSupThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return A.W <= 32 ? cudaLaunchKernelEx(&cfg, k_support_cluster<1>, A) : cudaLaunchKernelEx(&cfg, k_support_cluster<2>, A);
 }
 
 // Pauli frames: one CTA per 32-shot word.
@@ -957,8 +849,7 @@ int lsg_tab_download(lsg_tab t, uint8_t* x, uint8_t* z, uint8_t* r) {
     return LSG_OK;
 }
 
-// support() with a launch per column and phase (the path for devices that cannot run the
-// one-launch cluster kernel): pivot kernels and rowsum/XOR kernels, the Z constraints compacted
+// support() with a launch per column and phase (LSG_SUPPORT_STEPS, for comparison): pivot kernels and rowsum/XOR kernels, the Z constraints compacted
 // on the host
 static int support_steps(int n, int W, uint64_t* sx, uint64_t* sz, uint8_t* sr, char* b, size_t o_used, size_t o_piv, size_t o_pivots, size_t o_np, size_t o_zm,
                          size_t o_zb, size_t o_zp, size_t o_znp, size_t o_zused, cudaStream_t st,
@@ -1053,6 +944,10 @@ int lsg_tab_support(lsg_tab t, const int32_t* qubits, int32_t m, uint8_t* x0, ui
     const size_t o_zused = off; off += al(n);
     const size_t o_zc = off; off += al((size_t)n * 4);
     const size_t o_zrw = off; off += al((size_t)n * 4);
+    const size_t o_comb = off; off += al((size_t)n * 8);
+    const size_t o_px = off; off += al((size_t)64 * W * 8);
+    const size_t o_pz = off; off += al((size_t)64 * W * 8);
+    const size_t o_ps = off; off += al(64);
     LSG_CHECK(ensure(t->work2, off));
     char* b = (char*)t->work2.ptr;
     uint64_t* sx = (uint64_t*)(b + o_sx);
@@ -1060,12 +955,12 @@ int lsg_tab_support(lsg_tab t, const int32_t* qubits, int32_t m, uint8_t* x0, ui
     uint8_t* sr = (uint8_t*)(b + o_sr);
     k_tab_rows<<<std::max(1, std::min(152 * 8, (n * W + kS - 1) / kS)), kS, 0, st>>>(t->x, t->z, t->r, n, t->words, W, sx,
                                                                                    sz, sr);
+    bool identity = m == n;  // every qubit in order
+    for (int i = 0; identity && i < m; ++i) identity = qubits[i] == i;
     std::vector<uint8_t> xfull(n, 0);
     std::vector<int> pivots;
     std::vector<uint64_t> hsx((size_t)n * W);
-    size_t smem = 0;
-    const int C = support_cluster_size(n, W, &smem);
-    if (C > 0) {
+    if (!getenv("LSG_SUPPORT_STEPS")) {
         SupArgs A;
         A.sx = sx;
         A.sz = sz;
@@ -1075,9 +970,23 @@ int lsg_tab_support(lsg_tab t, const int32_t* qubits, int32_t m, uint8_t* x0, ui
         A.zcol = (int*)(b + o_zc);
         A.zrow = (int*)(b + o_zrw);
         A.counts = (int*)(b + o_np);
+        A.zused = (uint8_t*)(b + o_zused);
+        A.comb = (uint64_t*)(b + o_comb);
+        A.px = (uint64_t*)(b + o_px);
+        A.pz = (uint64_t*)(b + o_pz);
+        A.ps = (uint8_t*)(b + o_ps);
         A.n = n;
         A.W = W;
-        LSG_CUDA(launch_support_cluster(A, C, smem, st));
+        LSG_CUDA(cudaMemsetAsync(A.used, 0, n, st));
+        LSG_CUDA(cudaMemsetAsync(A.zused, 0, n, st));
+        LSG_CUDA(cudaMemsetAsync(A.counts, 0, 8, st));
+        const int threads = std::min(kPanelThreads, (n + 31) / 32 * 32);
+        for (int phase = 0; phase < 2; ++phase)
+            for (int w = 0; w < W; ++w) {
+                k_support_panel<<<1, threads, panel_smem(n), st>>>(A, phase, w);
+                k_support_rows<<<(unsigned)std::max(1, std::min(152 * 4, (n + 3) / 4)), 128, 0, st>>>(A, phase);
+            }
+        LSG_CUDA(cudaGetLastError());
         int counts[2] = {0, 0};
         LSG_CUDA(cudaMemcpyAsync(counts, A.counts, 8, cudaMemcpyDeviceToHost, st));
         LSG_CUDA(cudaStreamSynchronize(st));
@@ -1092,7 +1001,7 @@ int lsg_tab_support(lsg_tab t, const int32_t* qubits, int32_t m, uint8_t* x0, ui
             LSG_CUDA(cudaMemcpyAsync(zrw.data(), A.zrow, (size_t)nz * 4, cudaMemcpyDeviceToHost, st));
         }
         LSG_CUDA(cudaMemcpyAsync(hsr.data(), sr, n, cudaMemcpyDeviceToHost, st));
-        LSG_CUDA(cudaMemcpyAsync(hsx.data(), sx, rowsb, cudaMemcpyDeviceToHost, st));
+        if (basis || !identity) LSG_CUDA(cudaMemcpyAsync(hsx.data(), sx, rowsb, cudaMemcpyDeviceToHost, st));
         LSG_CUDA(cudaStreamSynchronize(st));
         // the solution of the Z constraints: each pivot column takes its reduced row's sign
         for (int j = 0; j < nz; ++j) {
@@ -1108,8 +1017,10 @@ int lsg_tab_support(lsg_tab t, const int32_t* qubits, int32_t m, uint8_t* x0, ui
     const int npiv = (int)pivots.size();
     for (int i = 0; i < m; ++i) x0[i] = xfull[qubits[i]];
     // basis: X parts of the pivot rows restricted to `qubits` (stabilizer.py:361-365)
-    bool identity = m == n;
-    for (int i = 0; identity && i < m; ++i) identity = qubits[i] == i;
+    if (identity && !basis) {
+        *rank = npiv;
+        return LSG_OK;
+    }
     std::vector<uint8_t> vec((size_t)npiv * m);
     for (int j = 0; j < npiv; ++j)
         for (int i = 0; i < m; ++i) {
@@ -1118,7 +1029,7 @@ int lsg_tab_support(lsg_tab t, const int32_t* qubits, int32_t m, uint8_t* x0, ui
         }
     if (identity) {
         *rank = npiv;
-        if (basis) std::memcpy(basis, vec.data(), vec.size());
+        std::memcpy(basis, vec.data(), vec.size());
         return LSG_OK;
     }
     // row basis of the restricted vectors (stabilizer.py:425-440), on the host: npiv x m bits
