@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "common.cuh"
@@ -301,15 +302,16 @@ __global__ void k_elim_xor(uint64_t* __restrict__ m, uint8_t* __restrict__ rhs, 
 
 // ---- support() in panels of 64 columns, two launches each. The pivots of a panel depend only on its
 // one word per row and on which rows are taken, so one CTA walks its columns on the rows' words in
-// shared memory, a barrier a column, and notes for every row the set of pivot rows multiplied onto it
+// registers, a barrier a column, and notes for every row the set of pivot rows multiplied onto it
 // (64 bits: pivot rows as they stood when the panel began; stabilizer rows commute, so neither a
 // product's words nor its sign depend on the order). Then all SMs form the products, a warp per row.
 // The X phase (pivots with the phase rowsum, stabilizer.py:371-395) is followed by the Z phase on
 // the rows no X pivot took (plain GF(2) elimination with the signs as right-hand side,
 // stabilizer.py:398-422). A column then costs a barrier and a few shared-memory reads of one CTA
-// where a cluster that held the rows exchanged a pivot row per column.
+// where a cluster that held the rows exchanged a pivot row per column (2048 qubits: 14.5 ms, now
+// 1.9).
 
-constexpr int kPanelThreads = 1024;
+constexpr int kPanelThreads = 256;
 
 struct SupArgs {
     uint64_t* sx;  // n rows x W words, row-major: in, the stabilizer rows; out, reduced
@@ -328,61 +330,78 @@ struct SupArgs {
     int n, W;
 };
 
-// shared memory of the panel kernel
-static size_t panel_smem(int n) { return (size_t)17 * n + 15; }
-
+// ROWS rows per thread: with few warps a column's fixed instructions (the reductions, the barrier, the
+// pivot's reads) issue few times, and rows in flight hide them. 2048 rows, a panel: 41 us with the
+// words in shared memory and 1024 threads, 31 in registers, 23 with 256 threads of 8 rows.
+template <int ROWS>
 __global__ void __launch_bounds__(kPanelThreads, 1) k_support_panel(SupArgs A, int phase, int w) {
-    extern __shared__ __align__(16) uint64_t panel_sm[];
-    __shared__ int slot[3], prow[64], pcol[64];
-    const int n = A.n, W = A.W, tid = threadIdx.x;
-    uint64_t* word = panel_sm;
-    uint64_t* comb = word + n;
-    uint8_t* taken = (uint8_t*)(comb + n);
+    // per warp its lowest eligible row, and that row's word and set: two buffers, a column each
+    __shared__ int row[2][32];
+    __shared__ uint4 row_data[2][32];
+    __shared__ int prow[64], pcol[64];
+    const int n = A.n, W = A.W, tid = threadIdx.x, lane = tid & 31, warps = blockDim.x >> 5;
     const uint64_t* M = phase == 0 ? A.sx : A.sz;
     uint8_t* flags = phase == 0 ? A.used : A.zused;
-    for (int t = tid; t < n; t += blockDim.x) {  // rows of X pivots take no part in the Z phase
-        word[t] = phase == 1 && A.used[t] ? 0 : M[(int64_t)t * W + w];
-        comb[t] = 0;
-        taken[t] = flags[t];
+    uint32_t word[2][ROWS], comb[2][ROWS], open[ROWS];  // open: all ones until the row is taken
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {  // rows of X pivots take no part in the Z phase
+        const int t = tid + i * blockDim.x;
+        const uint64_t m = t >= n || (phase == 1 && A.used[t]) ? 0 : M[(int64_t)t * W + w];
+        word[0][i] = (uint32_t)m;
+        word[1][i] = (uint32_t)(m >> 32);
+        open[i] = t < n && flags[t] ? 0u : ~0u;
+        comb[0][i] = comb[1][i] = 0;
     }
-    if (tid < 3) slot[tid] = INT_MAX;
     const int before = A.counts[phase];
-    __syncthreads();
     int np = 0;
     const int cols = min(64, n - 64 * w);
-    for (int j = 0; j < cols; ++j) {
-        int best = INT_MAX;  // the lowest row with the bit that is not taken
-        for (int t = tid; t < n; t += blockDim.x)
-            if (((word[t] >> j) & 1) && !taken[t]) {
-                best = t;
-                break;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        for (int j = 0; j < min(32, cols - 32 * h); ++j) {
+            const int at = j & 1;
+            const uint32_t bit = 1u << j;
+            int best = INT_MAX;  // the lowest row with the bit that is not taken
+#pragma unroll
+            for (int i = ROWS - 1; i >= 0; --i)
+                if (word[h][i] & open[i] & bit) best = tid + i * blockDim.x;
+            const int low = __reduce_min_sync(0xffffffffu, best);
+            if (lane == 0) row[at][tid >> 5] = low;
+            if (low != INT_MAX && low == best) {
+#pragma unroll
+                for (int i = 0; i < ROWS; ++i)
+                    if (low == tid + i * (int)blockDim.x)
+                        row_data[at][tid >> 5] = make_uint4(word[0][i], word[1][i], comb[0][i], comb[1][i]);
             }
-        best = __reduce_min_sync(0xffffffffu, best);
-        if ((tid & 31) == 0 && best != INT_MAX) atomicMin(&slot[j % 3], best);
-        __syncthreads();
-        // the slot read a column ago is free again: every thread passed this barrier after reading it
-        if (tid == 0) slot[(j + 2) % 3] = INT_MAX;
-        const int p = slot[j % 3];
-        if (p == INT_MAX) continue;
-        // (the pivot's own words change in later columns only, behind the next barrier)
-        const uint64_t wp = word[p], cp = comb[p] ^ (1ull << np);
-        for (int t = tid; t < n; t += blockDim.x) {
-            if (t == p) taken[t] = 1;
-            else if ((word[t] >> j) & 1) {
-                word[t] ^= wp;
-                comb[t] ^= cp;
+            __syncthreads();  // (a buffer is written again two columns on, behind the next barrier)
+            const int mine = lane < warps ? row[at][lane] : INT_MAX;
+            const int p = __reduce_min_sync(0xffffffffu, mine);
+            if (p == INT_MAX) continue;
+            uint4 d = row_data[at][__ffs(__ballot_sync(0xffffffffu, mine == p)) - 1];
+            if (np < 32) d.z ^= 1u << np;
+            else d.w ^= 1u << (np - 32);
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                if (tid + i * (int)blockDim.x == p) open[i] = 0u;
+                else if (word[h][i] & bit) {
+                    word[0][i] ^= d.x;
+                    word[1][i] ^= d.y;
+                    comb[0][i] ^= d.z;
+                    comb[1][i] ^= d.w;
+                }
             }
+            if (tid == 0) {
+                prow[np] = p;
+                pcol[np] = 64 * w + 32 * h + j;
+            }
+            ++np;
         }
-        if (tid == 0) {
-            prow[np] = p;
-            pcol[np] = 64 * w + j;
-        }
-        ++np;
-    }
     __syncthreads();
-    for (int t = tid; t < n; t += blockDim.x) {
-        A.comb[t] = comb[t];
-        flags[t] = taken[t];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const int t = tid + i * blockDim.x;
+        if (t >= n) continue;
+        A.comb[t] = (uint64_t)comb[1][i] << 32 | comb[0][i];
+        flags[t] = open[i] == 0u;
     }
     for (int i = tid; i < np * W; i += blockDim.x) {
         const int64_t from = (int64_t)prow[i / W] * W + i % W;
@@ -469,14 +488,13 @@ __global__ void k_frames(FrameArgs A) {
     for (int q = threadIdx.x; q < n; q += blockDim.x) {
         uint32_t zw = 0;
         const uint64_t base = (uint64_t)q * A.shots + shot0;
-        uint64_t cur_raw_index = ~0ull;
-        uint64_t raw = 0;
+        u128 state = pcg_advance(A.s0, A.inc, (base >> 3) + 1);  // one jump, then a step per raw draw
+        uint64_t raw = pcg_output(state);
         for (int j = 0; j < valid; ++j) {
             const uint64_t t = base + j;
-            const uint64_t ri = t >> 3;
-            if (ri != cur_raw_index) {
-                raw = pcg_raw(A.s0, A.inc, ri);
-                cur_raw_index = ri;
+            if (j && !(t & 7)) {
+                state = state * pcg_mult() + A.inc;
+                raw = pcg_output(state);
             }
             const uint32_t word = ((t >> 2) & 1) ? (uint32_t)(raw >> 32) : (uint32_t)raw;
             zw |= (uint32_t)((word >> (8 * (t & 3) + 7)) & 1) << j;
@@ -602,60 +620,42 @@ __global__ void k_gate_states(u128 s0, u128 inc, uint64_t base, uint64_t stride,
         out[k] = pcg_advance(s0, inc, base + (uint64_t)k * stride);
 }
 
-// The Pauli-noise masks of every noisy gate for every 32-shot word, over all SMs: a warp per
-// (gate, word), lane j drawing shot 32w + j's uniform (the gate's block state advanced by
-// 32w + j + 1: word jump, then lane jump) and choosing its branch; ballots give the word's X and Z
-// masks of the gate's (up to two) qubits. masks[w * nnoisy + nk] = {x0, z0, x1, z1}.
+// The Pauli-noise masks of every noisy gate for every 32-shot word, over all SMs: a thread per (gate,
+// word) steps the gate's generator through the word's 32 shots (one 128-bit product each) and sets
+// the bits of the rare shots whose uniform passes the first branch. masks[w * nnoisy + nk] =
+// {x0, z0, x1, z1}. A warp per (gate, word) with a lane per shot took two products, a division
+// and a branch search of dependent loads for every shot: 2.36 ms for 410,000 gates and 1000
+// shots, now 0.72, its 128-bit products.
 __global__ void k_noise_masks(const u128* __restrict__ gate_states, const int16_t* __restrict__ gate_table,
-                              const NTable* __restrict__ noise, int64_t nnoisy, int words, int shots,
-                              const u128* __restrict__ word_mult, const u128* __restrict__ word_plus,
-                              const u128* __restrict__ lane_mult, const u128* __restrict__ lane_plus, uint4* masks) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const u128 lm = lane_mult[lane], lp = lane_plus[lane];
-    for (int64_t t = (((int64_t)blockIdx.x * blockDim.x) + threadIdx.x) >> 5; t < nnoisy * words; t += nwarps) {
-        const int w = (int)(t / nnoisy);
-        const int64_t nk = t - (int64_t)w * nnoisy;
+                              const NTable* __restrict__ noise, int64_t nnoisy, int words, int shots, u128 inc,
+                              const u128* __restrict__ word_mult, const u128* __restrict__ word_plus, uint4* masks) {
+    const u128 mult = pcg_mult();
+    for (int64_t nk = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; nk < nnoisy; nk += (int64_t)gridDim.x * blockDim.x) {
         const NTable& nt = noise[gate_table[nk]];
-        const u128 st = lm * (word_mult[w] * gate_states[nk] + word_plus[w]) + lp;
-        const uint64_t m = pcg_output(st) >> 11;
-        int pick = 0;  // searchsorted(cumulative, u, side='right'), clamped
-        while (pick < nt.nb && nt.thr[pick] <= m) ++pick;
-        if (pick > nt.nb - 1) pick = nt.nb - 1;
-        const bool live = 32 * w + lane < shots;
-        const unsigned lab = live ? nt.label[pick] : 0u;
+        const u128 s0 = gate_states[nk];
+        const uint64_t first = nt.thr[0];
+        const unsigned none = nt.label[0];
         const int sh = 2 * (nt.k - 1);  // the first qubit's bits
-        uint4 out;
-        out.x = __ballot_sync(0xffffffffu, (lab >> (sh + 1)) & 1);
-        out.y = __ballot_sync(0xffffffffu, (lab >> sh) & 1);
-        out.z = nt.k == 2 ? __ballot_sync(0xffffffffu, (lab >> 1) & 1) : 0u;
-        out.w = nt.k == 2 ? __ballot_sync(0xffffffffu, lab & 1) : 0u;
-        if (lane == 0) masks[t] = out;
+        for (int w = blockIdx.y; w < words; w += gridDim.y) {
+            u128 st = word_mult[w] * s0 + word_plus[w];
+            const int valid = min(32, shots - 32 * w);
+            uint32_t m[4] = {0, 0, 0, 0};  // by label bit
+            for (int j = 0; j < valid; ++j) {
+                st = st * mult + inc;
+                const uint64_t um = pcg_output(st) >> 11;  // the uniform is um * 2^-53
+                unsigned lab = none;
+                if (um >= first) {  // searchsorted(cumulative, u, side='right'), clamped
+                    int pick = 1;
+                    while (pick < nt.nb && nt.thr[pick] <= um) ++pick;
+                    lab = nt.label[min(pick, nt.nb - 1)];
+                }
+                if (lab)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) m[i] |= ((lab >> i) & 1u) << j;
+            }
+            masks[(int64_t)w * nnoisy + nk] = sh ? make_uint4(m[3], m[2], m[1], m[0]) : make_uint4(m[1], m[0], 0u, 0u);
+        }
     }
-}
-
-// ASAP moments of a gate list: a gate's moment is one past the latest moment among its qubits
-static void moments_of(const GateRec* g, int64_t ng, int n, const int8_t* arity, std::vector<int64_t>& order,
-                       std::vector<int64_t>& starts) {
-    std::vector<int64_t> last(n, -1), level(ng);
-    int64_t maxl = -1;
-    for (int64_t i = 0; i < ng; ++i) {
-        int64_t l = last[g[i].a];
-        if (arity[i] > 1) l = std::max(l, last[g[i].b]);
-        if (arity[i] > 2) l = std::max(l, last[g[i].c]);
-        level[i] = l + 1;
-        last[g[i].a] = level[i];
-        if (arity[i] > 1) last[g[i].b] = level[i];
-        if (arity[i] > 2) last[g[i].c] = level[i];
-        maxl = std::max(maxl, level[i]);
-    }
-    std::vector<int64_t> count(maxl + 2, 0);
-    for (int64_t i = 0; i < ng; ++i) count[level[i] + 1]++;
-    for (int64_t l = 0; l <= maxl; ++l) count[l + 1] += count[l];
-    starts.assign(count.begin(), count.end());
-    order.assign(ng, 0);
-    std::vector<int64_t> fill(count.begin(), count.end() - 1);
-    for (int64_t i = 0; i < ng; ++i) order[fill[level[i]]++] = i;
 }
 
 }  // namespace lsg
@@ -671,10 +671,17 @@ struct lsg_tab_s {
 
 namespace {
 
-int gate_records(int n, const lsg_cgate* gates, int64_t ng, int32_t ntables, int32_t nnoise, std::vector<GateRec>& recs,
-                 std::vector<int8_t>& arity) {
-    recs.resize(ng);
-    arity.resize(ng);
+// The gates checked and sorted into ASAP moments (a gate's is one past the latest among its qubits), in
+// circuit order within one; noisy gates numbered in circuit order, `table` their noise tables. Two
+// passes over the gates and two lists, the levels and the records where they are wanted: with four
+// lists, 64-bit entries and a copy into order, first touches of their pages took most of it
+// (410,000 gates: the tableau's call 4.7 -> 3.0 ms, a frames run 7.3 -> 5.4).
+int gate_moments(int n, const lsg_cgate* gates, int64_t ng, int32_t ntables, int32_t nnoise, std::vector<GateRec>& sorted,
+                 std::vector<int64_t>& starts, std::vector<int16_t>* table) {
+    std::vector<int32_t> last(n, 0);  // per qubit: the moment it is free in
+    std::unique_ptr<int32_t[]> level(new int32_t[(size_t)std::max<int64_t>(ng, 1)]);
+    std::vector<int64_t> count(1, 0);
+    int64_t noisy = 0;
     for (int64_t i = 0; i < ng; ++i) {
         const lsg_cgate& g = gates[i];
         int k = 1;
@@ -687,14 +694,37 @@ int gate_records(int n, const lsg_cgate* gates, int64_t ng, int32_t ntables, int
             return fail(LSG_E_ARG, "gate %lld has a bad code", (long long)i);
         }
         const int q[3] = {g.a, g.b, g.c};
-        for (int j = 0; j < k; ++j)
+        int32_t l = 0;
+        for (int j = 0; j < k; ++j) {
             if (q[j] < 0 || q[j] >= n) return fail(LSG_E_ARG, "gate %lld names a missing qubit", (long long)i);
+            l = std::max(l, last[q[j]]);
+        }
         if (g.noise >= nnoise) return fail(LSG_E_ARG, "gate %lld names a missing noise table", (long long)i);
-        recs[i] = GateRec{(int16_t)g.code, (int16_t)g.noise, (int16_t)g.a, (int16_t)g.b, (int16_t)g.c, 0, -1};
-        arity[i] = (int8_t)k;
+        for (int j = 0; j < k; ++j) last[q[j]] = l + 1;
+        level[i] = l;
+        if ((size_t)l + 1 >= count.size()) count.resize((size_t)l + 2, 0);
+        ++count[(size_t)l + 1];
+        noisy += g.noise >= 0;
+    }
+    for (size_t l = 1; l < count.size(); ++l) count[l] += count[l - 1];
+    starts = count;
+    if (table) table->assign((size_t)std::max<int64_t>(noisy, 1), 0);
+    sorted.resize(ng);
+    int32_t nk = 0;
+    for (int64_t i = 0; i < ng; ++i) {
+        const lsg_cgate& g = gates[i];
+        const bool tell = table && g.noise >= 0;
+        if (tell) (*table)[(size_t)nk] = (int16_t)g.noise;
+        sorted[(size_t)count[(size_t)level[i]]++] =
+            GateRec{(int16_t)g.code, (int16_t)g.noise, (int16_t)g.a, (int16_t)g.b, (int16_t)g.c, 0, tell ? nk++ : -1};
     }
     return LSG_OK;
 }
+
+// Threads of a CTA that walks a circuit's moments over n qubits: a moment holds up to n gates, each a few
+// dependent loads, and few words leave one CTA on an SM.
+// (2048 qubits, 1024 threads for 256: the tableau 0.93 -> 0.37 ms, 1000 shots' frames 1.62 -> 0.60.)
+int column_threads(int n) { return std::max(kS, std::min(1024, (n / 2 + 31) / 32 * 32)); }
 
 int upload(Scratch& s, const void* host, size_t bytes, cudaStream_t st) {
     LSG_CHECK(ensure(s, bytes));
@@ -806,13 +836,9 @@ int lsg_tab_apply(lsg_tab t, const lsg_cgate* gates, int64_t ngates, const uint8
     clear_error();
     if (!t || ngates < 0 || (ngates && !gates) || ntables < 0 || (ntables && !tables)) return fail(LSG_E_ARG, "bad arguments");
     if (ngates == 0) return LSG_OK;
-    std::vector<GateRec> recs;
-    std::vector<int8_t> arity;
-    LSG_CHECK(gate_records(t->n, gates, ngates, ntables, 0x7fff, recs, arity));
-    std::vector<int64_t> order, starts;
-    moments_of(recs.data(), ngates, t->n, arity.data(), order, starts);
-    std::vector<GateRec> sorted(ngates);
-    for (int64_t i = 0; i < ngates; ++i) sorted[i] = recs[order[i]];
+    std::vector<GateRec> sorted;
+    std::vector<int64_t> starts;
+    LSG_CHECK(gate_moments(t->n, gates, ngates, ntables, 0x7fff, sorted, starts, nullptr));
     std::vector<CTable> ct;
     LSG_CHECK(tables_device(tables, ntables, ct));
     const size_t gb = ngates * sizeof(GateRec), mb = starts.size() * 8, tb = ct.size() * sizeof(CTable);
@@ -823,7 +849,7 @@ int lsg_tab_apply(lsg_tab t, const lsg_cgate* gates, int64_t ngates, const uint8
     LSG_CUDA(cudaMemcpyAsync(base + o_m, starts.data(), mb, cudaMemcpyHostToDevice, t->stream));
     LSG_CUDA(cudaMemcpyAsync(base + o_t, ct.data(), tb, cudaMemcpyHostToDevice, t->stream));
     const size_t smem = (size_t)2 * t->n * 4;
-    k_tab_apply<<<t->words, kS, smem, t->stream>>>(t->x, t->z, t->r, t->n, t->words, (const GateRec*)base,
+    k_tab_apply<<<t->words, column_threads(t->n), smem, t->stream>>>(t->x, t->z, t->r, t->n, t->words, (const GateRec*)base,
                                                    (const int64_t*)(base + o_m), (int64_t)starts.size() - 1,
                                                    (const CTable*)(base + o_t));
     LSG_CUDA(cudaGetLastError());
@@ -981,9 +1007,11 @@ int lsg_tab_support(lsg_tab t, const int32_t* qubits, int32_t m, uint8_t* x0, ui
         LSG_CUDA(cudaMemsetAsync(A.zused, 0, n, st));
         LSG_CUDA(cudaMemsetAsync(A.counts, 0, 8, st));
         const int threads = std::min(kPanelThreads, (n + 31) / 32 * 32);
+        static_assert(8 * kPanelThreads >= 2048, "every row has a thread");
+        auto panel = n > 2 * kPanelThreads ? k_support_panel<8> : k_support_panel<2>;
         for (int phase = 0; phase < 2; ++phase)
             for (int w = 0; w < W; ++w) {
-                k_support_panel<<<1, threads, panel_smem(n), st>>>(A, phase, w);
+                panel<<<1, threads, 0, st>>>(A, phase, w);
                 k_support_rows<<<(unsigned)std::max(1, std::min(152 * 4, (n + 3) / 4)), 128, 0, st>>>(A, phase);
             }
         LSG_CUDA(cudaGetLastError());
@@ -1073,12 +1101,11 @@ int lsg_frames_run(int n, const lsg_cgate* gates, int64_t ngates, const uint8_t*
         (nnoise && !noise))
         return fail(LSG_E_ARG, "lsg_frames_run: bad arguments");
     if (shots > (1ll << 30)) return fail(LSG_E_ARG, "too many shots for one frames run");
-    std::vector<GateRec> recs;
-    std::vector<int8_t> arity;
-    LSG_CHECK(gate_records(n, gates, ngates, ntables, nnoise, recs, arity));
-    int64_t nk = 0;
-    for (int64_t i = 0; i < ngates; ++i)
-        if (recs[i].noise >= 0) recs[i].nk = (int32_t)nk++;
+    std::vector<GateRec> sorted;
+    std::vector<int64_t> starts;
+    std::vector<int16_t> gate_table;  // per noisy gate, in circuit order
+    LSG_CHECK(gate_moments(n, gates, ngates, ntables, nnoise, sorted, starts, &gate_table));
+    const int64_t nk = std::count_if(gates, gates + ngates, [](const lsg_cgate& g) { return g.noise >= 0; });
     for (int j = 0; j < npairs; ++j)
         if (pair_qubit[j] < 0 || pair_qubit[j] >= n || pair_clbit[j] < 0 || pair_clbit[j] >= nclbits)
             return fail(LSG_E_ARG, "lsg_frames_run: bad measurement pair %d", j);
@@ -1096,10 +1123,6 @@ int lsg_frames_run(int n, const lsg_cgate* gates, int64_t ngates, const uint8_t*
             nt[i].thr[j] = !(c > 0.0) ? 0ull : c >= 1.0 ? (1ull << 53) : (uint64_t)std::ceil(std::ldexp(c, 53));
         }
     }
-    std::vector<int64_t> order, starts;
-    moments_of(recs.data(), ngates, n, arity.data(), order, starts);
-    std::vector<GateRec> sorted(ngates);
-    for (int64_t i = 0; i < ngates; ++i) sorted[i] = recs[order[i]];
     std::vector<CTable> ct;
     LSG_CHECK(tables_device(tables, ntables, ct));
     const u128 s0 = ((u128)rng_state[0] << 64) | rng_state[1];
@@ -1115,14 +1138,10 @@ int lsg_frames_run(int n, const lsg_cgate* gates, int64_t ngates, const uint8_t*
         if (pair_err[j] >= 0) ++nerr;
     if (raw_used) *raw_used = (int64_t)(base_flip + (uint64_t)nerr * shots);
     const int words = (int)((shots + 31) / 32);
-    std::vector<u128> wmul(words), wplus(words), lmul(32), lplus(32);
+    std::vector<u128> wmul(words), wplus(words);
     for (int w = 0; w < words; ++w) pcg_jump(inc, (uint64_t)32 * w, &wmul[w], &wplus[w]);
-    for (int j = 0; j < 32; ++j) pcg_jump(inc, (uint64_t)j + 1, &lmul[j], &lplus[j]);
     // the noise masks of all noisy gates and words drawn up front over every SM, when they fit a
     // quarter of the free device memory (else the frame kernel draws them per gate)
-    std::vector<int16_t> gate_table((size_t)std::max<int64_t>(nk, 1), 0);
-    for (int64_t i = 0; i < ngates; ++i)
-        if (recs[i].noise >= 0) gate_table[(size_t)recs[i].nk] = recs[i].noise;
     const size_t mask_bytes = (size_t)nk * (size_t)words * sizeof(uint4);
     size_t free_mem = 0, total_mem = 0;
     const bool premask = nk > 0 && cudaMemGetInfo(&free_mem, &total_mem) == cudaSuccess && mask_bytes <= free_mem / 4;
@@ -1145,8 +1164,6 @@ int lsg_frames_run(int n, const lsg_cgate* gates, int64_t ngates, const uint8_t*
     const size_t o_p1 = off; off += al((size_t)npairs * 8);
     const size_t o_x0 = off; off += al((size_t)npairs);
     const size_t o_out = off; off += al((size_t)shots * nclbits);
-    const size_t o_lm = off; off += al(32 * 16);
-    const size_t o_lp = off; off += al(32 * 16);
     const size_t o_gt = off; off += al(gate_table.size() * sizeof(int16_t));
     const size_t o_mk = off; off += premask ? al(mask_bytes) : 0;
     Scratch work;
@@ -1177,8 +1194,6 @@ int lsg_frames_run(int n, const lsg_cgate* gates, int64_t ngates, const uint8_t*
     H2D(o_p0, p01, (size_t)npairs * 8);
     H2D(o_p1, p10, (size_t)npairs * 8);
     H2D(o_x0, pair_x0, (size_t)npairs);
-    H2D(o_lm, lmul.data(), 32 * 16);
-    H2D(o_lp, lplus.data(), 32 * 16);
     if (premask) H2D(o_gt, gate_table.data(), gate_table.size() * sizeof(int16_t));
     if (ce == cudaSuccess) ce = cudaMemsetAsync(b + o_out, 0, (size_t)shots * nclbits, st);
     if (ce == cudaSuccess && nk)
@@ -1202,15 +1217,14 @@ int lsg_frames_run(int n, const lsg_cgate* gates, int64_t ngates, const uint8_t*
     A.masks = premask ? (const uint4*)(b + o_mk) : nullptr;
     A.nnoisy = nk;
     if (ce == cudaSuccess && premask) {
-        const int64_t warps = nk * (int64_t)words;
-        k_noise_masks<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((warps * 32 + kS - 1) / kS, 152 * 32)), kS, 0, st>>>(
-            (const u128*)(b + o_s), (const int16_t*)(b + o_gt), (const NTable*)(b + o_n), nk, words, (int)shots,
-            (const u128*)(b + o_wm), (const u128*)(b + o_wp), (const u128*)(b + o_lm), (const u128*)(b + o_lp),
-            (uint4*)(b + o_mk));
+        const dim3 grid((unsigned)std::min<int64_t>((nk + 127) / 128, 152 * 64), (unsigned)std::min(words, 1024));
+        k_noise_masks<<<grid, 128, 0, st>>>((const u128*)(b + o_s), (const int16_t*)(b + o_gt), (const NTable*)(b + o_n), nk,
+                                            words, (int)shots, inc, (const u128*)(b + o_wm), (const u128*)(b + o_wp),
+                                            (uint4*)(b + o_mk));
         ce = cudaGetLastError();
     }
     if (ce == cudaSuccess) {
-        k_frames<<<words, kS, (size_t)2 * n * 4, st>>>(A);
+        k_frames<<<words, column_threads(n), (size_t)2 * n * 4, st>>>(A);
         ce = cudaGetLastError();
     }
     if (ce == cudaSuccess) {
