@@ -661,7 +661,7 @@ static int launch_passes(lsg_program_s* p, lsg_state_s* s, cudaEvent_t* marks, c
         // each pass gets the shared memory its own operators need: short passes fit more CTAs per SM
         const bool swizzle = swizzle_enabled();
         LSG_CHECK(allow_smem(PassKernels<T>::pipe()));
-        for (int mode : {kSwz, kRounds, kMixed}) LSG_CHECK(allow_smem(PassKernels<T>::swz(mode)));
+        for (int mode : {kSwz, kRounds, kMixed, kDrawn}) LSG_CHECK(allow_smem(PassKernels<T>::swz(mode)));
         size_t last_smem = 0;
         const void* last_kern = nullptr;
         int64_t grid = 1;
@@ -671,9 +671,9 @@ static int launch_passes(lsg_program_s* p, lsg_state_s* s, cudaEvent_t* marks, c
             const int64_t total = tpm[i] * s->batch;
             const bool swz = swizzle && p->swz[i];
             const int mode = swz ? p->swz[i] : kPlain;
-            const bool rounds = mode == kRounds;
+            const bool rounds = mode == kRounds || mode == kDrawn;
             const void* kern = swz ? PassKernels<T>::swz(mode) : PassKernels<T>::pipe();
-            const size_t smem = 2 * tile_bytes + (swz ? 1024 : 0) + (size_t)pd.nops * (sizeof(TileOp) + 16) +
+            const size_t smem = 2 * tile_bytes + (swz ? 1024 : 0) + (size_t)pd.nops * (sizeof(TileOp) + (mode == kDrawn ? 32 : 16)) +
                                 (size_t)pd.nblocks * sizeof(BlockDesc) +
                                 (rounds ? (size_t)pd.rounds * 16 * round_words<T>() : 0);
             if (smem != last_smem || kern != last_kern) {
@@ -943,6 +943,13 @@ static bool ops_unitary(const lsg_op* ops, int32_t nops, const double* pool, int
     return true;
 }
 
+// Whether a pass moves swizzled tiles: its copies fit the tensor maps and all its blocks are register blocks.
+static bool pass_fits_swizzle(const PassDesc& pd, const Plan& plan, size_t eb, int nbits, int64_t batch) {
+    bool fits = pass_swizzle_fits(pd, eb, ((int64_t)eb << nbits) * batch) && (eb << pd.K) <= 65536;
+    for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks && fits; ++bi) fits = !plan.blocks[bi].generic;
+    return fits;
+}
+
 // Plan and lower `ops`; with `upload`, copy the program to the device (otherwise only the host
 // plan is made: no device call).
 static int program_build(int nbits, int precision, int64_t batch, const lsg_op* ops, int32_t nops, const double* pool,
@@ -1027,11 +1034,13 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     }
     if (!pred && !draw && !count) p->core_plan = p->plan;
     // Complex programs: outer factors of one-bit operators move on to the next ones, so that blocks
-    // lower to rounds (lower.cu). So do complex128 trajectory segments, whose operators all stand under
-    // one predicate; complex64 ones, not bound by arithmetic, keep their operators.
+    // lower to rounds (lower.cu). So do trajectory segments, whose operators all stand under one
+    // predicate; complex64 ones by whole passes, where nothing but rounds, renames and mixtures is left
+    // (tile.cuh kDrawn; among other operators a complex64 round is no faster than they are).
     const char* fuse_env = getenv("LSG_FUSE_BLOCKS");
     const bool fuse = !lsg_precision_real(precision) && !(fuse_env && fuse_env[0] == '0');
-    bool rounds = fuse && ((!pred && !draw && !count) || precision == LSG_C128);
+    bool rounds = fuse;
+    const bool drawn = rounds && trajectory && precision == LSG_C64;
     const int seg_pred = pred && nops > 0 ? pred[0] : 0;
     for (int32_t i = 0; pred && i < nops; ++i) rounds = rounds && pred[i] == seg_pred;
     std::vector<double> grown;
@@ -1066,11 +1075,29 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
             ext.push_back(0.0);
         }
     };
-    for (const PassDesc& pd : p->plan.passes)
+    std::vector<char> drawn_pass(p->plan.passes.size(), 0);
+    for (const PassDesc& pd : p->plan.passes) {
+        const double round_cost = precision == LSG_C64 ? 0.5 : 0.1;
+        std::vector<LoweredBlock> lowered(drawn && rounds ? (size_t)pd.nblocks : 0);
+        bool whole_pass = !lowered.empty() && pass_fits_swizzle(pd, p->plan, lsg_elem_bytes(precision), nbits, batch);
+        for (int i = 0; i < pd.nblocks && whole_pass; ++i) {
+            const BlockDesc& blk = p->plan.blocks[pd.first_block + i];
+            auto held = [](int c) { return (c >= kT_X1 && c < kT_SWAP + 16) || (c >= kT_MIX1 && c < kT_MIX2 + 16); };
+            bool pure = true;
+            for (int o = pd.first_op + blk.first; o < pd.first_op + blk.first + blk.nops; ++o)
+                pure = pure && held(p->plan.ops[o].tmpl);
+            LoweredBlock& low = lowered[i];
+            if (pure) continue;
+            lower_block(p->plan, pd, blk, moved, batch, pool, round_cost, true, &low);
+            whole_pass = low.members == 1 && !low.items.empty() && (int)low.items.size() <= blk.nops;
+            for (const LoweredItem& it : low.items) whole_pass = whole_pass && (it.code != kKeepOp || held(it.tmpl));
+        }
+        if (drawn && rounds) drawn_pass[&pd - p->plan.passes.data()] = whole_pass;
         for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks; ++bi) {
             BlockDesc& blk = p->plan.blocks[bi];
             if (blk.generic) continue;
-            if (rounds && blk.nops > 1) {
+            const bool ready = whole_pass && !lowered[bi - pd.first_block].items.empty();
+            if (rounds && (drawn ? ready : blk.nops > 1)) {
                 const double overhead = precision == LSG_C64 ? 0.5 : 0.1;
                 double cost = 0.0;
                 bool dense = blk.u >= 2;
@@ -1081,7 +1108,9 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 }
                 if (dense) cost = std::min(cost, 1.1 * ((double)(1 << blk.u) + overhead + (double)(1 << blk.u) / 16.0));
                 LoweredBlock low;
-                if (lower_block(p->plan, pd, blk, moved, batch, pool, overhead, precision == LSG_C64, &low) && low.cost < cost) {
+                if (ready) low = std::move(lowered[bi - pd.first_block]);
+                if (ready || (lower_block(p->plan, pd, blk, moved, batch, pool, overhead, precision == LSG_C64, &low) &&
+                              low.cost < cost)) {
                     const int D = 1 << blk.u;
                     std::vector<TileOp> made;
                     for (const LoweredItem& it : low.items) {
@@ -1162,7 +1191,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 std::copy(made.begin(), made.end(), p->plan.ops.begin() + pd.first_op + blk.first);
                 blk.nops = (int)made.size();
             }
-            if (fuse && blk.u >= 2 && blk.nops > 1) {
+            if (fuse && !whole_pass && blk.u >= 2 && blk.nops > 1) {
                 const int U = blk.u, D = 1 << U;
                 const double overhead = precision == LSG_C64 ? 0.5 : 0.1;
                 bool ok = true;
@@ -1258,6 +1287,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 t.stride = t.stride ? stride : 0;
             }
         }
+    }
     // every register-block operator now carries a kernel code (mixtures are resolved per member)
     for (const PassDesc& pd : p->plan.passes)
         for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks; ++bi) {
@@ -1275,10 +1305,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
         p->swz.assign(p->plan.passes.size(), 0);
         for (size_t i = 0; i < p->plan.passes.size(); ++i) {
             PassDesc& pd = p->plan.passes[i];
-            bool fits = pass_swizzle_fits(pd, eb, ((int64_t)eb << nbits) * batch) && (eb << pd.K) <= 65536;
-            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks && fits; ++bi)
-                fits = !p->plan.blocks[bi].generic;
-            if (!fits) continue;
+            if (!pass_fits_swizzle(pd, p->plan, eb, nbits, batch)) continue;
             for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks; ++bi) {
                 BlockDesc& b = p->plan.blocks[bi];
                 if (block_layout(pd, b, &p->plan.ops[pd.first_op + b.first], eb) != LSG_OK) {
@@ -1295,9 +1322,10 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                     lowered = lowered && t.pred == 0 && (t.tmpl == kT_ROUND || (t.tmpl >= kT_X1 && t.tmpl < kT_SWAP + 16));
                 }
             }
-            p->swz[i] = (char)(lowered ? kRounds : any ? kMixed : kSwz);
+            const bool draws = drawn_pass[i];
+            p->swz[i] = (char)(draws ? kDrawn : lowered ? kRounds : any ? kMixed : kSwz);
             for (int o = pd.first_op; lowered && o < pd.first_op + pd.nops; ++o) p->plan.ops[o].count = 0;
-            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks && lowered; ++bi) {
+            for (int bi = pd.first_block; bi < pd.first_block + pd.nblocks && (lowered || draws); ++bi) {
                 const BlockDesc& b = p->plan.blocks[bi];
                 for (int o = pd.first_op + b.first; o < pd.first_op + b.first + b.nops; ++o)
                     if (p->plan.ops[o].tmpl == kT_ROUND) p->plan.ops[o].count = pd.rounds++;

@@ -17,6 +17,8 @@ const void* PassKernels<T>::pipe() {
 template <typename T>
 const void* PassKernels<T>::swz(int mode) {
     if constexpr (Elem<T>::complex) {
+        if constexpr (sizeof(T) == 8)
+            if (mode == kDrawn) return reinterpret_cast<const void*>(k_tile_pipe_swz<T, kDrawn>);
         if (mode == kRounds) return reinterpret_cast<const void*>(k_tile_pipe_swz<T, kRounds>);
         if (mode == kMixed) return reinterpret_cast<const void*>(k_tile_pipe_swz<T, kMixed>);
     }
@@ -47,6 +49,8 @@ void PassKernels<T>::launch_swz(int mode, unsigned grid, size_t smem, cudaStream
                                           ctx, tmap);
     };
     if constexpr (Elem<T>::complex) {
+        if constexpr (sizeof(T) == 8)
+            if (mode == kDrawn) return launch(k_tile_pipe_swz<T, kDrawn>, compute_threads<kDrawn>() + 32);
         if (mode == kRounds) return launch(k_tile_pipe_swz<T, kRounds>, compute_threads<kRounds>() + 32);
         if (mode == kMixed) return launch(k_tile_pipe_swz<T, kMixed>, kPipeThreads);
     }

@@ -998,6 +998,19 @@ __device__ __forceinline__ void held_rename(T* v, int code) {
     }
 }
 
+// A dense operator on a held group (a mixture's branch: rare).
+template <typename T, int U, typename W>
+__device__ __forceinline__ void held_dense(W* w, int code, const T* m) {
+    T v[1 << U];
+    memcpy(v, w, sizeof v);
+    switch (code) {
+        LSG_P1(rb_dense1, kT_DENSE1)
+        LSG_P2(rb_dense2, kT_DENSE2)
+        default: break;
+    }
+    memcpy(w, v, sizeof v);
+}
+
 // A group's 2^U elements between shared memory and registers. With vec = 2 or 4 the group's last
 // positions are tile bits (1,) 0: runs of consecutive elements, moved with 8- or 16-byte accesses
 // where the element size allows (the run's address is then aligned: base and off[] have those bits
@@ -1293,6 +1306,13 @@ __device__ __forceinline__ void run_block_swz(T* tile, int tbits, const BlockDes
     }
 }
 
+// How a pass's blocks run.
+constexpr int kPlain = 0;   // plain tiles, any block
+constexpr int kSwz = 1;     // swizzled tiles, register blocks without rounds (fewer registers)
+constexpr int kMixed = 3;   // swizzled tiles, register blocks, rounds among their operators
+constexpr int kRounds = 2;  // swizzled tiles, lowered complex blocks (rounds and renames)
+constexpr int kDrawn = 4;   // kRounds with noise mixtures among them, of a complex64 trajectory pass
+
 // The staged data of one round: its diagonal and rotations at block width 4, in 16-byte words.
 template <typename T>
 constexpr int round_words() {
@@ -1303,7 +1323,7 @@ constexpr int round_words() {
 // their data's shared-memory addresses. Each thread takes NG groups at a time: every coefficient and
 // record read, every dispatch serves them all (a 16-byte read costs four wavefronts even when a
 // whole warp reads one address).
-template <typename T, int U, int NG, int NC>
+template <typename T, int U, int NG, int NC, int MODE = kRounds>
 __device__ __forceinline__ void run_groups(uint32_t t32, const BlockDesc& blk, const BlockMaps<U, NC>& maps,
                                            const OpRec* __restrict__ recs, int groups) {
     using W = typename Held<T>::W;
@@ -1321,6 +1341,11 @@ __device__ __forceinline__ void run_groups(uint32_t t32, const BlockDesc& blk, c
             const uint4 r = lds16(ops + (uint32_t)sizeof(OpRec) * o);  // code, mask, address
             if ((int)r.x == kT_ROUND) {
                 held_round<U, NG>(w, r.z, (int)r.y);
+            } else if (MODE == kDrawn && (int)r.x < kT_X1) {  // a mixture's branch; the identity has code -1
+                const T* m = reinterpret_cast<const T*>((uint64_t)r.w << 32 | r.z);
+                if ((int)r.x >= 0)
+#pragma unroll
+                    for (int k = 0; k < NG; ++k) held_dense<T, U>(w[k], (int)r.x, m);
             } else {
 #pragma unroll
                 for (int k = 0; k < NG; ++k) held_rename<U>(w[k], (int)r.x);
@@ -1330,18 +1355,18 @@ __device__ __forceinline__ void run_groups(uint32_t t32, const BlockDesc& blk, c
         for (int k = 0; k < NG; ++k) maps.template move<W, true>(t32, base[k], w[k]);
     }
 }
-template <typename T, int U, int NC>
+template <typename T, int U, int NC, int MODE = kRounds>
 __device__ __forceinline__ void run_block_rounds(T* tile, int tbits, const BlockDesc& blk, const OpRec* __restrict__ recs) {
     const uint32_t t32 = smem_u32(tile);
     const BlockMaps<U, NC> maps(blk);
     const int groups = 1 << (tbits - U);
     if constexpr (sizeof(T) == 8) {
         if (groups >= 2 * NC) {
-            run_groups<T, U, 2, NC>(t32, blk, maps, recs, groups);
+            run_groups<T, U, 2, NC, MODE>(t32, blk, maps, recs, groups);
             return;
         }
     }
-    run_groups<T, U, 1, NC>(t32, blk, maps, recs, groups);
+    run_groups<T, U, 1, NC, MODE>(t32, blk, maps, recs, groups);
 }
 
 template <typename T>
@@ -1380,16 +1405,36 @@ __device__ void run_ops(T* tile, int tbits, const TileOp* __restrict__ ops, int 
 }
 
 // All blocks of a pass on one tile (the 256 compute threads).
-// MODE: how the pass's blocks run.
-constexpr int kPlain = 0;   // plain tiles, any block
-constexpr int kSwz = 1;     // swizzled tiles, register blocks without rounds (fewer registers)
-constexpr int kMixed = 3;   // swizzled tiles, register blocks, rounds among their operators
-constexpr int kRounds = 2;  // swizzled tiles, lowered complex blocks (rounds and renames)
 template <typename T, int MODE = kPlain>
 __device__ __forceinline__ void compute_tile(T* tile, int K, const PassDesc& pd, const BlockDesc* sblk,
                                              const TileOp* sops, OpRec* recs, const T* __restrict__ data,
                                              int64_t member, const TrajCtx& ctx, uint4* staged = nullptr,
                                              int64_t* staged_member = nullptr) {
+    if constexpr (MODE == kDrawn) {  // the producer has resolved the tile's operators (resolve_drawn)
+        constexpr int NC = 128;
+        if (*staged_member < 0) {  // shared by all members
+            for (int i = threadIdx.x; i < pd.nops * round_words<T>(); i += NC) {
+                const TileOp& op = sops[i / round_words<T>()];
+                const int w = i % round_words<T>();
+                const int have = (int)((((sizeof(T) == 8 ? 2 : 1) << op.k) + op.k) * sizeof(T) + 15) / 16;
+                if (op.tmpl == kT_ROUND && w < have)
+                    staged[op.count * round_words<T>() + w] = __ldg(reinterpret_cast<const uint4*>(data + op.data) + w);
+            }
+            *staged_member = 0;
+        }
+        for (int bi = 0; bi < pd.nblocks; ++bi) {
+            const BlockDesc& blk = sblk[bi];
+            cbar<NC>();
+            switch (blk.u) {
+                case 1: run_block_rounds<T, 1, NC, MODE>(tile, K, blk, recs); break;
+                case 2: run_block_rounds<T, 2, NC, MODE>(tile, K, blk, recs); break;
+                case 3: run_block_rounds<T, 3, NC, MODE>(tile, K, blk, recs); break;
+                default: run_block_rounds<T, 4, NC, MODE>(tile, K, blk, recs); break;
+            }
+        }
+        cbar<NC>();
+        return;
+    }
     if constexpr (MODE == kRounds) {
         constexpr int NC = 128;
         // The rounds' data and the records of this tile's member, once for consecutive tiles of one
@@ -1508,11 +1553,23 @@ constexpr int pipe_ctas() {
 // pairs chunks 2q and 2q+1 (they differ in register bit hi[0]) in one 3-D box of 1 KB; larger
 // chunks move as 2-D boxes of min(chunk, 16 KB). Otherwise one plain bulk copy per chunk.
 // `pred` (trajectories): members without predicate bit pd.slot are passed over by both sides.
-template <typename T, bool Swz = false, int NC = kCompute, typename F>
+// `resolve(buffer, member)`, if any, runs on the producer warp with each tile's load and is seen by the
+// compute threads of that tile.
+struct NoResolve {};
+template <typename G>
+constexpr bool resolves() {
+    return true;
+}
+template <>
+constexpr bool resolves<NoResolve>() {
+    return false;
+}
+template <typename T, bool Swz = false, int NC = kCompute, typename F, typename G = NoResolve>
 __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_elems, const PassDesc& pd, T* buf0,
                                          T* buf1, uint64_t* full, uint64_t* empty, int64_t tiles_per_member,
                                          int64_t total_tiles, int* status, F&& compute, const Tmap* tmap = nullptr,
-                                         int64_t first = -1, int64_t stride = 0, const uint64_t* pred = nullptr) {
+                                         int64_t first = -1, int64_t stride = 0, const uint64_t* pred = nullptr,
+                                         G resolve = G()) {
     const int K = pd.K, L = pd.L;
     const int nchunks = 1 << (K - L);
     const uint32_t chunk_bytes = (uint32_t)(sizeof(T) << L);
@@ -1590,7 +1647,11 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
             T* mem;
             uint64_t base;
             tile_at(t, &mem, &base);
-            if (lane == 0) mbar_arrive_expect_tx(&full[b], chunk_bytes * (uint32_t)nchunks);
+            constexpr bool early = !resolves<G>();
+            if (lane == 0) {
+                if (early) mbar_arrive_expect_tx(&full[b], chunk_bytes * (uint32_t)nchunks);
+                else mbar_expect_tx(&full[b], chunk_bytes * (uint32_t)nchunks);
+            }
             __syncwarp();
             if constexpr (Swz) {
                 for (int q = lane; q < nboxes; q += 32) copy_in(box_elem(mem, base, q), buf + (size_t)q * box_elems, &full[b]);
@@ -1598,6 +1659,11 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
                 for (int c = lane; c < nchunks; c += 32)
                     bulk_g2s(buf + ((size_t)c << L), mem + (base | deposit((uint64_t)c, pd.hi, K - L)), chunk_bytes,
                              &full[b]);
+            }
+            if constexpr (!early) {  // while the copies run; the arrival releases what it wrote
+                resolve(b, t / tiles_per_member);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[b]);
             }
             ++it;
         }
@@ -1623,7 +1689,8 @@ __device__ __forceinline__ void pipe_run(T* __restrict__ state, int64_t member_e
         T* tile = b ? buf1 : buf0;
         const bool ok = mbar_wait_bounded(&full[b], (uint32_t)((it >> 1) & 1), status);
         if (cbar_or<NC>(!ok)) return;  // every compute thread leaves together on a timeout
-        compute(tile, t / tiles_per_member);
+        if constexpr (!resolves<G>()) compute(tile, t / tiles_per_member);
+        else compute(tile, t / tiles_per_member, b);
         fence_proxy_async_smem();  // this thread's writes, before the producer's bulk store reads them
         mbar_arrive(&empty[b]);
         ++it;
@@ -1668,19 +1735,43 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_ctas<T>()) k_tile_pipe(T* _
                 nullptr, -1, 0, ctx.pred);
 }
 
+// The records of a tile's operators for its member, by the producer warp (kDrawn): a round's staged data,
+// a mixture's branch from the member's uniform (code -1: the identity). Resolved by the compute
+// threads they kept every tile waiting for three dependent reads of global memory. Measured, 512 shots
+// of 18 qubits x 16 rounds: 40 passes over all shots and 64 over a branch's 61.7 -> 37.0 ms, 0.7 ms a full
+// pass of 1 GiB (0.32 at the copy rate).
+template <typename T>
+__device__ __forceinline__ void resolve_drawn(const PassDesc& pd, const TileOp* sops, OpRec* recs, const uint4* staged,
+                                              const T* __restrict__ data, int64_t member, const TrajCtx& ctx) {
+    const int64_t cur = ctx.u ? ctx.cursor[member] : 0;
+    for (int o = threadIdx.x & 31; o < pd.nops; o += 32) {
+        const TileOp& op = sops[o];
+        OpRec r{op.tmpl, op.zmask, nullptr};
+        if (op.tmpl == kT_ROUND) {
+            r.m = reinterpret_cast<const void*>((uintptr_t)smem_u32(staged + op.count * round_words<T>()));
+        } else if (op.kind == kOpMixture) {
+            const T* m = ctx.u ? mixture_pick<T>(op, data + op.data + member * op.stride, ctx.u[member * ctx.ustride + cur + op.draw])
+                               : nullptr;
+            r.m = m;
+            r.code = m ? (op.k == 1 ? kT_DENSE1 : kT_DENSE2) + (op.tmpl - (op.k == 1 ? kT_MIX1 : kT_MIX2)) : -1;
+        }
+        recs[o] = r;
+    }
+}
+
 // The same pass on tiles moved by swizzled tensor copies, the register blocks addressing them through
 // their GF(2) maps. Plain tiles of 512-byte chunks put every group of a block on low register bits
 // into the same banks (8-way conflicts: 9,700 cycles a block, where the arithmetic takes a
 // tenth); the swizzle, with the lanes driving bits that reach different banks, leaves one or two.
 template <int MODE>
 constexpr int compute_threads() {
-    return MODE == kRounds ? 128 : kCompute;
+    return MODE == kRounds || MODE == kDrawn ? 128 : kCompute;
 }
 // CTAs per SM the swizzled kernels are compiled for. Lowered passes run 128 threads with 16
 // (complex128) or 32 (complex64) amplitudes each: their registers leave room for two and three CTAs.
 template <typename T, int MODE>
 constexpr int swz_ctas() {
-    return MODE == kRounds ? (sizeof(T) == 8 ? 3 : 2) : pipe_ctas<T>();
+    return MODE == kRounds || MODE == kDrawn ? (sizeof(T) == 8 ? 3 : 2) : pipe_ctas<T>();
 }
 template <typename T, int MODE>
 __global__ void __launch_bounds__(compute_threads<MODE>() + 32, (swz_ctas<T, MODE>())) k_tile_pipe_swz(T* __restrict__ state, int64_t member_elems,
@@ -1702,10 +1793,20 @@ __global__ void __launch_bounds__(compute_threads<MODE>() + 32, (swz_ctas<T, MOD
     OpRec* recs = reinterpret_cast<OpRec*>(sblk + pass_g->nblocks);
     if (threadIdx.x == 0) pd = *pass_g;
     stage_pass<T>(pass_g, ops, blocks, sops, sblk);
-    uint4* staged = reinterpret_cast<uint4*>(recs + pass_g->nops);
+    uint4* staged = reinterpret_cast<uint4*>(recs + (MODE == kDrawn ? 2 : 1) * pass_g->nops);
     pipe_init<compute_threads<MODE>()>(full, empty);
     __syncthreads();
     int64_t staged_member = -1;
+    if constexpr (MODE == kDrawn) {  // two sets of records, one per tile buffer
+        const int nops = pd.nops;
+        pipe_run<T, true, compute_threads<MODE>()>(state, member_elems, pd, buf0, buf1, full, empty, tiles_per_member, total_tiles, status,
+                          [&](T* tile, int64_t member, int b) {
+                              compute_tile<T, MODE>(tile, pd.K, pd, sblk, sops, recs + b * nops, data, member, ctx, staged, &staged_member);
+                          },
+                          &tmap, -1, 0, ctx.pred,
+                          [&](int b, int64_t member) { resolve_drawn<T>(pd, sops, recs + b * nops, staged, data, member, ctx); });
+        return;
+    }
     pipe_run<T, true, compute_threads<MODE>()>(state, member_elems, pd, buf0, buf1, full, empty, tiles_per_member, total_tiles, status,
                       [&](T* tile, int64_t member) {
                           compute_tile<T, MODE>(tile, pd.K, pd, sblk, sops, recs, data, member, ctx, staged, &staged_member);
