@@ -36,8 +36,8 @@ template <typename T>
 void PassKernels<T>::launch_pipe(unsigned grid, size_t smem, cudaStream_t st, T* state, int64_t member_elems,
                                  const PassDesc* pass, const TileOp* ops, const BlockDesc* blocks, const T* data,
                                  int64_t tiles_per_member, int64_t total_tiles, int* status, const TrajCtx& ctx) {
-    k_tile_pipe<T><<<grid, kPipeThreads, smem, st>>>(state, member_elems, pass, ops, blocks, data, tiles_per_member,
-                                                     total_tiles, status, ctx);
+    launch_chained(total_tiles <= 16 * (int64_t)grid, k_tile_pipe<T>, grid, kPipeThreads, smem, st, state, member_elems, pass, ops, blocks, data,
+                   tiles_per_member, total_tiles, status, ctx);
 }
 template <typename T>
 void PassKernels<T>::launch_swz(int mode, unsigned grid, size_t smem, cudaStream_t st, T* state, int64_t member_elems,
@@ -45,8 +45,8 @@ void PassKernels<T>::launch_swz(int mode, unsigned grid, size_t smem, cudaStream
                                 int64_t tiles_per_member, int64_t total_tiles, int* status, const TrajCtx& ctx,
                                 const Tmap& tmap) {
     auto launch = [&](auto kern, int threads) {
-        kern<<<grid, threads, smem, st>>>(state, member_elems, pass, ops, blocks, data, tiles_per_member, total_tiles, status,
-                                          ctx, tmap);
+        launch_chained(total_tiles <= 16 * (int64_t)grid, kern, grid, threads, smem, st, state, member_elems, pass, ops, blocks, data, tiles_per_member,
+                       total_tiles, status, ctx, tmap);
     };
     if constexpr (Elem<T>::complex) {
         if constexpr (sizeof(T) == 8)

@@ -1730,6 +1730,8 @@ __global__ void __launch_bounds__(kPipeThreads, pipe_ctas<T>()) k_tile_pipe(T* _
     stage_pass<T>(pass_g, ops, blocks, sops, sblk);
     pipe_init(full, empty);
     __syncthreads();
+    chain_trigger();
+    chain_wait();  // (the pass's operators are older than the kernel before)
     pipe_run<T>(state, member_elems, pd, buf0, buf1, full, empty, tiles_per_member, total_tiles, status,
                 [&](T* tile, int64_t member) { compute_tile<T>(tile, pd.K, pd, sblk, sops, recs, data, member, ctx); },
                 nullptr, -1, 0, ctx.pred);
@@ -1796,6 +1798,8 @@ __global__ void __launch_bounds__(compute_threads<MODE>() + 32, (swz_ctas<T, MOD
     uint4* staged = reinterpret_cast<uint4*>(recs + (MODE == kDrawn ? 2 : 1) * pass_g->nops);
     pipe_init<compute_threads<MODE>()>(full, empty);
     __syncthreads();
+    chain_trigger();
+    chain_wait();
     int64_t staged_member = -1;
     if constexpr (MODE == kDrawn) {  // two sets of records, one per tile buffer
         const int nops = pd.nops;

@@ -100,6 +100,8 @@ __global__ void k_t_basis(Cx<R>* state, int64_t elems, int64_t total) {
 }
 
 __global__ void k_t_advance(int64_t* cursor, const uint64_t* pred, int slot, int64_t count, int64_t batch) {
+    chain_trigger();
+    chain_wait();
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x)
         if (has(pred, b, slot)) cursor[b] += count;
 }
@@ -109,6 +111,7 @@ __global__ void k_t_advance(int64_t* cursor, const uint64_t* pred, int slot, int
 template <typename R>
 __global__ void k_t_p1(const Cx<R>* __restrict__ state, int64_t elems, int q, const uint64_t* pred, int slot,
                        double* __restrict__ partials) {
+    chain_trigger();
     const int64_t b = blockIdx.y;
     double acc = 0.0;
     if (has(pred, b, slot)) {
@@ -163,10 +166,12 @@ __device__ __forceinline__ void set_last(uint64_t* last, int q, int v) {
 
 // one warp per member: sum the partials, draw the outcome (and the readout flip), record the classical
 // bit and the qubit's value
-__global__ void k_t_decide(const double* __restrict__ partials, int nparts, int64_t* cursor, const double* __restrict__ u,
+__global__ void k_t_decide(const double* partials, int nparts, int64_t* cursor, const double* __restrict__ u,
                            int64_t ustride, const uint64_t* pred, int slot, int q, int clbit, int readout, double p01,
                            double p10, int is_reset, uint64_t* clbits, int words, uint64_t* last, int* outcome,
                            double* prob, unsigned long long* near, int64_t batch) {
+    chain_trigger();
+    chain_wait();
     const int lane = threadIdx.x & 31;
     for (int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; b < batch;
          b += ((int64_t)gridDim.x * blockDim.x) >> 5) {
@@ -202,6 +207,7 @@ template <typename R>
 __global__ void k_t_collapse(Cx<R>* __restrict__ state, int64_t elems, int q, const int* outcome, const double* prob,
                              int is_reset, int q_next, const uint64_t* pred, int slot_next,
                              double* __restrict__ partials) {
+    chain_trigger();
     const int64_t b = blockIdx.y;
     const int out = outcome[b];
     const bool want = q_next >= 0 && has(pred, b, slot_next);
@@ -344,6 +350,7 @@ constexpr int kGroupUnroll = 4;  // groups per lane per iteration: independent l
 template <typename R>
 __global__ void k_t_hist(const Cx<R>* __restrict__ state, int64_t elems, Group gr, const uint64_t* pred, int slot,
                          double* __restrict__ partials) {
+    chain_trigger();
     __shared__ double buf[kT];
     const int64_t b = blockIdx.y;
     const int k = threadIdx.x & ((1 << gr.g) - 1);
@@ -379,10 +386,12 @@ __global__ void k_t_hist(const Cx<R>* __restrict__ state, int64_t elems, Group g
 // one thread per member: the group's outcomes in program order from the joint bins, each with its
 // readout flip and classical bit as k_t_decide records them; outcome[b] = drawn pattern | final
 // pattern << 8 (-1: not taken), prob[b] = the scale that renormalises the kept slice
-__global__ void k_t_decide_group(const double* __restrict__ partials, int nparts, int64_t* cursor,
+__global__ void k_t_decide_group(const double* partials, int nparts, int64_t* cursor,
                                  const double* __restrict__ u, int64_t ustride, const uint64_t* pred, int slot, Group gr,
                                  uint64_t* clbits, int words, uint64_t* last, int* outcome, double* prob,
                                  unsigned long long* near, int64_t batch) {
+    chain_trigger();
+    chain_wait();
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
         if (!has(pred, b, slot)) {
             outcome[b] = -1;
@@ -427,6 +436,8 @@ __global__ void k_t_decide_group(const double* __restrict__ partials, int nparts
 __global__ void k_t_decide_known(int64_t* cursor, const double* __restrict__ u, int64_t ustride, const uint64_t* pred,
                                  int slot, Group gr, uint64_t* clbits, int words, uint64_t* last, int* outcome,
                                  double* prob, unsigned long long* near, int64_t batch) {
+    chain_trigger();
+    chain_wait();
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
         outcome[b] = -1;
         if (!has(pred, b, slot)) continue;
@@ -454,6 +465,7 @@ __global__ void k_t_decide_known(int64_t* cursor, const double* __restrict__ u, 
 template <typename R>
 __global__ void k_t_collapse_group(Cx<R>* __restrict__ state, int64_t elems, Group gr, const int* outcome,
                                    const double* prob) {
+    chain_trigger();
     const int64_t b = blockIdx.y;
     const int oc = outcome[b];
     if (oc < 0) return;  // the whole block leaves: the member is not in this branch
@@ -498,6 +510,7 @@ __global__ void k_t_collapse_group(Cx<R>* __restrict__ state, int64_t elems, Gro
 template <typename R>
 __global__ void k_t_rdm(const Cx<R>* __restrict__ state, int64_t elems, int k, int b0, int b1, const uint64_t* pred,
                         int slot, double* __restrict__ partials) {
+    chain_trigger();
     const int64_t b = blockIdx.y;
     const int d = 1 << k;
     double acc[32];
@@ -533,10 +546,12 @@ __global__ void k_t_rdm(const Cx<R>* __restrict__ state, int64_t elems, int k, i
 // one thread per member: Born weights Tr(K rho K^dagger) in order, pick by the member's uniform,
 // write K/sqrt(w) (or the identity when no branch has weight) for the member
 template <typename R>
-__global__ void k_t_kraus_decide(const double* __restrict__ partials, int nparts, int k, const double* __restrict__ kraus,
+__global__ void k_t_kraus_decide(const double* partials, int nparts, int k, const double* __restrict__ kraus,
                                  int nkraus, int64_t* cursor, const double* __restrict__ u, int64_t ustride,
                                  const uint64_t* pred, int slot, Cx<R>* dyn, int* apply, unsigned long long* near,
                                  int64_t batch) {
+    chain_trigger();
+    chain_wait();
     const int d = 1 << k;
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
         apply[b] = 0;
@@ -588,6 +603,7 @@ __global__ void k_t_kraus_decide(const double* __restrict__ partials, int nparts
 template <typename R>
 __global__ void k_t_apply_dyn(Cx<R>* __restrict__ state, int64_t elems, int k, int b0, int b1, const Cx<R>* dyn,
                               const int* apply) {
+    chain_trigger();
     const int64_t b = blockIdx.y;
     if (!apply[b]) return;
     const int d = 1 << k;
@@ -621,6 +637,8 @@ struct Cond {
 
 __global__ void k_t_if(uint64_t* pred, const uint64_t* clbits, int words, int parent, int then_slot, int else_slot,
                        Cond c, int64_t batch) {
+    chain_trigger();
+    chain_wait();
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < batch; b += (int64_t)gridDim.x * blockDim.x) {
         uint64_t p = pred[b] & ~((1ull << then_slot) | (1ull << else_slot));
         if ((p >> parent) & 1) {
@@ -755,7 +773,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
         switch (sp.kind) {
             case STEP_SEG: LSG_CHECK(program_run_ctx(sp.seg, s, nullptr, ctx)); break;
             case STEP_ADVANCE:
-                k_t_advance<<<t_grid(B), kT, 0, st>>>(c.cursor, c.pred, sp.slot, sp.count, B);
+                launch_chained(true, k_t_advance, t_grid(B), kT, 0, st, c.cursor, c.pred, sp.slot, sp.count, B);
                 break;
             case STEP_MEASURE: {
                 double* part = (double*)t->parts.ptr;
@@ -773,7 +791,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                         gr.p10[i] = m.p10;
                     }
                     if (sp.known) {
-                        k_t_decide_known<<<t_grid(B), kT, 0, st>>>(c.cursor, u, ustride, c.pred, sp.slot, gr, c.clbits, t->words,
+                        launch_chained(true, k_t_decide_known, t_grid(B), kT, 0, st, c.cursor, u, ustride, c.pred, sp.slot, gr, c.clbits, t->words,
                                                                   c.last, c.outcome, c.prob, c.near, B);
                         bool moves = false;  // only a reset of a 1 moves amplitudes
                         for (int i = 0; i < glen; ++i) moves = moves || gr.is_reset[i];
@@ -783,7 +801,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                         }
                     } else {
                         k_t_hist<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, gr, c.pred, sp.slot, part);
-                        k_t_decide_group<<<t_grid(B), kT, 0, st>>>(part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, gr,
+                        launch_chained(true, k_t_decide_group, t_grid(B), kT, 0, st, part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, gr,
                                                                   c.clbits, t->words, c.last, c.outcome, c.prob, c.near, B);
                     }
                     k_t_collapse_group<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, gr, c.outcome, c.prob);
@@ -792,7 +810,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                 }
                 if (!p1_ready)
                     k_t_p1<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.q, c.pred, sp.slot, part);
-                k_t_decide<<<t_grid(B * 32), kT, 0, st>>>(part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.q, sp.clbit,
+                launch_chained(true, k_t_decide, t_grid(B * 32), kT, 0, st, part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.q, sp.clbit,
                                                          sp.readout, sp.p01, sp.p10, sp.is_reset, c.clbits, t->words, c.last,
                                                          c.outcome, c.prob, c.near, B);
                 // a measurement right after this one: its p(1) partials come out of this collapse
@@ -809,7 +827,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                 const unsigned gk = B > 16 ? gx : (gx + 3) / 4;
                 k_t_rdm<R><<<dim3(gk, (unsigned)B), kT, 0, st>>>(state, elems, sp.k, sp.bits[0], sp.bits[1], c.pred,
                                                                sp.slot, part);
-                k_t_kraus_decide<R><<<t_grid(B), kT, 0, st>>>(part, (int)gk, sp.k, (const double*)t->kraus.ptr + 2 * sp.kraus_at,
+                launch_chained(true, k_t_kraus_decide<R>, t_grid(B), kT, 0, st, part, (int)gk, sp.k, (const double*)t->kraus.ptr + 2 * sp.kraus_at,
                                                              sp.nkraus, c.cursor, u, ustride, c.pred, sp.slot,
                                                              (Cx<R>*)t->dyn.ptr, c.apply, c.near, B);
                 k_t_apply_dyn<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.k, sp.bits[0], sp.bits[1],
@@ -822,7 +840,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                 cd.negate = sp.negate;
                 cd.value = sp.value;
                 for (int i = 0; i < sp.ncond; ++i) cd.bits[i] = sp.cond[i];
-                k_t_if<<<t_grid(B), kT, 0, st>>>(c.pred, c.clbits, t->words, sp.slot, sp.then_slot, sp.else_slot, cd, B);
+                launch_chained(true, k_t_if, t_grid(B), kT, 0, st, c.pred, c.clbits, t->words, sp.slot, sp.then_slot, sp.else_slot, cd, B);
                 break;
             }
             default: break;
