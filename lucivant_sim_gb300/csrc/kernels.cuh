@@ -14,7 +14,7 @@ struct PassKernels {
     static const void* swz(int mode);
     static const void* pass();
     static const void* ragged();
-    // k_tile_pipe<T> and k_tile_pipe_swz<T, mode> with kPipeThreads threads (kRounds: 160), k_tile_pass<T> with 256, k_tile_pipe_ragged<T>
+    // k_tile_pipe<T> and k_tile_pipe_swz<T, mode> with kPipeThreads threads (kRounds, kDrawn: 160), k_tile_pass<T> with 256, k_tile_pipe_ragged<T>
     static void launch_pipe(unsigned grid, size_t smem, cudaStream_t st, T* state, int64_t member_elems,
                             const PassDesc* pass, const TileOp* ops, const BlockDesc* blocks, const T* data,
                             int64_t tiles_per_member, int64_t total_tiles, int* status, const TrajCtx& ctx);

@@ -67,7 +67,7 @@ struct TileOp {
     long long stride;  // per batch member, complex entries
     int pred;       // predicate bit the member must have set (0: always set)
     int draw;       // trajectory ops: uniform offset from the member's cursor
-    int count;      // mixture branches
+    int count;      // mixture branches; a round: its number in the pass
     int tmpl;       // register-block code: kind and positions (see tile.cuh)
     int pos[8];     // positions of the operator's bits within its block (0 = block MSB)
     int zmask;      // trace-preserving 4x4 operators: coefficients zero for every member
