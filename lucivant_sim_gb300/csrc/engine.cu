@@ -1043,11 +1043,12 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     const bool drawn = rounds && trajectory && precision == LSG_C64;
     const int seg_pred = pred && nops > 0 ? pred[0] : 0;
     for (int32_t i = 0; pred && i < nops; ++i) rounds = rounds && pred[i] == seg_pred;
-    std::vector<double> grown;
+    std::vector<double> grown, grown_low;
+    const int64_t own = 2 * pool_entries;
     std::vector<char> moved;
     if (rounds && nops > 0) {
         grown.assign(pool, pool + 2 * pool_entries);
-        moved = move_outer_factors(p->plan, batch, grown);
+        moved = move_outer_factors(p->plan, batch, grown, grown_low);
         pool = grown.data();
         pool_entries = (int64_t)grown.size() / 2;
     }
@@ -1088,7 +1089,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 pure = pure && held(p->plan.ops[o].tmpl);
             LoweredBlock& low = lowered[i];
             if (pure) continue;
-            lower_block(p->plan, pd, blk, moved, batch, pool, round_cost, true, &low);
+            lower_block(p->plan, pd, blk, moved, batch, Pool{pool, grown_low.data(), own}, round_cost, true, &low);
             whole_pass = low.members == 1 && !low.items.empty() && (int)low.items.size() <= blk.nops;
             for (const LoweredItem& it : low.items) whole_pass = whole_pass && (it.code != kKeepOp || held(it.tmpl));
         }
@@ -1109,7 +1110,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 if (dense) cost = std::min(cost, 1.1 * ((double)(1 << blk.u) + overhead + (double)(1 << blk.u) / 16.0));
                 LoweredBlock low;
                 if (ready) low = std::move(lowered[bi - pd.first_block]);
-                if (ready || (lower_block(p->plan, pd, blk, moved, batch, pool, overhead, precision == LSG_C64, &low) &&
+                if (ready || (lower_block(p->plan, pd, blk, moved, batch, Pool{pool, grown_low.data(), own}, overhead, precision == LSG_C64, &low) &&
                               low.cost < cost)) {
                     const int D = 1 << blk.u;
                     std::vector<TileOp> made;

@@ -6,16 +6,16 @@
 // it costs 2: the rotation is one multiply-add per real component, because its cosine is taken out
 // as a factor, and every diagonal next to it (e, s, P, diagonal gates) merges over the whole
 // block into one multiplication by a table of 2^u entries (4 multiply-adds per amplitude, shared
-// by all rotations of the round). Leaving the cosine out loses nothing: a0 - t * a1 is one fused
-// multiply-add, its error is relative to the result, and t <= 1 (the larger of cosine and sine
-// is the one taken out, `flip` says which), so the four rotations of a round grow an amplitude
-// by at most 4, which the diagonal's factor has taken back before. complex64 rounds
+// by all rotations of the round). The cosine left out costs no accuracy in the arithmetic:
+// a0 - t * a1 is one fused multiply-add, its error is relative to the result, and t <= 1 (the larger
+// of cosine and sine is the one taken out, `flip` says which), so the four rotations of a round grow
+// an amplitude by at most 4, which the diagonal's factor has taken back before. complex64 rounds
 // keep the cosine in the rotation (tile.cuh rb_round).
 //
 // The outer factor P need not stay in the block: a qubit that controls a cx (or meets a diagonal)
 // passes a phase through it, and a cx's target passes a rotation about X, so P is taken as whichever
 // the qubit's next operators let through and multiplied into the next one-bit operator on that
-// qubit, in FP64 on the host. A brickwork layer then costs one diagonal per block, and no diagonal
+// qubit, on the host. A brickwork layer then costs one diagonal per block, and no diagonal
 // is left over behind it.
 //
 // Everything here is decided per member from that member's own data, or from the operators'
@@ -41,91 +41,147 @@ constexpr double kUnitary = 2e-15;
 // factors): taken as one, so the diagonal that would hold it is left out.
 constexpr double kResidue = 1e-15;
 
+// A real as v + e, e what the roundings of the operations that made v left over, to first order. A
+// rotation or a diagonal's entry takes some twenty operations from the matrices it comes from, and its
+// error is common to all amplitudes it multiplies: coefficients formed in double precision were
+// most of a program's error. Each is now rounded once. Measured, 12 seeds of 11 qubits x 20 layers
+// of u3 and cx in complex128, against the gates as given (their double matrices) in 80 bits: 2.6e-15
+// before, 1.4e-15 now, dense products 1.1e-15; against the gates the angles stand for: 3.3e-15 before,
+// 2.9e-15 now, dense products 3.1e-15. The arithmetic on the amplitudes has 0.8e-15 of it.
+// (inlined by force: as calls, g++ 13 loses parts of the pairs it holds in vector registers at -O1 and -O2
+// with FMA instructions)
+#define LSG_INLINE __attribute__((always_inline)) inline
+struct Two {
+    double v = 0.0, e = 0.0;
+    Two() = default;
+    Two(double x, double y = 0.0) : v(x), e(y) {}
+    double value() const { return v + e; }
+};
+LSG_INLINE Two operator-(Two a) { return Two(-a.v, -a.e); }
+LSG_INLINE Two operator+(Two a, Two b) {
+    const double s = a.v + b.v, t = s - a.v;
+    return Two(s, ((a.v - (s - t)) + (b.v - t)) + (a.e + b.e));
+}
+LSG_INLINE Two operator-(Two a, Two b) { return a + -b; }
+LSG_INLINE Two operator*(Two a, Two b) {
+    const double p = a.v * b.v;
+    return Two(p, std::fma(a.v, b.v, -p) + (a.v * b.e + a.e * b.v));
+}
+LSG_INLINE Two tidy(Two a) {  // v the rounding of the sum (after a cancellation it may not be)
+    const double s = a.v + a.e;
+    return Two(s, a.e - (s - a.v));
+}
+LSG_INLINE Two operator/(Two a, Two b) {
+    b = tidy(b);
+    const double q = a.v / b.v;
+    return Two(q, (std::fma(-q, b.v, a.v) + (a.e - q * b.e)) / b.v);
+}
+LSG_INLINE Two root(Two a) {
+    a = tidy(a);
+    if (!(a.v > 0.0)) return Two();
+    const double r = std::sqrt(a.v);
+    return Two(r, (std::fma(-r, r, a.v) + a.e) / (2.0 * r));
+}
+
+struct Cpx {
+    Two re, im;
+    Cpx() = default;
+    Cpx(double x) : re(x) {}
+    Cpx(Two x, Two y) : re(x), im(y) {}
+    cd value() const { return cd(re.value(), im.value()); }
+    bool one() const { return re.v + re.e == 1.0 && im.v + im.e == 0.0; }
+};
+LSG_INLINE Cpx conj(Cpx a) { return Cpx(a.re, -a.im); }
+LSG_INLINE Cpx operator-(Cpx a) { return Cpx(-a.re, -a.im); }
+LSG_INLINE Cpx operator+(Cpx a, Cpx b) { return Cpx(a.re + b.re, a.im + b.im); }
+LSG_INLINE Cpx operator*(Cpx a, Cpx b) { return Cpx(a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re); }
+LSG_INLINE Cpx operator*(Cpx a, Two b) { return Cpx(a.re * b, a.im * b); }
+LSG_INLINE Cpx operator/(Cpx a, Two b) { return a * (Two(1.0) / b); }
+LSG_INLINE Two norm(Cpx a) { return a.re * a.re + a.im * a.im; }
+LSG_INLINE bool zero(Cpx a) { return a.re.v == 0.0 && a.im.v == 0.0; }
+// a phase, exactly one where it is the rounding of one
+LSG_INLINE Cpx settled(Cpx a) {
+    const double x = a.re.v - 1.0, y = a.im.v;
+    return x * x + y * y < kResidue * kResidue ? Cpx(1.0) : a;
+}
+
 struct Mat {
-    cd a, b, c, d;  // rows (a, b), (c, d)
+    Cpx a, b, c, d;  // rows (a, b), (c, d)
 };
 
 Mat mul(const Mat& x, const Mat& y) {
     return Mat{x.a * y.a + x.b * y.c, x.a * y.b + x.b * y.d, x.c * y.a + x.d * y.c, x.c * y.b + x.d * y.d};
 }
 
-// 1 / sqrt(x + y * y + z * z) with the rounding of the result beside it (one Newton step on the exact
-// residual).
-struct Exact {
-    double v, err;
+// The matrix nearest to m whose columns are orthogonal, [[a, -w * conj(c)], [c, w * conj(a)]]: what m is
+// away from it is the rounding of its entries. (The columns keep their lengths and phases, six of m's
+// eight real numbers. The nearest unitary matrix keeps four: 1.6e-15 against the gates as given,
+// 2.7e-15 against those the angles stand for.) False when m is farther than rounding.
+struct Unitary {
+    Cpx a, c, w;
 };
-Exact inverse_length(double x, double y, double z) {
-    const double yy = y * y, ye = std::fma(y, y, -yy), zz = z * z, ze = std::fma(z, z, -zz);
-    const double a = x + yy, at = a - x, ae = (x - (a - at)) + (yy - at);
-    const double h = a + zz, ht = h - a, he = (a - (h - ht)) + (zz - ht) + ae + ye + ze;
-    const double r = 1.0 / std::sqrt(h);
-    const double q = r * r, qe = std::fma(r, r, -q);
-    return Exact{r, 0.5 * r * (std::fma(-h, q, 1.0) - h * qe - he * q)};
+bool nearest(const Mat& m, Unitary* out) {
+    const Two all = norm(m.a) + norm(m.b) + norm(m.c) + norm(m.d);
+    if (!(all.v > 0.0) || !std::isfinite(all.v)) return false;
+    const Cpx lean = (conj(m.a) * m.b + conj(m.c) * m.d) / all;  // the columns' product, over twice their length
+    if (!(std::fabs(lean.re.v) + std::fabs(lean.im.v) <= kUnitary)) return false;
+    out->a = m.a + -(m.b * conj(lean));
+    out->c = m.c + -(m.d * conj(lean));
+    out->w = (m.a * m.d + -(m.b * m.c)) / (norm(out->a) + norm(out->c));
+    return std::fabs(norm(out->w).v - 1.0) <= 2.0 * kUnitary;
+}
+
+Mat matrix(const Unitary& u) { return Mat{u.a, -(u.w * conj(u.c)), u.c, u.w * conj(u.a)}; }
+
+// The phase ph of u = diag(1, ph) * N with N's first column in a real, positive ratio.
+Cpx outer_phase(const Unitary& u) {
+    if (zero(u.a) || zero(u.c)) return 1.0;
+    const Cpx ph = u.c * conj(u.a);
+    return settled(ph / root(norm(ph)));
+}
+Unitary without_phase(const Unitary& u, Cpx ph) {
+    return ph.one() ? u : Unitary{u.a, u.c * conj(ph), u.w * conj(ph)};
 }
 
 // s * R * diag(1, e), R = [[1, -t], [t, 1]] or, with flip, [[t, -1], [1, t]]
 struct Rotation {
-    cd s, s_err{0.0}, e;
-    double t = 0.0, sine = 0.0;
+    Cpx s, e;
+    Two t;
+    double sine = 0.0;
     bool flip = false;
 };
 
-// m as a rotation; false when its first column has no real ratio or it is not that to rounding.
+// m, its columns orthogonal, as a rotation; false when its first column has no real ratio.
 bool rotation(const Mat& m, Rotation* out) {
-    const double p = std::abs(m.a), q = std::abs(m.c);
-    const double big = std::max(p, q);
-    if (!(big > 0.0) || !std::isfinite(big)) return false;
-    out->flip = q > p;
-    cd r, miss;
-    if (!out->flip) {
-        r = m.c / m.a;
-        out->s = m.a;
-        out->e = m.d / m.a;
-        miss = m.b + r.real() * out->e * m.a;
-    } else {
-        r = m.a / m.c;
-        out->s = m.c;
-        out->e = -m.b / m.c;
-        miss = m.d - r.real() * out->e * m.c;
-    }
-    out->t = r.real();
-    if (!(std::abs(r.imag()) <= kUnitary) || !(std::abs(miss) <= kUnitary * big)) return false;
-    if (!(std::abs(std::abs(out->e) - 1.0) <= 1e-9)) return false;
-    // A unitary's factor s has modulus 1 / sqrt(1 + t^2): set to it beyond double precision. (Its own
-    // rounding is common to all amplitudes and the norm would drift by it: 1.6e-15 over 20 layers of
-    // 12 qubits, 4e-16 with it set.)
-    if (std::abs(std::norm(out->s) * (1.0 + out->t * out->t) - 1.0) <= 2.0 * kUnitary) {
-        const Exact u = inverse_length(0.0, out->s.real(), out->s.imag()), w = inverse_length(1.0, out->t, 0.0);
-        const double k = u.v * w.v, ke = std::fma(u.v, w.v, -k) + u.v * w.err + u.err * w.v;
-        const double re = out->s.real() * k, im = out->s.imag() * k;
-        out->s_err = cd(std::fma(out->s.real(), k, -re) + out->s.real() * ke, std::fma(out->s.imag(), k, -im) + out->s.imag() * ke);
-        out->s = cd(re, im);
-    }
-    if (std::abs(out->e - 1.0) < kResidue) out->e = 1.0;
+    const Two aa = norm(m.a), cc = norm(m.c);
+    out->flip = cc.v > aa.v;
+    const Cpx top = out->flip ? m.c : m.a, rest = out->flip ? m.a : m.c;
+    const Cpx back = conj(top) / (out->flip ? cc : aa);  // 1 / top
+    const Cpx ratio = rest * back;
+    if (!(std::fabs(ratio.im.v) <= kUnitary) || !std::isfinite(ratio.re.v)) return false;
+    out->t = tidy(ratio.re);
+    // (the rotation as it will be, with the rounded t, has another length)
+    out->s = top * Two(1.0, out->t.v * out->t.e / (1.0 + out->t.v * out->t.v));
+    out->e = settled((out->flip ? -m.b : m.d) * back);
     return true;
 }
 
-// The phase ph of m = diag(1, ph) * N with N's first column in a real, positive ratio.
-cd outer_phase(const Mat& m) {
-    if (m.a == 0.0 || m.c == 0.0) return 1.0;
-    cd ph = m.c * std::conj(m.a);
-    ph /= std::abs(ph);
-    return std::abs(ph - 1.0) < kResidue ? cd(1.0) : ph;
-}
-
-// (divided by the phase as it is, not multiplied by its conjugate: its modulus is one only to
-// rounding, and P * N is m whatever it is)
-Mat without_phase(const Mat& m, cd ph) {
-    return ph == cd(1.0) ? m : Mat{m.a, m.b, m.c / ph, m.d / ph};
-}
-
-// The angle of m = Rx(angle) * N with N's first column in a real ratio, its first entry the larger:
-// Rx turns (y, z) of the column's Bloch vector, so that it ends at y = 0, z >= 0.
-Mat outer_x(const Mat& m) {
-    const double y = 2.0 * (std::conj(m.a) * m.c).imag(), z = std::norm(m.a) - std::norm(m.c);
-    const double angle = (y == 0.0 && z >= 0.0) ? 0.0 : std::atan2(-y, z);
-    const double c = std::cos(0.5 * angle), s = std::sin(0.5 * angle);
-    return Mat{cd(c), cd(0.0, -s), cd(0.0, -s), cd(c)};
+// u = Rx * N with N's first column in a real ratio, its first entry the larger: Rx turns (y, z) of the
+// column's Bloch vector, so that it ends at y = 0, z >= 0. Returns N, Rx in *outer.
+Unitary without_x(const Unitary& u, Mat* outer) {
+    const Two y = (conj(u.a) * u.c).im * Two(2.0), z = norm(u.a) - norm(u.c);
+    const double angle = (y.v == 0.0 && z.v >= 0.0) ? 0.0 : std::atan2(-y.v, z.v);
+    Two co = std::cos(0.5 * angle), si = std::sin(0.5 * angle);
+    // the angle's own rounding: what its sine and cosine leave of y, a turn of the half angle
+    const Two s = si * co * Two(2.0), c = co * co - si * si, left = y * c + z * s, len = root(y * y + z * z);
+    if (len.v > 0.0) {
+        const Two turn = left / len * Two(-0.5), before = co;
+        co = co - si * turn, si = si + before * turn;
+    }
+    const Two unit = Two(1.0) / root(co * co + si * si);
+    const Cpx x(co * unit, Two()), i(Two(), si * unit);
+    *outer = Mat{x, -i, -i, x};
+    return Unitary{x * u.a + i * u.c, i * u.a + x * u.c, u.w};
 }
 
 bool is_dense1(const TileOp& t) {
@@ -133,9 +189,14 @@ bool is_dense1(const TileOp& t) {
 }
 bool is_rename(int code) { return code >= kT_X1 && code < kT_SWAP + 16; }
 
-Mat matrix_of(const TileOp& t, const double* pool, int64_t b) {
-    const double* p = pool + 2 * (t.data + (t.stride ? b * t.stride : 0));
-    return Mat{cd(p[0], p[1]), cd(p[2], p[3]), cd(p[4], p[5]), cd(p[6], p[7])};
+// (entries that move_outer_factors appended have their rounding errors in `low`)
+Mat matrix_of(const TileOp& t, const Pool& pool, int64_t b) {
+    const int64_t at = 2 * (t.data + (t.stride ? b * t.stride : 0));
+    const double* p = pool.data + at;
+    if (at < pool.own) return Mat{Cpx(p[0], p[1]), Cpx(p[2], p[3]), Cpx(p[4], p[5]), Cpx(p[6], p[7])};
+    const double* e = pool.low + (at - pool.own);
+    auto entry = [&](int i) { return Cpx(Two(p[i], e[i]), Two(p[i + 1], e[i + 1])); };
+    return Mat{entry(0), entry(2), entry(4), entry(6)};
 }
 
 // What an operator lets through on its local bit `lb`: 1 phases, 2 rotations about X.
@@ -167,52 +228,38 @@ int rename_of(const TileOp& t, const double* pool, int64_t members) {
     return is(0, 2, 1, 3) ? kT_SWAP + 4 * t.pos[0] + t.pos[1] : -1;
 }
 
-// A product of complex factors with the rounding errors of its steps beside it: a round's factor is
-// common to all amplitudes, so its errors would add up over the program.
-struct Factor {
-    cd v{1.0}, err{0.0};
-    void times(cd x, cd x_err) {
-        auto prod = [](double a, double b, double* e) {
-            const double p = a * b;
-            *e = std::fma(a, b, -p);
-            return p;
-        };
-        auto sum = [](double a, double b, double* e) {
-            const double s = a + b, t = s - a;
-            *e = (a - (s - t)) + (b - t);
-            return s;
-        };
-        double e1, e2, e3, e4, e5, e6;
-        const double re = sum(prod(v.real(), x.real(), &e1), -prod(v.imag(), x.imag(), &e2), &e3);
-        const double im = sum(prod(v.real(), x.imag(), &e4), prod(v.imag(), x.real(), &e5), &e6);
-        err = err * x + v * x_err + cd(e1 - e2 + e3, e4 + e5 + e6);
-        v = cd(re, im);
-    }
-    cd value() const { return v + err; }
-};
-
 // A diagonal over a block's amplitudes, per member, and the positions it depends on by structure.
 constexpr unsigned kNoBit = 1u << 8;
 struct Diagonal {
     int64_t members;
     int D;
-    std::vector<cd> v;
+    std::vector<Cpx> v;
     unsigned dep = 0;
-    Diagonal(int64_t m, int d) : members(m), D(d), v((size_t)(m * d), cd(1.0)) {}
+    Diagonal(int64_t m, int d) : members(m), D(d), v((size_t)(m * d), Cpx(1.0)) {}
     bool one(int64_t b) const {
-        return std::all_of(v.begin() + b * D, v.begin() + (b + 1) * D, [](cd x) { return x == cd(1.0); });
+        return std::all_of(v.begin() + b * D, v.begin() + (b + 1) * D, [](const Cpx& x) { return x.one(); });
     }
     bool one() const {
-        return std::all_of(v.begin(), v.end(), [](cd x) { return x == cd(1.0); });
+        return std::all_of(v.begin(), v.end(), [](const Cpx& x) { return x.one(); });
     }
-    void scale(int64_t b, cd s) {
-        for (int e = 0; e < D; ++e) v[(size_t)(b * D + e)] *= s;
+    void scale(int64_t b, Cpx s) {
+        for (int e = 0; e < D; ++e) times(b, e, s);
+    }
+    void times(int64_t b, int e, Cpx s) {
+        Cpx& x = v[(size_t)(b * D + e)];
+        x = x.one() ? s : x * s;
+    }
+    std::vector<cd> rounded() const {
+        std::vector<cd> out(v.size());
+        std::transform(v.begin(), v.end(), out.begin(), [](const Cpx& x) { return x.value(); });
+        return out;
     }
 };
 
 }  // namespace
 
-std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<double>& pool) {
+std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<double>& pool, std::vector<double>& low) {
+    const int64_t own = (int64_t)pool.size();
     std::vector<char> moved(plan.ops.size(), 0);
     struct Touch {
         int op, lb;
@@ -245,23 +292,24 @@ std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<doub
             const int64_t members = std::max<int64_t>(t.stride ? batch : 1, (int64_t)carry.size());
             std::vector<Mat> m((size_t)members), inner, outer;
             for (int64_t b = 0; b < members; ++b) {
-                m[(size_t)b] = matrix_of(t, pool.data(), b);
+                m[(size_t)b] = matrix_of(t, Pool{pool.data(), low.data(), own}, b);
                 if (!carry.empty()) m[(size_t)b] = mul(m[(size_t)b], carry[carry.size() == 1 ? 0 : (size_t)b]);
             }
             for (int64_t b = 0; b < members && through; ++b) {
-                Rotation r;
-                Mat n, p;
-                if (through & 1) {
-                    const cd ph = outer_phase(m[(size_t)b]);
-                    n = without_phase(m[(size_t)b], ph);
-                    p = Mat{cd(1.0), cd(0.0), cd(0.0), ph};
-                } else {
-                    p = outer_x(m[(size_t)b]);
-                    const double d = p.a.real() * p.a.real() + p.b.imag() * p.b.imag();  // its determinant
-                    n = mul(Mat{p.a / d, -p.b / d, -p.c / d, p.d / d}, m[(size_t)b]);
+                Unitary u;
+                Mat p;
+                if (!nearest(m[(size_t)b], &u)) {
+                    through = 0;
+                    break;
                 }
-                if (!rotation(n, &r)) through = 0;
-                inner.push_back(n);
+                if (through & 1) {
+                    const Cpx ph = outer_phase(u);
+                    u = without_phase(u, ph);
+                    p = Mat{Cpx(1.0), Cpx(0.0), Cpx(0.0), ph};
+                } else {
+                    u = without_x(u, &p);
+                }
+                inner.push_back(matrix(u));
                 outer.push_back(p);
             }
             const bool carried = !carry.empty();
@@ -275,17 +323,18 @@ std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<doub
             t.data = (int64_t)pool.size() / 2;
             t.stride = members > 1 ? 4 : 0;
             for (const Mat& x : m)
-                for (const cd& v : {x.a, x.b, x.c, x.d}) {
-                    pool.push_back(v.real());
-                    pool.push_back(v.imag());
-                }
+                for (const Cpx& v : {x.a, x.b, x.c, x.d})
+                    for (Two part : {tidy(v.re), tidy(v.im)}) {
+                        pool.push_back(part.v);
+                        low.push_back(part.e);
+                    }
         }
     }
     return moved;
 }
 
 bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, const std::vector<char>& moved,
-                 int64_t batch, const double* pool, double overhead, bool whole, LoweredBlock* out) {
+                 int64_t batch, const Pool& pool, double overhead, bool whole, LoweredBlock* out) {
     const int U = blk.u, D = 1 << U;
     const int first = pd.first_op + blk.first, last = first + blk.nops;
     int64_t members = 1;
@@ -299,7 +348,7 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
     int open = -1;              // the round that later rotations may still join
     unsigned in_round = 0, touched = 0;
     Diagonal pre(members, D);   // the open round's diagonal
-    std::vector<Factor> gain((size_t)members);  // the open round's factors taken out
+    std::vector<Cpx> gain((size_t)members, Cpx(1.0));  // the open round's factors taken out
     int rounds = 0, rotations = 0;
     double cost = 0.0;
 
@@ -307,11 +356,11 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
         LoweredItem it;
         it.code = kT_ROUND;  // without rotations
         it.mask = 16;
-        it.diag = d.v;
+        it.diag = d.rounded();
         out->items.push_back(std::move(it));
         touched |= d.dep;
         cost += 1.0 + overhead;
-        std::fill(d.v.begin(), d.v.end(), cd(1.0));
+        std::fill(d.v.begin(), d.v.end(), Cpx(1.0));
         d.dep = 0;
     };
     // The open round is complete: its factor goes into its own diagonal where a member has one, else
@@ -319,14 +368,14 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
     auto close = [&](bool at_end) {
         if (open < 0) return;
         for (int64_t b = 0; b < members; ++b) {
-            if (!pre.one(b) || (at_end && pend.one(b))) pre.scale(b, gain[(size_t)b].value());
-            else pend.scale(b, gain[(size_t)b].value());
+            if (!pre.one(b) || (at_end && pend.one(b))) pre.scale(b, gain[(size_t)b]);
+            else pend.scale(b, gain[(size_t)b]);
         }
         LoweredItem& it = out->items[(size_t)open];
         it.mask = (int)in_round;
         if (!pre.one()) {
             it.mask |= 16;
-            it.diag = pre.v;
+            it.diag = pre.rounded();
         }
         open = -1;
     };
@@ -356,7 +405,7 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
             const int x = bit((code - kT_SWAP) / 4), y = bit((code - kT_SWAP) % 4);
             return ((e & x) != 0) != ((e & y) != 0) ? e ^ x ^ y : e;
         };
-        std::vector<cd> v(pend.v.size());
+        std::vector<Cpx> v(pend.v.size());
         for (int64_t b = 0; b < members; ++b)
             for (int e = 0; e < D; ++e) v[(size_t)(b * D + e)] = pend.v[(size_t)(b * D + src(e))];
         pend.v.swap(v);
@@ -376,27 +425,29 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
         if (is_dense1(t)) {
             const int P = t.pos[0];
             std::vector<Rotation> r((size_t)members);
-            std::vector<cd> post((size_t)members, cd(1.0));
+            std::vector<Cpx> post((size_t)members, Cpx(1.0));
             bool ok = true;
             for (int64_t b = 0; b < members && ok; ++b) {
                 Mat m = matrix_of(t, pool, b);
                 if (!moved[(size_t)o]) {
-                    post[(size_t)b] = outer_phase(m);
-                    m = without_phase(m, post[(size_t)b]);
+                    Unitary u;
+                    ok = nearest(m, &u);
+                    if (!ok) break;
+                    post[(size_t)b] = outer_phase(u);
+                    m = matrix(without_phase(u, post[(size_t)b]));
                 }
                 ok = rotation(m, &r[(size_t)b]);
             }
             if (ok && whole)  // the rotation with its cosine and sine; what is left of s is a phase
                 for (int64_t b = 0; b < members; ++b) {
                     Rotation& x = r[(size_t)b];
-                    const double h = std::hypot(1.0, x.t);
-                    const double c = (x.flip ? x.t : 1.0) / h, sn = (x.flip ? 1.0 : x.t) / h;
+                    const double h = std::hypot(1.0, x.t.v);
+                    const double c = (x.flip ? x.t.v : 1.0) / h, sn = (x.flip ? 1.0 : x.t.v) / h;
                     x.t = c;
                     x.sine = sn;
                     // the FP32 pair's length is not one to rounding, the same for every amplitude: a
                     // drift of the norm that the diagonal can take back
-                    x.s *= h / std::hypot((double)(float)c, (double)(float)sn);
-                    x.s_err = 0.0;
+                    x.s = x.s * Two(h / std::hypot((double)(float)c, (double)(float)sn));
                 }
             if (ok) {
                 if (open < 0 || ((in_round | touched | pend.dep) & bits)) {
@@ -408,23 +459,23 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
                     open = (int)out->items.size();
                     out->items.push_back(std::move(it));
                     pre = pend;
-                    std::fill(pend.v.begin(), pend.v.end(), cd(1.0));
+                    std::fill(pend.v.begin(), pend.v.end(), Cpx(1.0));
                     pend.dep = 0;
                     in_round = touched = 0;
-                    std::fill(gain.begin(), gain.end(), Factor());
+                    std::fill(gain.begin(), gain.end(), Cpx(1.0));
                     ++rounds;
                     cost += 1.0 + overhead;
                 }
                 LoweredItem& it = out->items[(size_t)open];
                 for (int64_t b = 0; b < members; ++b) {
                     const Rotation& x = r[(size_t)b];
-                    it.t[(size_t)(b * U + P)] = x.t;
+                    it.t[(size_t)(b * U + P)] = x.t.value();
                     it.second[(size_t)(b * U + P)] = whole ? x.sine : x.flip;
-                    gain[(size_t)b].times(x.s, x.s_err);
+                    gain[(size_t)b] = gain[(size_t)b].one() ? x.s : gain[(size_t)b] * x.s;
                     for (int e = 0; e < D; ++e)
                         if (e & bit(P)) {
-                            if (x.e != cd(1.0)) pre.v[(size_t)(b * D + e)] *= x.e;
-                            if (post[(size_t)b] != cd(1.0)) pend.v[(size_t)(b * D + e)] *= post[(size_t)b];
+                            if (!x.e.one()) pre.times(b, e, x.e);
+                            if (!post[(size_t)b].one()) pend.times(b, e, post[(size_t)b]);
                         }
                 }
                 if (!moved[(size_t)o]) pend.dep |= bits | kNoBit;
@@ -436,27 +487,27 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
         }
         if (t.tmpl == kT_DIAG || t.tmpl == kT_SCALE) {
             for (int64_t b = 0; b < members; ++b) {
-                const double* p = pool + 2 * (t.data + (t.stride ? b * t.stride : 0));
+                const double* p = pool.data + 2 * (t.data + (t.stride ? b * t.stride : 0));
                 for (int e = 0; e < D; ++e) {
                     int j = 0;
                     for (int i = 0; i < t.k; ++i) j = (j << 1) | ((e & bit(t.pos[i])) ? 1 : 0);
-                    pend.v[(size_t)(b * D + e)] *= cd(p[2 * j], p[2 * j + 1]);
+                    pend.times(b, e, Cpx(p[2 * j], p[2 * j + 1]));
                 }
             }
             pend.dep |= bits | kNoBit;  // (a factor depends on no position, and is still to be applied)
             continue;
         }
-        const int code = is_rename(t.tmpl) ? t.tmpl : rename_of(t, pool, members);
+        const int code = is_rename(t.tmpl) ? t.tmpl : rename_of(t, pool.data, members);
         if (code >= 0) {  // a rename, and its phases as a diagonal after it
             permute(code);
             if (pend.dep & bits) pend.dep |= bits;
             if (code != t.tmpl) {
                 for (int64_t b = 0; b < members; ++b) {
-                    const double* p = pool + 2 * (t.data + (t.stride ? b * t.stride : 0));
+                    const double* p = pool.data + 2 * (t.data + (t.stride ? b * t.stride : 0));
                     for (int e = 0; e < D; ++e) {
                         int j = 0;
                         for (int i = 0; i < t.k; ++i) j = (j << 1) | ((e & bit(t.pos[i])) ? 1 : 0);
-                        pend.v[(size_t)(b * D + e)] *= cd(p[2 * j], p[2 * j + 1]);
+                        pend.times(b, e, Cpx(p[2 * j], p[2 * j + 1]));
                     }
                 }
                 pend.dep |= bits;

@@ -13,9 +13,17 @@ namespace lsg {
 
 // Move the outer factor of every one-bit operator of a planned complex program through the renames
 // and diagonals that let it pass, into the next one-bit operator on the same register bit. The
-// operators then read their matrices from entries appended to `pool` (complex entries as pairs).
-// Returns which operators (indexed like plan.ops) had their outer factor taken.
-std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<double>& pool);
+// operators then read their matrices from entries appended to `pool` (complex entries as pairs), what
+// the entries' rounding left over to `low`. Returns which operators (indexed like plan.ops) had their
+// outer factor taken.
+std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<double>& pool, std::vector<double>& low);
+
+// A program's data: `own` doubles of the caller's, then what move_outer_factors appended, with its `low`.
+struct Pool {
+    const double* data;
+    const double* low;
+    int64_t own;
+};
 
 // A lowered block: items in order, each a round (kT_ROUND: mask, diagonal, rotations) or an operator
 // kept as it is (kKeepOp: index into plan.ops, its register-block code).
@@ -38,6 +46,6 @@ struct LoweredBlock {
 // Lower a block whose operators have their positions and codes (whole: rotations as (cosine, sine)). False when it holds no rotation, or
 // would hold more operators than before.
 bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, const std::vector<char>& moved,
-                 int64_t batch, const double* pool, double overhead, bool whole, LoweredBlock* out);
+                 int64_t batch, const Pool& pool, double overhead, bool whole, LoweredBlock* out);
 
 }  // namespace lsg
