@@ -18,9 +18,12 @@
 // qubit, on the host. A brickwork layer then costs one diagonal per block, and no diagonal
 // is left over behind it.
 //
-// Everything here is decided per member from that member's own data, or from the operators'
-// structure alone, so a member of a batch gets the arithmetic it would get by itself: a diagonal
-// that some members do not need multiplies them by exact ones.
+// A member of a batch gets the arithmetic it would get by itself: what is decided from values is decided
+// per member from its own (a diagonal that some members do not need multiplies them by exact ones),
+// all else from the operators' structure. Two decisions are taken for all members: an operator that
+// is not unitary for one of them stays dense for all, and a permutation is a rename where it is the
+// same one for all. The gates of circuits are unitary, and their permutations shared; beside a member
+// of a caller's own list that is otherwise, a member differs by rounding from what it would be alone.
 #include <algorithm>
 #include <cmath>
 
@@ -33,10 +36,12 @@ namespace {
 
 using cd = std::complex<double>;
 
-// How far an operator may be from a rotation between phases, relative to its largest entry: gate
-// matrices (and products of a few) are unitary to a few units in the last place. Anything less
-// unitary stays dense.
-constexpr double kUnitary = 2e-15;
+// How far an operator may be from a rotation between phases, relative to its largest entry. Gate
+// matrices are unitary to a few units in the last place, products of n of them to some sqrt(n) times
+// 1e-16: this holds for any run of gates on a qubit, so that whether an operator is lowered depends
+// on what it is and not on a member's rounding (2e-15 left a tenth of the products of 50 gates dense,
+// for every member of the batch). Anything less unitary stays dense.
+constexpr double kUnitary = 1e-13;
 // A phase this close to one is the rounding of one (gate matrices are products of a few rounded
 // factors): taken as one, so the diagonal that would hold it is left out.
 constexpr double kResidue = 1e-15;
