@@ -229,8 +229,9 @@ int lsg_outcome_probabilities(lsg_state s, int dm_qubits, const int32_t* measure
                               const int32_t* pair_pos, const double* pair_p01, const double* pair_p10, double threshold,
                               double* out);
 /* <P> for Pauli terms given by x/z masks (Y sets both; qubit q = bit q), for every member.
- * out[t * batch + b]. Statevector: sum_b conj(psi[b^x]) c(b) psi[b]; density register:
- * sum_s c(s) rho[s][s^x]. Replaces the per-term loops of expectation
+ * out[t * batch + b]. Statevector: sum_b conj(psi[b^x]) c(b) psi[b], in complex64 over the member's
+ * sum_b |psi[b]|^2 where that is within 1e-5 of one (the drift of FP32 rounding; other norms are taken
+ * as meant); density register: sum_s c(s) rho[s][s^x]. Replaces the per-term loops of expectation
  * (src/lucivant_sim/simulator.py:505-527). */
 int lsg_expect_pauli(lsg_state s, int dm_qubits, const uint64_t* xmask, const uint64_t* zmask,
                      int32_t nterms, double* out);

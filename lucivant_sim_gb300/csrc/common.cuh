@@ -84,7 +84,6 @@ struct lsg_state_s {
     lsg::Scratch program;  // uploaded pass programs
     lsg::Scratch scratch;  // reduction partials, CDFs, sampling buffers
     lsg::Scratch scratch2;
-    bool unit_norm = false;  // a basis state and unitary operators since (complex registers)
     uint64_t uid = 0;  // distinct for every register made in this process (graphs are bound to one)
     size_t elem_bytes() const { return lsg_elem_bytes(precision); }
     bool real() const { return lsg_precision_real(precision); }

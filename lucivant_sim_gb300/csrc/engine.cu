@@ -591,7 +591,6 @@ struct lsg_program_s {
     // the pool section (caller's pool, then relocated and fused data) in the register precision:
     // kept by host-only builds, whose data a program of the same structure takes over
     std::vector<unsigned char> pool_bytes;
-    bool unitary = false;  // every operator keeps the norm of a statevector
     lsg::PlanChoice choice;  // the plan choices it was made with
     // the operator table and the plan before lowering: a template's new data is lowered onto this
     // plan without planning again (lsg_program_set_data)
@@ -915,34 +914,6 @@ static void host_block_op(std::complex<double>* v, int U, const TileOp& t, const
     }
 }
 
-// Whether every operator is unitary to 1e-12 (for every member).
-static bool ops_unitary(const lsg_op* ops, int32_t nops, const double* pool, int64_t batch) {
-    for (int32_t i = 0; i < nops; ++i) {
-        const lsg_op& op = ops[i];
-        if (op.kind == LSG_OP_DEPOL) return false;
-        const int d = 1 << op.nbits;
-        for (int64_t b = 0; b < (op.batch_stride ? batch : 1); ++b) {
-            const double* m = pool + 2 * (op.data + b * op.batch_stride);
-            if (op.kind != LSG_OP_MATRIX) {  // phases (a permutation's first entries)
-                for (int r = 0; r < (op.kind == LSG_OP_SCALE ? 1 : d); ++r)
-                    if (!(std::abs(m[2 * r] * m[2 * r] + m[2 * r + 1] * m[2 * r + 1] - 1.0) <= 1e-12)) return false;
-                continue;
-            }
-            for (int x = 0; x < d; ++x)
-                for (int y = x; y < d; ++y) {  // columns x and y
-                    double re = 0.0, im = 0.0;
-                    for (int r = 0; r < d; ++r) {
-                        const double *p = m + 2 * (r * d + x), *q = m + 2 * (r * d + y);
-                        re += p[0] * q[0] + p[1] * q[1];
-                        im += p[0] * q[1] - p[1] * q[0];
-                    }
-                    if (!(std::abs(re - (x == y)) <= 1e-12) || !(std::abs(im) <= 1e-12)) return false;
-                }
-        }
-    }
-    return true;
-}
-
 // Whether a pass moves swizzled tiles: its copies fit the tensor maps and all its blocks are register blocks.
 static bool pass_fits_swizzle(const PassDesc& pd, const Plan& plan, size_t eb, int nbits, int64_t batch) {
     bool fits = pass_swizzle_fits(pd, eb, ((int64_t)eb << nbits) * batch) && (eb << pd.K) <= 65536;
@@ -960,7 +931,6 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     p->precision = precision;
     p->batch = batch;
     p->choice = t_choice;
-    p->unitary = precision == LSG_C64 && !pred && !draw && !count && ops_unitary(ops, nops, pool, batch);
     p->dev.stream = stream;
     p->K = tile_bits_for(nbits, precision);
     // Complex128 trajectory segments on half tiles while every half has an SM to itself: the passes
@@ -1487,7 +1457,6 @@ static int program_launch(lsg_program_s* p, lsg_state_s* s, cudaEvent_t* marks, 
         return fail(LSG_E_STATE, "the program was built for a register of %d bits, precision %d, batch %lld",
                     p->nbits, p->precision, (long long)p->batch);
     if (p->plan.passes.empty()) return LSG_OK;
-    s->unit_norm = s->unit_norm && p->unitary;
     switch (s->precision) {
         case LSG_C128: return launch_passes<Cx<double>>(p, s, marks, ctx, from_basis);
         case LSG_C64: return launch_passes<Cx<float>>(p, s, marks, ctx, from_basis);
@@ -1732,7 +1701,6 @@ int set_basis_async(lsg_state_s* s, int64_t index) {
     const int64_t limit = s->real() ? (1ll << (s->nbits / 2)) : s->elems;  // real: |index><index| of nbits/2 qubits
     if (index < 0 || index >= limit) return fail(LSG_E_ARG, "basis index %lld out of range", (long long)index);
     LSG_CUDA(cudaMemsetAsync(s->data, 0, s->member_bytes() * (size_t)s->batch, s->stream));
-    s->unit_norm = !s->real();
     const int n = s->nbits / 2;
     if (s->precision == LSG_C128)
         k_basis_one<double><<<grid_for(s->batch), 256, 0, s->stream>>>((Cx<double>*)s->data, s->elems, s->batch, index);
@@ -1845,7 +1813,6 @@ int lsg_state_upload(lsg_state s, const double* host, int64_t nbytes) {
     const int64_t n = s->elems * s->batch;
     const int64_t want = n * (s->real() ? 8 : 16);  // float64 per element for real registers
     if (nbytes != want) return fail(LSG_E_ARG, "upload expects %lld bytes, got %lld", (long long)want, (long long)nbytes);
-    s->unit_norm = false;
     if (s->precision == LSG_C128 || s->precision == LSG_R64) {
         LSG_CUDA(cudaMemcpyAsync(s->data, host, (size_t)nbytes, cudaMemcpyHostToDevice, s->stream));
     } else {
@@ -1928,7 +1895,6 @@ int lsg_state_to_complex(lsg_state src, int64_t member, lsg_state dst) {
     if (src->nbits != dst->nbits) return fail(LSG_E_ARG, "lsg_state_to_complex: registers of different sizes");
     if (member < 0 || member >= src->batch) return fail(LSG_E_ARG, "member %lld out of range", (long long)member);
     LSG_CUDA(cudaStreamSynchronize(src->stream));  // dst's stream reads what src's stream wrote
-    dst->unit_norm = false;
     const int64_t n = src->elems;
     const unsigned g = grid_for(n);
     if (src->precision == LSG_RD && dst->precision == LSG_C128)
@@ -2071,7 +2037,6 @@ int lsg_programs_run_ragged(int32_t count, const lsg_program* programs, const ls
             continue;
         }
         if (p->plan.passes.empty()) continue;
-        s->unit_norm = s->unit_norm && p->unitary;
         ragged.emplace_back(p, s);
         if (s->stream != st) {  // the ragged launches go after this register's basis state
             cudaEvent_t e;
@@ -2146,7 +2111,6 @@ int lsg_program_set_data(lsg_program p, lsg_state s, const lsg_op* ops, int32_t 
         program_destroy(q);
         return program_remake(p, ops, nops, pool, pool_entries);
     }
-    p->unitary = q->unitary;
     // after the register's earlier work (a run may still read the old data); pageable source:
     // staged before the call returns
     const cudaError_t e = cudaMemcpyAsync(static_cast<unsigned char*>(p->dev.ptr) + p->head_aligned, q->pool_bytes.data(),
@@ -2185,7 +2149,6 @@ int lsg_program_graph_run(lsg_program p, lsg_state s, int64_t index) {
         return LSG_OK;  // this call's run was the plain one before the capture
     }
     LSG_CHECK(basis_passes_for(p, s, index));  // another index may have run in between
-    s->unit_norm = !s->real() && p->unitary;
     LSG_CUDA(cudaGraphLaunch(p->graph, s->stream));
     return LSG_OK;
 }

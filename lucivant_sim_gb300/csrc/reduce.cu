@@ -262,6 +262,13 @@ struct PauliTerm {
 // Density matrices (dm_n > 0): the summands are the diagonal-block entries rho[i, i ^ x], in FP64.
 // The masks come with the launch when they are few (no copy to wait for), else from xm and zm.
 constexpr int kTermsWithLaunch = 64;
+
+// FP32 rounding lets the norm of a complex64 statevector drift (1e-6 in the square over 40 layers of 26
+// qubits), and that is most of the error of its expectations. So the sums of a member whose squared norm
+// is one to within kUnitNorm are divided by it, whatever made the state: 1.1e-6 -> 2.6e-7 (26 qubits,
+// 40 layers). Other norms are the caller's, their sums stay as they are.
+constexpr double kUnitNorm = 1e-5;
+__host__ __device__ inline bool unit_norm(double square) { return fabs(square - 1.0) <= kUnitNorm; }
 struct TermMasks {
     uint64_t x[kTermsWithLaunch], z[kTermsWithLaunch];
 };
@@ -652,6 +659,24 @@ int lsg_outcome_probabilities(lsg_state s, int dm_qubits, const int32_t* measure
     return LSG_OK;
 }
 
+namespace {
+
+// Statevector members go through in groups small enough to stay in L2 while every term reads them (one
+// group per launch); density-matrix diagonals are small and go all at once.
+int64_t expect_chunk(int64_t elems, int precision, int dm_qubits) {
+    const int64_t member_bytes = elems * (precision == LSG_C128 ? 16 : 8);
+    return dm_qubits ? kMaxGridY : std::min<int64_t>(kMaxGridY, std::max<int64_t>(1, kExpectL2Bytes / member_bytes));
+}
+
+// Blocks per term and member, for `rows` of them in a launch: eight indices per thread, within a launch of
+// some 64k blocks.
+int64_t expect_grid(int64_t count, int64_t rows) {
+    return std::max<int64_t>(
+        1, std::min<int64_t>({(count + 8 * kThreads - 1) / (8 * kThreads), 152 * 8, std::max<int64_t>(1, 65536 / rows)}));
+}
+
+}  // namespace
+
 int lsg_expect_pauli(lsg_state s, int dm_qubits, const uint64_t* xmask, const uint64_t* zmask, int32_t nterms,
                      double* out) {
     clear_error();
@@ -691,15 +716,9 @@ int lsg_expect_pauli(lsg_state s, int dm_qubits, const uint64_t* xmask, const ui
         return LSG_OK;
     }
     const int64_t count = dm_qubits ? (1ll << dm_qubits) : s->elems;
-    // Statevector members go through in groups small enough to stay in L2 while every term reads
-    // them (one group per launch); density-matrix diagonals are small and go all at once.
-    const int64_t member_bytes = s->elems * (s->precision == LSG_C128 ? 16 : 8);
-    const int64_t chunk = dm_qubits ? kMaxGridY
-                                    : std::min<int64_t>(kMaxGridY, std::max<int64_t>(1, kExpectL2Bytes / member_bytes));
-    // A complex64 statevector made by unitary operators alone has norm one; FP32 rounding lets it drift
-    // (1e-6 over 40 layers), most of the error of an expectation. Its own norm, one more term, is
-    // divided out.
-    const bool normalise = !dm_qubits && s->precision == LSG_C64 && s->unit_norm;
+    const int64_t chunk = expect_chunk(s->elems, s->precision, dm_qubits);
+    // a complex64 statevector's squared norm is one more term (kUnitNorm)
+    const bool normalise = !dm_qubits && s->precision == LSG_C64;
     const int terms = nterms + (normalise ? 1 : 0);
     TermMasks few{};
     std::vector<uint64_t> many;
@@ -718,10 +737,7 @@ int lsg_expect_pauli(lsg_state s, int dm_qubits, const uint64_t* xmask, const ui
         off += (bytes + 255) & ~size_t(255);
         return at;
     };
-    // blocks per term and member: eight indices per thread, within a launch of some 64k blocks
-    const int64_t at_once = (int64_t)terms * std::min(chunk, s->batch);
-    const unsigned grid = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>({(count + 8 * kThreads - 1) / (8 * kThreads), 152 * 8, std::max<int64_t>(1, 65536 / at_once)}));
+    const unsigned grid = (unsigned)expect_grid(count, (int64_t)terms * std::min(chunk, s->batch));
     const int64_t rows = (int64_t)terms * s->batch;
     const size_t o_m = take(many.size() * 8), o_part = take((size_t)rows * grid * 8), o_out = take((size_t)rows * 8);
     LSG_CHECK(ensure(s->scratch, off));
@@ -749,8 +765,8 @@ int lsg_expect_pauli(lsg_state s, int dm_qubits, const uint64_t* xmask, const ui
     LSG_CUDA(cudaMemcpyAsync(tmp.data(), base + (grid > 1 ? o_out : o_part), tmp.size() * 8, cudaMemcpyDeviceToHost, s->stream));
     LSG_CUDA(cudaStreamSynchronize(s->stream));
     for (int64_t b = 0; b < s->batch; ++b) {
-        const double norm = normalise ? tmp[b * terms + nterms] : 1.0;
-        for (int t = 0; t < nterms; ++t) out[(int64_t)t * s->batch + b] = norm > 0.0 ? tmp[b * terms + t] / norm : tmp[b * terms + t];
+        const double norm = normalise && unit_norm(tmp[b * terms + nterms]) ? tmp[b * terms + nterms] : 1.0;
+        for (int t = 0; t < nterms; ++t) out[(int64_t)t * s->batch + b] = tmp[b * terms + t] / norm;
     }
     return LSG_OK;
 }
@@ -781,7 +797,6 @@ int lsg_collapse(lsg_state s, int qubit, int outcome, double probability, int64_
     if (!s) return fail(LSG_E_ARG, "null register");
     if (qubit < 0 || qubit >= s->nbits || (outcome != 0 && outcome != 1)) return fail(LSG_E_ARG, "bad qubit or outcome");
     if (member < 0 || member >= s->batch) return fail(LSG_E_ARG, "member out of range");
-    s->unit_norm = false;
     const double div = probability > 0 ? sqrt(probability) : 1.0;
     const int do_scale = probability > 0 ? 1 : 0;
     if (s->precision == LSG_C128)
@@ -849,6 +864,18 @@ __global__ void k_sum_rows_to_terms(const double* __restrict__ partials, int64_t
     }
 }
 
+// out[t * batch + b] over member b's squared norm (the sum of its `ncols` partials) where unit_norm.
+__global__ void k_divide_by_norm(const double* __restrict__ partials, int64_t ncols, int nterms, int64_t batch,
+                                 double* __restrict__ out) {
+    for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
+        double acc = 0.0;
+        for (int64_t c = threadIdx.x; c < ncols; c += blockDim.x) acc += partials[b * ncols + c];
+        const double norm = block_sum(acc);
+        if (unit_norm(norm))
+            for (int t = threadIdx.x; t < nterms; t += blockDim.x) out[t * batch + b] /= norm;
+    }
+}
+
 }  // namespace lsg
 
 extern "C" int lsg_expect_pauli_noalloc(const void* amplitudes, int precision, int nbits, int64_t batch, int dm_qubits,
@@ -878,8 +905,11 @@ extern "C" int lsg_expect_pauli_noalloc(const void* amplitudes, int precision, i
                     "(at most %zu partial sums)", nterms, (long long)batch, kNoAllocScratchBytes, room / 8);
     const int64_t count = dm_qubits ? (1ll << dm_qubits) : (1ll << nbits);
     const int64_t fit = (int64_t)(room / 8 / (size_t)rows);
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>({(int64_t)reduce_grid(count), fit,
-                                                                             std::max<int64_t>(1, 4096 / batch)}));
+    // the blocks lsg_expect_pauli takes (its order of the sums), as far as their partial sums fit
+    const int64_t chunk = expect_chunk(1ll << nbits, precision, dm_qubits);
+    const bool normalise = !dm_qubits && precision == LSG_C64;
+    const unsigned grid =
+        (unsigned)std::max<int64_t>(1, std::min(fit, expect_grid(count, (nterms + normalise) * std::min(chunk, batch))));
     // both buffers must be device memory of the current device: the scratch array used below is
     // the current device's, and the kernels read and write the buffers from that device
     int dev = 0;
@@ -915,6 +945,12 @@ extern "C" int lsg_expect_pauli_noalloc(const void* amplitudes, int precision, i
                                                 dx, dz, nterms, part);
     k_sum_rows_to_terms<<<(unsigned)std::min<int64_t>(rows, 152 * 16), kThreads, 0, st>>>(part, grid, nterms, batch,
                                                                                         out_device);
+    if (normalise) {  // the norms, in the place of the terms' partial sums
+        k_expect<float><<<dim3(grid, (unsigned)batch), kThreads, 0, st>>>(static_cast<const Cx<float>*>(amplitudes), elems, 0,
+                                                                         TermMasks{}, nullptr, nullptr, 1, part);
+        k_divide_by_norm<<<(unsigned)std::min<int64_t>(batch, 152 * 16), kThreads, 0, st>>>(part, grid, nterms, batch,
+                                                                                          out_device);
+    }
     LSG_CUDA(cudaGetLastError());
     // the masks are copied from the caller's host memory: wait, so the caller may reuse it
     LSG_CUDA(cudaStreamSynchronize(st));

@@ -758,7 +758,6 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
     const int64_t B = s->batch;
     const int64_t elems = s->elems;
     cudaStream_t st = s->stream;
-    s->unit_norm = false;
     Cx<R>* state = (Cx<R>*)s->data;
     TrajCtx ctx;
     ctx.u = u;
