@@ -141,13 +141,18 @@ int lsg_program_run_from_basis(lsg_program p, lsg_state s, int64_t index, float*
 int lsg_programs_run_ragged(int32_t count, const lsg_program* programs, const lsg_state* states, const int64_t* index,
                             float* step_ms);
 /* Circuit templates. lsg_program_set_data gives program p the operator data of `ops`/`pool` — the
- * same circuit template with other parameters — without planning or allocating again: the
- * operators must plan exactly as p's did (same passes, blocks, operator codes and data layout;
- * otherwise LSG_E_STATE and p is unchanged). The copy is ordered on register s's stream, after
- * its earlier work. lsg_program_graph_run is lsg_program_run_from_basis(p, s, index, NULL) as
+ * same circuit template with other parameters — without planning again: the operators must plan
+ * exactly as p's did (same passes, blocks, operator codes and data layout; otherwise LSG_E_STATE
+ * and p is unchanged). The copy is ordered on register s's stream, after its earlier work, and
+ * allocates nothing. One case does more: values that need an operation which no earlier set of p's
+ * needed (p made from angles that are exactly zero has no diagonals, the next set has). p then takes
+ * the larger form once and keeps it: device memory for it is allocated and the old one released,
+ * which waits for the device, specialized passes are compiled for it, and the graph below is
+ * captured again. Not while a stream is captured. Create p from values of the general kind to
+ * have its final form at once. lsg_program_graph_run is lsg_program_run_from_basis(p, s, index, NULL) as
  * one CUDA graph launch: the first call for a (register, index) pair runs the program and
  * captures basis state + passes into a graph that later calls replay; data set since stays in
- * effect (the graph reads p's device data). Neither waits. No counterpart in the reference, which
+ * effect (the graph reads p's device data). Otherwise neither waits. No counterpart in the reference, which
  * parses a template again for every set of `input` parameters (qasm.py:842-870) and evolves each
  * circuit from scratch (simulator.py:229-251). */
 int lsg_program_set_data(lsg_program p, lsg_state s, const lsg_op* ops, int32_t nops, const double* pool,

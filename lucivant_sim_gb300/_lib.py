@@ -493,7 +493,8 @@ class Program:
 
     def set_data(self, reg: Register, ops: OpList) -> None:
         """Take the operator data of ``ops`` (the same template with other parameters) without
-        planning or allocating again. :class:`EngineError` when ``ops`` plan differently (another
+        planning again. Allocates only where values need an operation that no earlier set did (general
+        angles after ones that were exactly zero): the program keeps the larger form. :class:`EngineError` when ``ops`` plan differently (another
         structure). Ordered after ``reg``'s earlier work."""
         table, pool = ops.packed()
         check(self.lib.lsg_program_set_data(self.handle, reg.handle, table.ctypes.data, len(table),

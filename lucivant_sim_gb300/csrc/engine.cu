@@ -588,9 +588,10 @@ struct lsg_program_s {
     std::vector<lsg::PassDesc> basis_passes;
     int64_t basis_index = -1;
     size_t basis_off = 0;
-    // the pool section (caller's pool, then relocated and fused data) in the register precision:
-    // kept by host-only builds, whose data a program of the same structure takes over
-    std::vector<unsigned char> pool_bytes;
+    // the device memory's content (the pool, in the register precision, from head_aligned on): kept by
+    // host-only builds, which a program of the same structure takes over
+    std::vector<unsigned char> content;
+    std::vector<lsg::Choices> form;  // what its values have decided: per block, and of the moves between them
     lsg::PlanChoice choice;  // the plan choices it was made with
     // the operator table and the plan before lowering: a template's new data is lowered onto this
     // plan without planning again (lsg_program_set_data)
@@ -921,11 +922,23 @@ static bool pass_fits_swizzle(const PassDesc& pd, const Plan& plan, size_t eb, i
     return fits;
 }
 
+// Copy a program's content to device memory of its own.
+static int program_upload(lsg_program_s* p, const std::vector<unsigned char>& content, cudaStream_t stream) {
+    LSG_CHECK(ensure(p->dev, content.size()));
+    // the host's copy may be released on return: the transfer must have consumed it
+    cudaError_t e = stream ? cudaMemcpyAsync(p->dev.ptr, content.data(), content.size(), cudaMemcpyHostToDevice, stream)
+                           : cudaMemcpy(p->dev.ptr, content.data(), content.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && stream) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return fail(LSG_E_CUDA, "uploading the program failed: %s", cudaGetErrorString(e));
+    return LSG_OK;
+}
+
 // Plan and lower `ops`; with `upload`, copy the program to the device (otherwise only the host
-// plan is made: no device call).
+// plan is made: no device call). `form`: the choices to take at least.
 static int program_build(int nbits, int precision, int64_t batch, const lsg_op* ops, int32_t nops, const double* pool,
                          int64_t pool_entries, const int* pred, const int* draw, const int* count, lsg_program_s** out,
-                         cudaStream_t stream, bool upload, const Plan* preplanned = nullptr) {
+                         cudaStream_t stream, bool upload, const Plan* preplanned = nullptr,
+                         const std::vector<Choices>* form = nullptr) {
     auto* p = new lsg_program_s();
     p->nbits = nbits;
     p->precision = precision;
@@ -962,6 +975,9 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
         delete p;
         return LSG_E_ARG;
     }
+    if (form) p->form = *form;
+    p->form.resize(p->plan.blocks.size() + 1);
+    for (Choices& c : p->form) c.at = 0;
     for (PassDesc& pd : p->plan.passes) {  // a predicate shared by the whole pass
         pd.slot = pd.nops ? p->plan.ops[pd.first_op].pred : 0;
         for (int o = pd.first_op; o < pd.first_op + pd.nops; ++o)
@@ -1028,7 +1044,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     const bool transfer = precision == LSG_R64 && !pred && !draw && !count && !(fuse_env && fuse_env[0] == '0');
     if (transfer && nops > 0) {
         grown.assign(pool, pool + 2 * pool_entries);
-        move_outer_rotations(p->plan, batch, grown);
+        move_outer_rotations(p->plan, batch, grown, p->form.back());
         pool = grown.data();
         pool_entries = (int64_t)grown.size() / 2;
     }
@@ -1059,7 +1075,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 pure = pure && held(p->plan.ops[o].tmpl);
             LoweredBlock& low = lowered[i];
             if (pure) continue;
-            lower_block(p->plan, pd, blk, moved, batch, Pool{pool, grown_low.data(), own}, round_cost, true, &low);
+            lower_block(p->plan, pd, blk, moved, batch, Pool{pool, grown_low.data(), own}, round_cost, true, p->form[pd.first_block + i], &low);
             whole_pass = low.members == 1 && !low.items.empty() && (int)low.items.size() <= blk.nops;
             for (const LoweredItem& it : low.items) whole_pass = whole_pass && (it.code != kKeepOp || held(it.tmpl));
         }
@@ -1080,7 +1096,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
                 if (dense) cost = std::min(cost, 1.1 * ((double)(1 << blk.u) + overhead + (double)(1 << blk.u) / 16.0));
                 LoweredBlock low;
                 if (ready) low = std::move(lowered[bi - pd.first_block]);
-                if (ready || (lower_block(p->plan, pd, blk, moved, batch, Pool{pool, grown_low.data(), own}, overhead, precision == LSG_C64, &low) &&
+                if (ready || (lower_block(p->plan, pd, blk, moved, batch, Pool{pool, grown_low.data(), own}, overhead, precision == LSG_C64, p->form[bi], &low) &&
                               low.cost < cost)) {
                     const int D = 1 << blk.u;
                     std::vector<TileOp> made;
@@ -1128,7 +1144,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
             }
             std::vector<TransferItem> shears;
             int64_t shear_members = 1;
-            if (transfer && lower_transfer_block(p->plan, pd, blk, batch, pool, &shears, &shear_members)) {
+            if (transfer && lower_transfer_block(p->plan, pd, blk, batch, pool, p->form[bi], &shears, &shear_members)) {
                 std::vector<TileOp> made;
                 for (const TransferItem& it : shears) {
                     if (it.op >= 0) {
@@ -1352,18 +1368,11 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     put(pool, base_entries, dst);
     put(ext.data(), (int64_t)ext.size() / 2, dst + (size_t)base_entries * elt);
     if (!upload) {
-        p->pool_bytes.assign(dst, dst + (size_t)pool_entries * elt);
+        p->content = std::move(blob);
         *out = p;
         return LSG_OK;
     }
-    int rc = ensure(p->dev, total);
-    if (rc == LSG_OK) {
-        // the host blob is released on return: the copy must have consumed it
-        cudaError_t e = stream ? cudaMemcpyAsync(p->dev.ptr, blob.data(), total, cudaMemcpyHostToDevice, stream)
-                               : cudaMemcpy(p->dev.ptr, blob.data(), total, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && stream) e = cudaStreamSynchronize(stream);
-        if (e != cudaSuccess) rc = fail(LSG_E_CUDA, "uploading the program failed: %s", cudaGetErrorString(e));
-    }
+    const int rc = program_upload(p, blob, stream);
     if (rc != LSG_OK) {
         release(p->dev);
         delete p;
@@ -1426,29 +1435,25 @@ void program_destroy(lsg_program_s* p) {
     delete p;
 }
 
-// Put a program made anew from `ops` (its plan choices, its kind of passes) in the place of `p`'s
-// content. The old device memory is released with cudaFree, which waits for runs that still read
-// it; the graph is captured again by the next graph run.
-static int program_remake(lsg_program_s* p, const lsg_op* ops, int32_t nops, const double* pool, int64_t pool_entries) {
-    lsg_program_s* q = nullptr;
-    const PlanChoice keep = t_choice;
-    t_choice = p->choice;
-    const Plan raw = p->raw_plan;
-    int rc = program_build(p->nbits, p->precision, p->batch, ops, nops, pool, pool_entries, nullptr, nullptr, nullptr,
-                           &q, nullptr, true, &raw);
-    if (rc == LSG_OK && p->jit) {
+// Put q, a host-only build of the same operators that needs a larger form, in the place of p's content. p's
+// old memory is released with cudaFree, which waits for runs that still read it; the graph is captured
+// again by the next graph run, specialized passes are compiled for the form (or found compiled).
+static int program_adopt(lsg_program_s* p, lsg_program_s* q, cudaStream_t stream) {
+    LSG_CHECK(program_upload(q, q->content, stream));
+    q->content.clear();
+    q->content.shrink_to_fit();
+    if (p->jit) {
         const size_t eb = lsg_elem_bytes(p->precision);
+        const PlanChoice keep = t_choice;
+        t_choice = p->choice;
         q->jit = jit_build(q->plan, p->precision, jit_ctas(p->precision),
                            jit_swizzle_fits(q->plan, eb, ((int64_t)eb << p->nbits) * p->batch), jit_packed(p->precision));
+        t_choice = keep;
     }
-    t_choice = keep;
-    LSG_CHECK(rc);
+    q->src_ops = p->src_ops;
+    q->raw_plan = p->raw_plan;
     std::swap(*p, *q);
     std::swap(p->events, q->events);
-    if (p->graph) cudaGraphExecDestroy(p->graph);
-    p->graph = nullptr;
-    p->graph_uid = 0;
-    program_destroy(q);
     return LSG_OK;
 }
 
@@ -2091,7 +2096,7 @@ int lsg_program_set_data(lsg_program p, lsg_state s, const lsg_op* ops, int32_t 
     const PlanChoice keep = t_choice;  // the plan choices the program was made with
     t_choice = p->choice;
     const int rc = program_build(p->nbits, p->precision, p->batch, ops, nops, pool, pool_entries, nullptr, nullptr,
-                                 nullptr, &q, nullptr, false, &p->raw_plan);
+                                 nullptr, &q, nullptr, false, &p->raw_plan, &p->form);
     t_choice = keep;
     LSG_CHECK(rc);
     auto same_bytes = [](const auto& a, const auto& b) {
@@ -2105,16 +2110,17 @@ int lsg_program_set_data(lsg_program p, lsg_state s, const lsg_op* ops, int32_t 
         return fail(LSG_E_STATE, "lsg_program_set_data: the operators plan differently from the program's (another "
                                  "structure): build a new program");
     }
-    if (!same_plan(q->plan, p->plan) || p->head_aligned + q->pool_bytes.size() > p->dev.bytes) {
-        // the same operators, but their values lower to other blocks (a rotation whose phase is
-        // exactly one needs no diagonal): the program is made again with the new values
-        program_destroy(q);
-        return program_remake(p, ops, nops, pool, pool_entries);
+    if (!same_plan(q->plan, p->plan) || q->content.size() > p->dev.bytes) {
+        // the same operators, of values that need more than any before them did
+        const int rc = program_adopt(p, q, s->stream);
+        program_destroy(q);  // p's old content, when it was taken over
+        return rc;
     }
+    p->form = std::move(q->form);
     // after the register's earlier work (a run may still read the old data); pageable source:
     // staged before the call returns
-    const cudaError_t e = cudaMemcpyAsync(static_cast<unsigned char*>(p->dev.ptr) + p->head_aligned, q->pool_bytes.data(),
-                                          q->pool_bytes.size(), cudaMemcpyHostToDevice, s->stream);
+    const cudaError_t e = cudaMemcpyAsync(static_cast<unsigned char*>(p->dev.ptr) + p->head_aligned, q->content.data() + q->head_aligned,
+                                          q->content.size() - q->head_aligned, cudaMemcpyHostToDevice, s->stream);
     program_destroy(q);
     if (e != cudaSuccess) return fail(LSG_E_CUDA, "lsg_program_set_data: %s", cudaGetErrorString(e));
     return LSG_OK;

@@ -138,11 +138,16 @@ bool nearest(const Mat& m, Unitary* out) {
 
 Mat matrix(const Unitary& u) { return Mat{u.a, -(u.w * conj(u.c)), u.c, u.w * conj(u.a)}; }
 
-// The phase ph of u = diag(1, ph) * N with N's first column in a real, positive ratio.
+// The phase ph of u = diag(1, ph) * N with N's first column in a real ratio. Of its two signs the one that
+// leaves N's e (Rotation) the positive real part: a rotation's e is then one for either sign of its
+// cosine and sine, and whether it needs a diagonal does not depend on its angle.
 Cpx outer_phase(const Unitary& u) {
     if (zero(u.a) || zero(u.c)) return 1.0;
-    const Cpx ph = u.c * conj(u.a);
-    return settled(ph / root(norm(ph)));
+    Cpx ph = u.c * conj(u.a);
+    ph = ph / root(norm(ph));
+    const cd a = u.a.value(), c = u.c.value(), w = u.w.value(), p = ph.value();
+    const cd e = std::norm(c) > std::norm(a) ? w * p * std::conj(c * c) : w * std::conj(p * a * a);
+    return settled(e.real() < 0.0 ? -ph : ph);
 }
 Unitary without_phase(const Unitary& u, Cpx ph) {
     return ph.one() ? u : Unitary{u.a, u.c * conj(ph), u.w * conj(ph)};
@@ -339,7 +344,7 @@ std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<doub
 }
 
 bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, const std::vector<char>& moved,
-                 int64_t batch, const Pool& pool, double overhead, bool whole, LoweredBlock* out) {
+                 int64_t batch, const Pool& pool, double overhead, bool whole, Choices& form, LoweredBlock* out) {
     const int U = blk.u, D = 1 << U;
     const int first = pd.first_op + blk.first, last = first + blk.nops;
     int64_t members = 1;
@@ -378,7 +383,7 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
         }
         LoweredItem& it = out->items[(size_t)open];
         it.mask = (int)in_round;
-        if (!pre.one()) {
+        if (form.at_least(!pre.one())) {
             it.mask |= 16;
             it.diag = pre.rounded();
         }
@@ -528,11 +533,11 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
     flush_late();
     close(true);
     // A diagonal left over: by structure (whether the block is lowered is the same for every member's
-    // data), emitted when some member's is not one.
+    // data), emitted when some member's is not one (or has not been).
     const bool left = pend.dep != 0;
     const int items = (int)out->items.size() + left;
     out->cost = cost + (left ? 1.0 + overhead : 0.0);
-    if (!pend.one()) emit_diag(pend);
+    if (left && form.at_least(!pend.one())) emit_diag(pend);
     return rotations > 0 && items <= blk.nops;
 }
 

@@ -43,9 +43,9 @@ struct LoweredBlock {
     double cost = 0.0;    // complex multiply-adds per amplitude, `overhead` per operator included
 };
 
-// Lower a block whose operators have their positions and codes (whole: rotations as (cosine, sine)). False when it holds no rotation, or
-// would hold more operators than before.
+// Lower a block whose operators have their positions and codes (whole: rotations as (cosine, sine)). False
+// when it holds no rotation, or would hold more operators than before. `form`: its diagonals so far.
 bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, const std::vector<char>& moved,
-                 int64_t batch, const Pool& pool, double overhead, bool whole, LoweredBlock* out);
+                 int64_t batch, const Pool& pool, double overhead, bool whole, Choices& form, LoweredBlock* out);
 
 }  // namespace lsg

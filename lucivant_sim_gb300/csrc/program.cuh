@@ -85,6 +85,19 @@ static_assert(offsetof(BlockDesc, gb) % 16 == 0, "a block's address maps are rea
 #endif
 
 #ifndef __CUDACC_RTC__
+// What an operator list's values, beyond its structure, have decided about a program's form: bits per
+// choice, in the order they are met (a diagonal there, the parts of an operator). New values of the
+// same structure take at least these, as exact ones and zeros where they need less, so that a form
+// only grows.
+struct Choices {
+    std::vector<int> bits;
+    std::size_t at = 0;
+    int at_least(int need) {
+        if (at == bits.size()) bits.push_back(0);
+        return bits[at++] |= need;
+    }
+};
+
 struct Plan {
     std::vector<PassDesc> passes;
     std::vector<TileOp> ops;

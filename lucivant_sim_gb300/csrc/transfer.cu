@@ -253,7 +253,7 @@ int passes(const Composite& c, int64_t b, int U, int P0, int P1) {
 
 }  // namespace
 
-void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool) {
+void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, Choices& form) {
     struct Touch {
         int op, pass, block;
     };
@@ -338,18 +338,19 @@ void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool) 
                 mine.push_back(m);
                 next.push_back(x);
             }
-            if (!any) continue;
+            if (!form.at_least(any)) continue;
             auto put = [&](TileOp& op, const std::vector<Mat4>& ms) {
                 op.data = (int64_t)pool.size() / 2;
                 op.stride = members > 1 ? 16 : 0;
-                op.zmask = (1 << 12) - 1;
+                int entries = 0;
                 for (const Mat4& m : ms)
                     for (int e = 0; e < 16; ++e) {
                         const double y = m.a[e / 4][e % 4];
-                        if (e >= 4 && y != 0.0) op.zmask &= ~(1 << (e - 4));
+                        if (e >= 4 && y != 0.0) entries |= 1 << (e - 4);
                         pool.push_back(y);
                         pool.push_back(0.0);
                     }
+                op.zmask = ~form.at_least(entries) & ((1 << 12) - 1);
             };
             put(t, mine);
             put(n, next);
@@ -357,7 +358,7 @@ void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool) 
 }
 
 bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, int64_t batch, const double* pool,
-                          std::vector<TransferItem>* items, int64_t* members_out) {
+                          Choices& form, std::vector<TransferItem>* items, int64_t* members_out) {
     const int U = blk.u, D = 1 << U;
     const int first = pd.first_op + blk.first, last = first + blk.nops;
     int64_t members = 1;
@@ -435,6 +436,7 @@ bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc&
             it.v[it.v.size() - 21] = f.shift[2];
             for (int e = 0; e < D; ++e) scales[(size_t)(b * D + e)] *= f.scale[(e & B0 ? 2 : 0) + (e & B1 ? 1 : 0)];
         }
+        it.mask = form.at_least(it.mask);
         items->push_back(std::move(it));
         touched |= bits;
         if (left) dep |= bits;
