@@ -285,8 +285,11 @@ std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<doub
                     at[t.lb[i] < pd.L ? t.lb[i] : pd.hi[t.lb[i] - pd.L]].push_back(Touch{o, t.lb[i], !blk.generic});
             }
         }
+    std::vector<Mat> m, inner, outer;
+    std::vector<Mat> carry;  // what the operator before handed on: empty, one entry or one per member
+    bool phases = false;     // diag(1, phase)
     for (const std::vector<Touch>& seq : at) {
-        std::vector<Mat> carry;  // what the operator before handed on: empty, one entry or one per member
+        carry.clear();
         for (size_t i = 0; i < seq.size(); ++i) {
             TileOp& t = plan.ops[(size_t)seq[i].op];
             if (!seq[i].block || !is_dense1(t)) continue;
@@ -300,10 +303,15 @@ std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<doub
             }
             if (j >= seq.size()) through = 0;
             const int64_t members = std::max<int64_t>(t.stride ? batch : 1, (int64_t)carry.size());
-            std::vector<Mat> m((size_t)members), inner, outer;
+            m.resize((size_t)members);
+            inner.clear(), outer.clear();
             for (int64_t b = 0; b < members; ++b) {
                 m[(size_t)b] = matrix_of(t, Pool{pool.data(), low.data(), own}, b);
-                if (!carry.empty()) m[(size_t)b] = mul(m[(size_t)b], carry[carry.size() == 1 ? 0 : (size_t)b]);
+                if (carry.empty()) continue;
+                const Mat& c = carry[carry.size() == 1 ? 0 : (size_t)b];
+                Mat& x = m[(size_t)b];
+                if (!phases) x = mul(x, c);
+                else if (!c.d.one()) x.b = x.b * c.d, x.d = x.d * c.d;
             }
             for (int64_t b = 0; b < members && through; ++b) {
                 Unitary u;
@@ -322,6 +330,7 @@ std::vector<char> move_outer_factors(Plan& plan, int64_t batch, std::vector<doub
                 inner.push_back(matrix(u));
                 outer.push_back(p);
             }
+            phases = through & 1;
             const bool carried = !carry.empty();
             carry.clear();
             if (through) {
@@ -359,6 +368,8 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
     unsigned in_round = 0, touched = 0;
     Diagonal pre(members, D);   // the open round's diagonal
     std::vector<Cpx> gain((size_t)members, Cpx(1.0));  // the open round's factors taken out
+    std::vector<Rotation> r;
+    std::vector<Cpx> post;
     int rounds = 0, rotations = 0;
     double cost = 0.0;
 
@@ -434,8 +445,8 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
         }
         if (is_dense1(t)) {
             const int P = t.pos[0];
-            std::vector<Rotation> r((size_t)members);
-            std::vector<Cpx> post((size_t)members, Cpx(1.0));
+            r.assign((size_t)members, Rotation());
+            post.assign((size_t)members, Cpx(1.0));
             bool ok = true;
             for (int64_t b = 0; b < members && ok; ++b) {
                 Mat m = matrix_of(t, pool, b);
