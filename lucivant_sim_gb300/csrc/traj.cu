@@ -215,12 +215,16 @@ __global__ void k_t_collapse(Cx<R>* __restrict__ state, int64_t elems, int q, co
     const double p = out >= 0 ? prob[b] : 1.0;
     const double div = p > 0 ? sqrt(p) : 1.0;
     const bool scale = out >= 0 && p > 0;
-    // complex128 divides by the FP64 norm exactly as Orrery does; complex64 multiplies by its
+    // complex128 amplitudes are the quotients by the FP64 norm, as Orrery's; complex64 multiplies by its
     // FP64 reciprocal rounded once (an FP64 division per element would bind the pass to FP64)
     const R inv = (R)(1.0 / div);
-    // (the quotient from the reciprocal and one correction by its exact remainder, Markstein 1990:
-    // three FP64 operations where the division's own sequence bound the pass)
+    // The quotient from the rounded reciprocal and one correction by its exact remainder (Markstein 1990):
+    // three FP64 operations where the division's own sequence bound the pass. Correctly rounded where
+    // nothing leaves the normal range, 2^-900 <= |x| < 2^400 for any div = sqrt(p); other x are divided
+    // (zeros, nearly always: they keep their sign).
     auto quotient = [&](double x, double r) {
+        const unsigned exponent = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+        if (exponent - 123u >= 1300u) return x == 0.0 ? x : x / div;
         const double y = x * r;
         return fma(fma(-y, div, x), r, y);
     };
@@ -976,7 +980,6 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
                 sp.known = slot == 0 && ((known >> sp.q) & 1);
                 // under a branch only some members measure it: what the others hold stays unknown
                 if (slot == 0) known |= 1ull << sp.q;
-                else if (!((known >> sp.q) & 1)) known &= ~(1ull << sp.q);
                 draws += 1 + sp.readout;
                 t->steps.push_back(sp);
                 break;
