@@ -49,6 +49,7 @@ struct Step {
     // MEASURE / RESET
     int q = 0, clbit = -1, readout = 0, is_reset = 0;
     int known = 0;  // the qubit's value was measured and no operator has changed it since
+    int settle = 0;  // complex64, after a known qubit's measurement: weights over the state's squared norm
     double p01 = 0, p10 = 0;
     // KRAUS
     int k = 0, bits[2] = {0, 0}, nkraus = 0;
@@ -107,13 +108,13 @@ __global__ void k_t_advance(int64_t* cursor, const uint64_t* pred, int slot, int
 }
 
 // per-member partial sums of |a|^2 over indices with bit q = 1; partials[b * gridDim.x + block].
-// complex64 reads 16 bytes (two amplitudes) at a time.
+// complex64 reads 16 bytes (two amplitudes) at a time; with `rest` (complex64) the sums over bit q = 0 go there.
 template <typename R>
 __global__ void k_t_p1(const Cx<R>* __restrict__ state, int64_t elems, int q, const uint64_t* pred, int slot,
-                       double* __restrict__ partials) {
+                       double* __restrict__ partials, double* __restrict__ rest) {
     chain_trigger();
     const int64_t b = blockIdx.y;
-    double acc = 0.0;
+    double acc = 0.0, low = 0.0;
     if (has(pred, b, slot)) {
         const Cx<R>* s = state + b * elems;
         const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -122,6 +123,7 @@ __global__ void k_t_p1(const Cx<R>* __restrict__ state, int64_t elems, int q, co
                 for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < (elems >> 1); j += stride) {
                     const float4 w = *reinterpret_cast<const float4*>(s + 2 * j);
                     acc += nrm2(Cx<R>(w.z, w.w));
+                    if (rest) low += nrm2(Cx<R>(w.x, w.y));
                 }
             } else {  // two consecutive amplitudes with bit q set per load
                 for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < (elems >> 2); j += stride) {
@@ -129,6 +131,9 @@ __global__ void k_t_p1(const Cx<R>* __restrict__ state, int64_t elems, int q, co
                     const uint64_t idx = ((i >> q) << (q + 1)) | (1ull << q) | (i & ((1ull << q) - 1));
                     const float4 w = *reinterpret_cast<const float4*>(s + idx);
                     acc += nrm2(Cx<R>(w.x, w.y)) + nrm2(Cx<R>(w.z, w.w));
+                    if (!rest) continue;
+                    const float4 v = *reinterpret_cast<const float4*>(s + (idx ^ (1ull << q)));
+                    low += nrm2(Cx<R>(v.x, v.y)) + nrm2(Cx<R>(v.z, v.w));
                 }
             }
         } else {
@@ -142,6 +147,10 @@ __global__ void k_t_p1(const Cx<R>* __restrict__ state, int64_t elems, int q, co
     }
     const double tot = t_block_sum(acc);
     if (threadIdx.x == 0) partials[b * gridDim.x + blockIdx.x] = tot;
+    if (rest) {
+        const double other = t_block_sum(low);
+        if (threadIdx.x == 0) rest[b * gridDim.x + blockIdx.x] = other;
+    }
 }
 
 // Record a drawn outcome: the readout flip (the member's next uniform), the classical bit.
@@ -165,8 +174,8 @@ __device__ __forceinline__ void set_last(uint64_t* last, int q, int v) {
 }
 
 // one warp per member: sum the partials, draw the outcome (and the readout flip), record the classical
-// bit and the qubit's value
-__global__ void k_t_decide(const double* partials, int nparts, int64_t* cursor, const double* __restrict__ u,
+// bit and the qubit's value. With `rest` (k_t_p1) the probabilities are of the state's squared norm.
+__global__ void k_t_decide(const double* partials, const double* rest, int nparts, int64_t* cursor, const double* __restrict__ u,
                            int64_t ustride, const uint64_t* pred, int slot, int q, int clbit, int readout, double p01,
                            double p10, int is_reset, uint64_t* clbits, int words, uint64_t* last, int* outcome,
                            double* prob, unsigned long long* near, int64_t batch) {
@@ -179,11 +188,19 @@ __global__ void k_t_decide(const double* partials, int nparts, int64_t* cursor, 
             if (lane == 0) outcome[b] = -1;
             continue;
         }
-        double p1 = 0.0;
-        for (int g = lane; g < nparts; g += 32) p1 += partials[b * nparts + g];
+        double p1 = 0.0, p0 = 0.0;
+        for (int g = lane; g < nparts; g += 32) {
+            p1 += partials[b * nparts + g];
+            if (rest) p0 += rest[b * nparts + g];
+        }
 #pragma unroll
-        for (int off = 16; off; off >>= 1) p1 += __shfl_down_sync(~0u, p1, off);
+        for (int off = 16; off; off >>= 1) {
+            p1 += __shfl_down_sync(~0u, p1, off);
+            p0 += __shfl_down_sync(~0u, p0, off);
+        }
         if (lane) continue;
+        const double kept[2] = {p0, p1};
+        if (rest && p0 + p1 > 0.0) p1 /= p0 + p1;
         p1 = fmin(fmax(p1, 0.0), 1.0);
         int64_t cur = cursor[b];
         const double r = u[b * ustride + cur];
@@ -191,7 +208,7 @@ __global__ void k_t_decide(const double* partials, int nparts, int64_t* cursor, 
         if (fabs(r - p1) < kNear) atomicAdd(near, 1ull);
         const int out = r < p1 ? 1 : 0;
         outcome[b] = out;
-        prob[b] = out ? p1 : 1.0 - p1;
+        prob[b] = rest ? kept[out] : out ? p1 : 1.0 - p1;
         if (!is_reset) record_outcome(out, clbit, readout, p01, p10, &cur, u + b * ustride, clbits + b * words);
         set_last(last + b, q, is_reset ? 0 : out);
         cursor[b] = cur;
@@ -553,7 +570,7 @@ template <typename R>
 __global__ void k_t_kraus_decide(const double* partials, int nparts, int k, const double* __restrict__ kraus,
                                  int nkraus, int64_t* cursor, const double* __restrict__ u, int64_t ustride,
                                  const uint64_t* pred, int slot, Cx<R>* dyn, int* apply, unsigned long long* near,
-                                 int64_t batch) {
+                                 int64_t batch, int settle) {
     chain_trigger();
     chain_wait();
     const int d = 1 << k;
@@ -566,8 +583,13 @@ __global__ void k_t_kraus_decide(const double* partials, int nparts, int k, cons
             for (int g = 0; g < nparts; ++g) s += partials[(b * nparts + g) * 2 * d * d + i];
             rho[i] = s;
         }
-        const double r = u[b * ustride + cursor[b]];
+        double r = u[b * ustride + cursor[b]];
         cursor[b] += 1;
+        if (settle) {  // the weights' sum is the state's squared norm
+            double trace = 0.0;
+            for (int i = 0; i < d; ++i) trace += rho[2 * (i * d + i)];
+            r *= trace;
+        }
         double acc = 0.0, w = 0.0;
         int pick = -1;
         for (int i = 0; i < nkraus; ++i) {
@@ -811,14 +833,15 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                     si += glen - 1;
                     break;
                 }
+                double* const rest = sp.settle ? part + B * (int64_t)gx : nullptr;
                 if (!p1_ready)
-                    k_t_p1<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.q, c.pred, sp.slot, part);
-                launch_chained(true, k_t_decide, t_grid(B * 32), kT, 0, st, part, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.q, sp.clbit,
+                    k_t_p1<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.q, c.pred, sp.slot, part, rest);
+                launch_chained(true, k_t_decide, t_grid(B * 32), kT, 0, st, part, rest, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.q, sp.clbit,
                                                          sp.readout, sp.p01, sp.p10, sp.is_reset, c.clbits, t->words, c.last,
                                                          c.outcome, c.prob, c.near, B);
                 // a measurement right after this one: its p(1) partials come out of this collapse
                 const Step* nx = si + 1 < t->steps.size() ? &t->steps[si + 1] : nullptr;
-                const bool fuse = nx && nx->kind == STEP_MEASURE && !nx->known && (B == 1 || group_length(t->steps, si + 1) == 1);
+                const bool fuse = nx && nx->kind == STEP_MEASURE && !nx->known && !nx->settle && (B == 1 || group_length(t->steps, si + 1) == 1);
                 k_t_collapse<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.q, c.outcome, c.prob, sp.is_reset,
                                                                     fuse ? nx->q : -1, c.pred, fuse ? nx->slot : 0, part);
                 next_p1_ready = fuse;
@@ -832,7 +855,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                                                                sp.slot, part);
                 launch_chained(true, k_t_kraus_decide<R>, t_grid(B), kT, 0, st, part, (int)gk, sp.k, (const double*)t->kraus.ptr + 2 * sp.kraus_at,
                                                              sp.nkraus, c.cursor, u, ustride, c.pred, sp.slot,
-                                                             (Cx<R>*)t->dyn.ptr, c.apply, c.near, B);
+                                                             (Cx<R>*)t->dyn.ptr, c.apply, c.near, B, sp.settle);
                 k_t_apply_dyn<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.k, sp.bits[0], sp.bits[1],
                                                                      (const Cx<R>*)t->dyn.ptr, c.apply);
                 break;
@@ -895,6 +918,9 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
     // measurement or reset makes one known, an operator that is not diagonal (or a channel) on it,
     // on any branch, ends that
     uint64_t known = nbits >= 64 ? ~0ull : (1ull << nbits) - 1;
+    // A known qubit's measurement sums no norm and so takes out no drift of FP32 rounding: what draws
+    // next does.
+    bool settle = false;
     auto fail_out = [&](int code) {
         delete t;
         return code;
@@ -978,6 +1004,8 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
                 sp.p01 = op.p01;
                 sp.p10 = op.p10;
                 sp.known = slot == 0 && ((known >> sp.q) & 1);
+                sp.settle = settle && !sp.known;
+                settle = sp.known ? t->precision == LSG_C64 : settle && slot != 0;
                 // under a branch only some members measure it: what the others hold stays unknown
                 if (slot == 0) known |= 1ull << sp.q;
                 draws += 1 + sp.readout;
@@ -994,6 +1022,8 @@ int lsg_traj_create(lsg_state shape, const lsg_traj_op* ops, int32_t nops, const
                 }
                 sp.kind = STEP_KRAUS;
                 sp.k = op.nq;
+                sp.settle = settle;
+                settle = settle && slot != 0;
                 sp.bits[0] = op.qubits[0];
                 sp.bits[1] = op.nq > 1 ? op.qubits[1] : 0;
                 sp.nkraus = op.count;
