@@ -1044,7 +1044,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     const bool transfer = precision == LSG_R64 && !pred && !draw && !count && !(fuse_env && fuse_env[0] == '0');
     if (transfer && nops > 0) {
         grown.assign(pool, pool + 2 * pool_entries);
-        move_outer_rotations(p->plan, batch, grown, p->form.back());
+        move_outer_rotations(p->plan, batch, grown, grown_low, p->form.back());
         pool = grown.data();
         pool_entries = (int64_t)grown.size() / 2;
     }
@@ -1144,7 +1144,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
             }
             std::vector<TransferItem> shears;
             int64_t shear_members = 1;
-            if (transfer && lower_transfer_block(p->plan, pd, blk, batch, pool, p->form[bi], &shears, &shear_members)) {
+            if (transfer && lower_transfer_block(p->plan, pd, blk, batch, Pool{pool, grown_low.data(), own}, p->form[bi], &shears, &shear_members)) {
                 std::vector<TileOp> made;
                 for (const TransferItem& it : shears) {
                     if (it.op >= 0) {

@@ -9,10 +9,13 @@
 // into a diagonal of the block, there already for the two-qubit gate's noise. That is 6
 // multiply-adds and the shift. A gate and phase-covariant noise on a qubit that controls the next cx
 // needs no S: its rotation about Z commutes with all that and is multiplied into the qubit's next
-// operator, in FP64 on the host: 4 and the shift. Measured (12 qubits, 12 layers of noisy u3 and cx, 64
+// operator, on the host: 4 and the shift. Measured (12 qubits, 12 layers of noisy u3 and cx, 64
 // noise models): 426 -> 286 multiply-adds a coefficient, 610 -> 416 ms, FP64 units 90% busy before
-// and after; 9 qubits, 20 layers, 8 models, interpreted passes: 3.25 -> 2.28 ms. Against complex128
-// matrices the largest error of a probability was 6.1e-15 and is 6.3e-15.
+// and after; 9 qubits, 20 layers, 8 models, interpreted passes: 3.25 -> 2.28 ms.
+//
+// A coefficient's error is common to all it multiplies, so each is formed as a pair of doubles and
+// rounded once. Measured, 6 qubits x 20 layers, 12 models, against the operators as given in 80 bits:
+// 6.0e-16 for the dense products, 1.14e-15 with coefficients formed in double precision, 6.9e-16 now.
 //
 // Decided per member from its own data or from the operators' structure, so a member of a batch gets
 // the arithmetic it would get by itself. A member whose operator does not factor well (a reset, full
@@ -22,6 +25,7 @@
 
 #include "../../include/lsg.h"
 #include "transfer.cuh"
+#include "two.cuh"
 
 namespace lsg {
 
@@ -35,21 +39,25 @@ constexpr double kSteep = 64.0;
 enum { Z = 1, X = 2, Y = 3 };
 
 struct Mat4 {
-    double a[4][4];
+    Two a[4][4];
 };
 struct Pair {  // rows (a, b), (c, d)
-    double a, b, c, d;
+    Two a, b, c, d;
 };
 
 bool is_transfer(const TileOp& t) { return t.tmpl >= kT_TPD2 && t.tmpl < kT_TPD2 + 16; }
 bool is_rename(int code) { return code >= kT_X1 && code < kT_SWAP + 16; }
 bool is_diagonal(const TileOp& t) { return t.tmpl == kT_DIAG || t.tmpl == kT_SCALE; }
 
-Mat4 matrix_of(const TileOp& t, const double* pool, int64_t b) {
-    const double* p = pool + 2 * (t.data + (t.stride ? b * t.stride : 0));
+// (entries that move_outer_rotations appended have their rounding errors in `low`)
+Mat4 matrix_of(const TileOp& t, const Pool& pool, int64_t b) {
+    const int64_t at = 2 * (t.data + (t.stride ? b * t.stride : 0));
     Mat4 m;
     for (int r = 0; r < 4; ++r)
-        for (int c = 0; c < 4; ++c) m.a[r][c] = p[2 * (4 * r + c)];
+        for (int c = 0; c < 4; ++c) {
+            const int64_t i = at + 2 * (4 * r + c);
+            m.a[r][c] = Two(pool.data[i], i < pool.own ? 0.0 : pool.low[i - pool.own]);
+        }
     return m;
 }
 
@@ -57,8 +65,8 @@ Mat4 mul(const Mat4& x, const Mat4& y) {
     Mat4 m;
     for (int r = 0; r < 4; ++r)
         for (int c = 0; c < 4; ++c) {
-            double s = 0.0;
-            for (int k = 0; k < 4; ++k) s = std::fma(x.a[r][k], y.a[k][c], s);
+            Two s = x.a[r][0] * y.a[0][c];
+            for (int k = 1; k < 4; ++k) s = s + x.a[r][k] * y.a[k][c];
             m.a[r][c] = s;
         }
     return m;
@@ -67,52 +75,52 @@ Mat4 mul(const Mat4& x, const Mat4& y) {
 double largest(const Mat4& m) {
     double big = 0.0;
     for (int r = 1; r < 4; ++r)
-        for (int c = 1; c < 4; ++c) big = std::max(big, std::fabs(m.a[r][c]));
+        for (int c = 1; c < 4; ++c) big = std::max(big, std::fabs(m.a[r][c].v));
     return big;
 }
 
 // The inverse of S on rows (X, Y): its second row leaves Y without Z, its first row leaves X parallel to
 // Z in the columns (X, Y). Rows of unit length. False when they are not defined well.
 bool outer_inverse(const Mat4& m, double big, Pair* out) {
-    const double xz = m.a[X][Z], yz = m.a[Y][Z], h = std::hypot(xz, yz);
-    const double ca = m.a[X][X] * m.a[Z][Y] - m.a[X][Y] * m.a[Z][X];
-    const double cb = m.a[Y][X] * m.a[Z][Y] - m.a[Y][Y] * m.a[Z][X];
-    const double g = std::hypot(ca, cb);
-    if (!(h > 1e-6 * big) || !(g > 1e-6 * big * big)) return false;
-    Pair s{cb / g, -ca / g, -yz / h, xz / h};
-    if (s.a < 0.0) s.a = -s.a, s.b = -s.b;
-    if (s.d < 0.0) s.c = -s.c, s.d = -s.d;
+    const Two xz = m.a[X][Z], yz = m.a[Y][Z], h = root(xz * xz + yz * yz);
+    const Two ca = m.a[X][X] * m.a[Z][Y] - m.a[X][Y] * m.a[Z][X];
+    const Two cb = m.a[Y][X] * m.a[Z][Y] - m.a[Y][Y] * m.a[Z][X];
+    const Two g = root(ca * ca + cb * cb);
+    if (!(h.v > 1e-6 * big) || !(g.v > 1e-6 * big * big)) return false;
+    Pair s{tidy(cb / g), tidy(-ca / g), tidy(-yz / h), tidy(xz / h)};
+    if (s.a.v < 0.0) s.a = -s.a, s.b = -s.b;
+    if (s.d.v < 0.0) s.c = -s.c, s.d = -s.d;
     // a rotation to rounding is one (with a quarter turn, either sign of its zero cosine is)
-    if (std::fabs(s.b - s.c) <= kZero && std::fabs(s.a) <= kZero && std::fabs(s.d) <= kZero) s.b = -s.b;
-    if (std::fabs(s.a - s.d) <= 4.0 * kZero && std::fabs(s.b + s.c) <= 4.0 * kZero) s.a = s.d, s.b = -s.c;
-    if (std::fabs(s.b) <= kZero && std::fabs(s.c) <= kZero) s = Pair{1.0, 0.0, 0.0, 1.0};
+    if (std::fabs(s.b.v - s.c.v) <= kZero && std::fabs(s.a.v) <= kZero && std::fabs(s.d.v) <= kZero) s.b = -s.b;
+    if (std::fabs(s.a.v - s.d.v) <= 4.0 * kZero && std::fabs(s.b.v + s.c.v) <= 4.0 * kZero) s.a = s.d, s.b = -s.c;
+    if (std::fabs(s.b.v) <= kZero && std::fabs(s.c.v) <= kZero) s = Pair{1.0, 0.0, 0.0, 1.0};
     *out = s;
     return true;
 }
-bool is_rotation(const Pair& s) { return s.a == s.d && s.b == -s.c; }
+bool is_rotation(const Pair& s) { return s.a.v == s.d.v && s.b.v == -s.c.v; }
 
 // f = [[1, p], [q, 1]] * diag(x, y), the pair exchanged between them when `flip`; or, from the left,
 // diag(x, y) * [[1, p], [q, 1]] after the exchange.
 struct Shears {
-    double p = 0.0, q = 0.0, x = 1.0, y = 1.0;
+    Two p, q, x = 1.0, y = 1.0;
     bool flip = false, ok = true;
 };
 Shears shears(Pair f, bool left) {
     Shears s;
-    s.flip = std::fabs(f.a * f.d) < std::fabs(f.b * f.c);
+    s.flip = std::fabs(f.a.v * f.d.v) < std::fabs(f.b.v * f.c.v);
     if (s.flip) f = Pair{f.b, f.a, f.d, f.c};
-    s.p = f.b / (left ? f.a : f.d);
-    s.q = f.c / (left ? f.d : f.a);
+    s.p = tidy(f.b / (left ? f.a : f.d));
+    s.q = tidy(f.c / (left ? f.d : f.a));
     s.x = s.flip && !left ? f.d : f.a;
     s.y = s.flip && !left ? f.a : f.d;
-    s.ok = std::fabs(s.p) <= kSteep && std::fabs(s.q) <= kSteep && s.x != 0.0 && s.y != 0.0;
+    s.ok = std::fabs(s.p.v) <= kSteep && std::fabs(s.q.v) <= kSteep && s.x.v != 0.0 && s.y.v != 0.0;
     return s;
 }
 
 struct Factors {
     int parts = 0;
     double v[2] = {0, 0}, w[2] = {0, 0}, s[2] = {0, 0}, shift[3] = {0, 0, 0};  // shift: Z, X, Y
-    double scale[4] = {1.0, 1.0, 1.0, 1.0};                                    // by row of the 4x4 operator
+    Two scale[4] = {1.0, 1.0, 1.0, 1.0};                                       // by row of the 4x4 operator
 };
 
 // m as shears with its scales before them (or, `left`, after them). Parts kTrDense when it does not
@@ -126,29 +134,30 @@ Factors factor(const Mat4& m, bool left) {
     };
     const double big = largest(m);
     if (!(big > 0.0) || !std::isfinite(big)) return dense();
-    Pair si{1, 0, 0, 1}, v{m.a[X][X], m.a[X][Y], m.a[Y][X], m.a[Y][Y]}, w{1, 0, 0, m.a[Z][Z]};
-    const double coupled = std::max({std::fabs(m.a[X][Z]), std::fabs(m.a[Y][Z]), std::fabs(m.a[Z][X]), std::fabs(m.a[Z][Y])});
+    Pair si{1.0, 0.0, 0.0, 1.0}, v{m.a[X][X], m.a[X][Y], m.a[Y][X], m.a[Y][Y]}, w{1.0, 0.0, 0.0, m.a[Z][Z]};
+    const double coupled = std::max({std::fabs(m.a[X][Z].v), std::fabs(m.a[Y][Z].v), std::fabs(m.a[Z][X].v), std::fabs(m.a[Z][Y].v)});
     if (coupled > kZero * big) {
         if (!outer_inverse(m, big, &si)) return dense();
-        double n[4][4];
+        Two n[4][4];
         for (int c = Z; c <= Y; ++c) {
-            n[X][c] = std::fma(si.a, m.a[X][c], si.b * m.a[Y][c]);
-            n[Y][c] = std::fma(si.c, m.a[X][c], si.d * m.a[Y][c]);
+            n[X][c] = si.a * m.a[X][c] + si.b * m.a[Y][c];
+            n[Y][c] = si.c * m.a[X][c] + si.d * m.a[Y][c];
             n[Z][c] = m.a[Z][c];
         }
-        const int from = std::hypot(n[X][X], n[X][Y]) >= std::hypot(n[Z][X], n[Z][Y]) ? X : Z;
-        const double h = std::hypot(n[from][X], n[from][Y]), ux = n[from][X] / h, uy = n[from][Y] / h;
+        const Two nx = n[X][X] * n[X][X] + n[X][Y] * n[X][Y], nz = n[Z][X] * n[Z][X] + n[Z][Y] * n[Z][Y];
+        const int from = nx.v >= nz.v ? X : Z;
+        const Two h = root(from == X ? nx : nz), ux = n[from][X] / h, uy = n[from][Y] / h;
         v = Pair{ux, uy, n[Y][X], n[Y][Y]};
-        w = Pair{std::fma(n[X][X], ux, n[X][Y] * uy), n[X][Z], std::fma(n[Z][X], ux, n[Z][Y] * uy), n[Z][Z]};
+        w = Pair{n[X][X] * ux + n[X][Y] * uy, n[X][Z], n[Z][X] * ux + n[Z][Y] * uy, n[Z][Z]};
     }
-    const double det = si.a * si.d - si.b * si.c;
-    if (!(std::fabs(det) > 1.0 / kSteep)) return dense();
+    const Two det = si.a * si.d - si.b * si.c;
+    if (!(std::fabs(det.v) > 1.0 / kSteep)) return dense();
     const Pair s{si.d / det, -si.b / det, -si.c / det, si.a / det};
     {  // the product stands for m to rounding
-        const double wv[4][4] = {{0, 0, 0, 0}, {0, w.d, w.c * v.a, w.c * v.b}, {0, w.b, w.a * v.a, w.a * v.b}, {0, 0, v.c, v.d}};
+        const Two wv[4][4] = {{}, {Two(), w.d, w.c * v.a, w.c * v.b}, {Two(), w.b, w.a * v.a, w.a * v.b}, {Two(), Two(), v.c, v.d}};
         for (int c = Z; c <= Y; ++c) {
-            const double x = s.a * wv[X][c] + s.b * wv[Y][c], y = s.c * wv[X][c] + s.d * wv[Y][c];
-            const double off = std::max({std::fabs(x - m.a[X][c]), std::fabs(y - m.a[Y][c]), std::fabs(wv[Z][c] - m.a[Z][c])});
+            const Two x = s.a * wv[X][c] + s.b * wv[Y][c], y = s.c * wv[X][c] + s.d * wv[Y][c];
+            const double off = std::max({std::fabs(x.v - m.a[X][c].v), std::fabs(y.v - m.a[Y][c].v), std::fabs(wv[Z][c].v - m.a[Z][c].v)});
             if (!(off <= 4.0 * kZero * big)) return dense();
         }
     }
@@ -166,18 +175,18 @@ Factors factor(const Mat4& m, bool left) {
     }
     if (!a.ok || !b.ok || !e.ok) return dense();
     auto part = [&](const Shears& h, int bit, int flip, double* to) {
-        to[0] = h.p, to[1] = h.q;
-        if (h.flip || h.p != 0.0 || h.q != 0.0) f.parts |= bit | (h.flip ? flip : 0);
+        to[0] = h.p.value(), to[1] = h.q.value();
+        if (h.flip || to[0] != 0.0 || to[1] != 0.0) f.parts |= bit | (h.flip ? flip : 0);
     };
     part(a, kTrV, kTrFlipV, f.v);
     part(b, kTrW, kTrFlipW, f.w);
     part(e, kTrS, kTrFlipS, f.s);
     for (int r = Z; r <= Y; ++r) {
-        f.shift[r - 1] = left ? m.a[r][0] / f.scale[r] : m.a[r][0];
-        if (m.a[r][0] != 0.0) f.parts |= r == Z ? kTrShiftZ : kTrShiftXY;
+        f.shift[r - 1] = (left ? m.a[r][0] / f.scale[r] : m.a[r][0]).value();
+        if (m.a[r][0].value() != 0.0) f.parts |= r == Z ? kTrShiftZ : kTrShiftXY;
     }
     for (int r = Z; r <= Y; ++r)
-        if (!std::isfinite(f.scale[r]) || !std::isfinite(f.shift[r - 1])) return dense();
+        if (!std::isfinite(f.scale[r].v) || !std::isfinite(f.shift[r - 1])) return dense();
     return f;
 }
 
@@ -211,19 +220,21 @@ unsigned positions(const TileOp& t) {
     return bits;
 }
 
-void permute(std::vector<double>& v, int64_t members, int U, int code) {
+template <typename T>
+void permute(std::vector<T>& v, int64_t members, int U, int code) {
     const int D = 1 << U;
-    std::vector<double> w(v.size());
+    std::vector<T> w(v.size());
     for (int64_t b = 0; b < members; ++b)
         for (int e = 0; e < D; ++e) w[(size_t)(b * D + e)] = v[(size_t)(b * D + rename_source(code, U, e))];
     v.swap(w);
 }
 
-void times_diagonal(std::vector<double>& v, int64_t members, int U, const TileOp& t, const double* pool) {
+template <typename T>
+void times_diagonal(std::vector<T>& v, int64_t members, int U, const TileOp& t, const double* pool) {
     const int D = 1 << U;
     for (int64_t b = 0; b < members; ++b) {
         const double* p = pool + 2 * (t.data + (t.stride ? b * t.stride : 0));
-        for (int e = 0; e < D; ++e) v[(size_t)(b * D + e)] *= p[2 * diag_entry(t, U, e)];
+        for (int e = 0; e < D; ++e) v[(size_t)(b * D + e)] = v[(size_t)(b * D + e)] * T(p[2 * diag_entry(t, U, e)]);
     }
 }
 
@@ -253,7 +264,8 @@ int passes(const Composite& c, int64_t b, int U, int P0, int P1) {
 
 }  // namespace
 
-void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, Choices& form) {
+void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, std::vector<double>& low, Choices& form) {
+    const int64_t own = (int64_t)pool.size();
     struct Touch {
         int op, pass, block;
     };
@@ -316,22 +328,23 @@ void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, 
             std::vector<Mat4> mine, next;
             bool any = false;
             for (int64_t b = 0; b < members; ++b) {
-                Mat4 m = matrix_of(t, pool.data(), b), x = matrix_of(n, pool.data(), b);
+                const Pool now{pool.data(), low.data(), own};
+                Mat4 m = matrix_of(t, now, b), x = matrix_of(n, now, b);
                 Pair s;
                 const int way = passes(c, b, U, n.pos[0], n.pos[1]);
-                if (way && outer_inverse(m, largest(m), &s) && is_rotation(s) && s.c != 0.0) {
+                if (way && outer_inverse(m, largest(m), &s) && is_rotation(s) && s.c.v != 0.0) {
                     any = true;
-                    const double k = s.a * s.a + s.b * s.b;
+                    const Two k = s.a * s.a + s.b * s.b;
                     Mat4 in = m, turned = x;
                     for (int q = 0; q < 4; ++q) {
-                        in.a[X][q] = std::fma(s.a, m.a[X][q], s.b * m.a[Y][q]);
-                        in.a[Y][q] = q == Z ? 0.0 : std::fma(s.c, m.a[X][q], s.d * m.a[Y][q]);
+                        in.a[X][q] = s.a * m.a[X][q] + s.b * m.a[Y][q];
+                        in.a[Y][q] = q == Z ? Two() : s.c * m.a[X][q] + s.d * m.a[Y][q];
                     }
                     // the rotation taken out, [[a, -b], [b, a]] / k by rows, or the other way round
-                    const double ga = s.a / k, gb = (way > 0 ? s.b : -s.b) / k;
+                    const Two ga = s.a / k, gb = (way > 0 ? s.b : -s.b) / k;
                     for (int q = 1; q < 4; ++q) {
-                        turned.a[q][X] = std::fma(x.a[q][X], ga, x.a[q][Y] * gb);
-                        turned.a[q][Y] = std::fma(x.a[q][Y], ga, -x.a[q][X] * gb);
+                        turned.a[q][X] = x.a[q][X] * ga + x.a[q][Y] * gb;
+                        turned.a[q][Y] = x.a[q][Y] * ga - x.a[q][X] * gb;
                     }
                     m = in, x = turned;
                 }
@@ -345,10 +358,12 @@ void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, 
                 int entries = 0;
                 for (const Mat4& m : ms)
                     for (int e = 0; e < 16; ++e) {
-                        const double y = m.a[e / 4][e % 4];
-                        if (e >= 4 && y != 0.0) entries |= 1 << (e - 4);
-                        pool.push_back(y);
+                        const Two y = tidy(m.a[e / 4][e % 4]);
+                        if (e >= 4 && y.v != 0.0) entries |= 1 << (e - 4);
+                        pool.push_back(y.v);
                         pool.push_back(0.0);
+                        low.push_back(y.e);
+                        low.push_back(0.0);
                     }
                 op.zmask = ~form.at_least(entries) & ((1 << 12) - 1);
             };
@@ -357,7 +372,7 @@ void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, 
         }
 }
 
-bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, int64_t batch, const double* pool,
+bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, int64_t batch, const Pool& pool,
                           Choices& form, std::vector<TransferItem>* items, int64_t* members_out) {
     const int U = blk.u, D = 1 << U;
     const int first = pd.first_op + blk.first, last = first + blk.nops;
@@ -372,15 +387,15 @@ bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc&
     *members_out = members;
     const double overhead = 0.05;  // multiply-adds per coefficient, for an operator's own instructions
     double before = 0.0, after = 0.0;
-    std::vector<double> pend((size_t)(members * D), 1.0);  // the diagonal not yet emitted
+    std::vector<Two> pend((size_t)(members * D), 1.0);  // the diagonal not yet emitted
+    std::vector<std::vector<Two>> diagonals;            // the emitted ones, rounded at the end
     unsigned dep = 0, touched = 0;                         // its positions; those changed since the last one emitted
     int open = -1;
     auto emit = [&] {
-        TransferItem it;
-        it.v = pend;
         open = (int)items->size();
-        items->push_back(std::move(it));
-        std::fill(pend.begin(), pend.end(), 1.0);
+        items->push_back(TransferItem());
+        diagonals.push_back(pend);
+        std::fill(pend.begin(), pend.end(), Two(1.0));
         dep = touched = 0;
         after += 1.0 + overhead;
     };
@@ -390,7 +405,7 @@ bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc&
         const unsigned bits = positions(t);
         if (done[(size_t)(o - first)]) continue;
         if (is_diagonal(t)) {
-            times_diagonal(pend, members, U, t, pool);
+            times_diagonal(pend, members, U, t, pool.data);
             dep |= bits | (1u << 8);  // (a factor depends on no position, and is still to be applied)
             before += 1.0 + overhead;
             continue;
@@ -427,14 +442,17 @@ bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc&
         it.pos[0] = t.pos[0], it.pos[1] = t.pos[1];
         it.mask = 0;
         const int B0 = 1 << (U - 1 - t.pos[0]), B1 = 1 << (U - 1 - t.pos[1]);
-        std::vector<double>& scales = left ? pend : (*items)[(size_t)open].v;
+        std::vector<Two>& scales = left ? pend : diagonals.back();
         for (int64_t b = 0; b < members; ++b) {
             const Factors f = factor(m[(size_t)b], left);
             it.mask |= f.parts;
             it.v.insert(it.v.end(), {(double)f.parts, 0.0, f.v[0], f.v[1], f.w[0], f.w[1], f.s[0], f.s[1], f.shift[0], f.shift[1]});
-            for (int e = 4; e < 16; ++e) it.v.push_back(f.parts & kTrDense ? m[(size_t)b].a[e / 4][e % 4] : 0.0);
+            for (int e = 4; e < 16; ++e) it.v.push_back(f.parts & kTrDense ? m[(size_t)b].a[e / 4][e % 4].value() : 0.0);
             it.v[it.v.size() - 21] = f.shift[2];
-            for (int e = 0; e < D; ++e) scales[(size_t)(b * D + e)] *= f.scale[(e & B0 ? 2 : 0) + (e & B1 ? 1 : 0)];
+            for (int e = 0; e < D; ++e) {
+                Two& x = scales[(size_t)(b * D + e)];
+                x = x * f.scale[(e & B0 ? 2 : 0) + (e & B1 ? 1 : 0)];
+            }
         }
         it.mask = form.at_least(it.mask);
         items->push_back(std::move(it));
@@ -443,6 +461,12 @@ bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc&
         after += 1.75 + overhead;
     }
     if (dep) emit();
+    size_t n = 0;
+    for (TransferItem& it : *items)
+        if (it.op < 0 && it.mask < 0) {
+            for (const Two& x : diagonals[n]) it.v.push_back(x.value());
+            ++n;
+        }
     return after < before && (int)items->size() <= blk.nops;
 }
 

@@ -6,14 +6,16 @@
 #include <cstdint>
 #include <vector>
 
+#include "lower.cuh"
 #include "program.cuh"
 
 namespace lsg {
 
 // Move the outer rotation of the last two coefficients of every such operator (a rotation about Z, with
 // the digits in the order I, Z, X, Y) through the renames and diagonals that let it pass into the next
-// one on the same register bits. The operators then read entries appended to `pool`.
-void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, Choices& form);
+// one on the same register bits. The operators then read entries appended to `pool` (and `low`, as
+// move_outer_factors).
+void move_outer_rotations(Plan& plan, int64_t batch, std::vector<double>& pool, std::vector<double>& low, Choices& form);
 
 struct TransferItem {
     int op = -1;     // an operator kept as it is: its index in plan.ops; -1: made here
@@ -27,7 +29,7 @@ struct TransferItem {
 constexpr int kTransferLen = 22;
 
 // False when the block would not take fewer operations. members: 1 when all data are shared.
-bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, int64_t batch, const double* pool,
+bool lower_transfer_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, int64_t batch, const Pool& pool,
                           Choices& form, std::vector<TransferItem>* items, int64_t* members);
 
 }  // namespace lsg
