@@ -818,32 +818,33 @@ static int block_layout(const PassDesc& pd, BlockDesc& b, const TileOp* ops, siz
     // lanes: bits of the group index in order; the first ones reach different banks of a phase
     int access = 0;
     while ((1 << access) < (int)(b.lvec * (int)eb)) ++access;
-    std::vector<int> rest, order;
+    // (fixed lists: this runs for every block of every new set of a template's values)
+    int rest[32], order[32], nrest = 0, norder = 0;
     for (int t = 0; t < K; ++t)
-        if (std::find(b.bits, b.bits + U, t) == b.bits + U) rest.push_back(t);
-    std::vector<uint32_t> span;  // reduced projections chosen so far
-    for (int t : rest) {
-        if ((int)span.size() == 7 - access) break;
-        uint32_t v = (bytes(1u << t) & 127u) >> access;
-        for (uint32_t s : span) v = std::min(v, v ^ s);
+        if (std::find(b.bits, b.bits + U, t) == b.bits + U) rest[nrest++] = t;
+    uint32_t span[8], taken = 0;  // reduced projections chosen so far; their bits
+    for (int i = 0; i < nrest && norder < 7 - access; ++i) {
+        uint32_t v = (bytes(1u << rest[i]) & 127u) >> access;
+        for (int k = 0; k < norder; ++k) v = std::min(v, v ^ span[k]);
         if (!v) continue;
-        span.push_back(v);
-        order.push_back(t);
+        span[norder] = v;
+        order[norder++] = rest[i];
+        taken |= 1u << i;
     }
-    for (int t : rest)
-        if (std::find(order.begin(), order.end(), t) == order.end()) order.push_back(t);
+    for (int i = 0; i < nrest; ++i)
+        if (!((taken >> i) & 1u)) order[norder++] = rest[i];
     std::fill(b.gb, b.gb + 16, (unsigned short)0);
-    if ((int)order.size() > 16) return fail(LSG_E_ARG, "internal planning error: a tile of 2^%d elements", K);
-    for (size_t i = 0; i < order.size(); ++i) b.gb[i] = (unsigned short)bytes(1u << order[i]);
+    if (norder > 16) return fail(LSG_E_ARG, "internal planning error: a tile of 2^%d elements", K);
+    for (int i = 0; i < norder; ++i) b.gb[i] = (unsigned short)bytes(1u << order[i]);
     // the maps reach every element of the tile once: K independent addresses below the tile's size
     for (const unsigned short* ob : {b.lob, b.sob}) {
-        std::vector<uint32_t> basis;
+        uint32_t by_top[32] = {};  // reduced addresses by their highest bit
         for (int i = 0; i < K; ++i) {
             uint32_t v = i < U ? ob[i] : b.gb[i - U];
             if (v >= (uint32_t)(eb << K) || (v & (eb - 1))) return fail(LSG_E_ARG, "internal planning error: block address");
-            for (uint32_t s : basis) v = std::min(v, v ^ s);
+            while (v && by_top[31 - __builtin_clz(v)]) v ^= by_top[31 - __builtin_clz(v)];
             if (!v) return fail(LSG_E_ARG, "internal planning error: block addresses collide");
-            basis.push_back(v);
+            by_top[31 - __builtin_clz(v)] = v;
         }
     }
     return LSG_OK;
