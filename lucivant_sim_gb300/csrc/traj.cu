@@ -145,11 +145,19 @@ __global__ void k_t_p1(const Cx<R>* __restrict__ state, int64_t elems, int q, co
             }
         }
     }
+    __shared__ double lows[kT / 32];  // (per warp, seen by thread 0 behind the other sum's barriers)
+    if (sizeof(R) == 4 && rest) {
+#pragma unroll
+        for (int off = 16; off; off >>= 1) low += __shfl_down_sync(~0u, low, off);
+        if ((threadIdx.x & 31) == 0) lows[threadIdx.x >> 5] = low;
+    }
     const double tot = t_block_sum(acc);
-    if (threadIdx.x == 0) partials[b * gridDim.x + blockIdx.x] = tot;
-    if (rest) {
-        const double other = t_block_sum(low);
-        if (threadIdx.x == 0) rest[b * gridDim.x + blockIdx.x] = other;
+    if (threadIdx.x == 0) {
+        partials[b * gridDim.x + blockIdx.x] = tot;
+        if (sizeof(R) == 4 && rest) {
+            for (int w = 1; w < kT / 32; ++w) low += lows[w];
+            rest[b * gridDim.x + blockIdx.x] = low;
+        }
     }
 }
 
@@ -174,7 +182,9 @@ __device__ __forceinline__ void set_last(uint64_t* last, int q, int v) {
 }
 
 // one warp per member: sum the partials, draw the outcome (and the readout flip), record the classical
-// bit and the qubit's value. With `rest` (k_t_p1) the probabilities are of the state's squared norm.
+// bit and the qubit's value. REST: with k_t_p1's `rest`, the probabilities are of the state's squared norm
+// (a form of its own: with the test in one kernel every measurement took 1 us longer).
+template <bool REST>
 __global__ void k_t_decide(const double* partials, const double* rest, int nparts, int64_t* cursor, const double* __restrict__ u,
                            int64_t ustride, const uint64_t* pred, int slot, int q, int clbit, int readout, double p01,
                            double p10, int is_reset, uint64_t* clbits, int words, uint64_t* last, int* outcome,
@@ -191,24 +201,23 @@ __global__ void k_t_decide(const double* partials, const double* rest, int npart
         double p1 = 0.0, p0 = 0.0;
         for (int g = lane; g < nparts; g += 32) {
             p1 += partials[b * nparts + g];
-            if (rest) p0 += rest[b * nparts + g];
+            if constexpr (REST) p0 += rest[b * nparts + g];
         }
 #pragma unroll
         for (int off = 16; off; off >>= 1) {
             p1 += __shfl_down_sync(~0u, p1, off);
-            p0 += __shfl_down_sync(~0u, p0, off);
+            if constexpr (REST) p0 += __shfl_down_sync(~0u, p0, off);
         }
         if (lane) continue;
-        const double kept[2] = {p0, p1};
-        if (rest && p0 + p1 > 0.0) p1 /= p0 + p1;
-        p1 = fmin(fmax(p1, 0.0), 1.0);
+        if constexpr (!REST) p1 = fmin(fmax(p1, 0.0), 1.0);
         int64_t cur = cursor[b];
-        const double r = u[b * ustride + cur];
+        double r = u[b * ustride + cur];
+        if constexpr (REST) r *= p0 + p1;
         cur += 1;
         if (fabs(r - p1) < kNear) atomicAdd(near, 1ull);
         const int out = r < p1 ? 1 : 0;
         outcome[b] = out;
-        prob[b] = rest ? kept[out] : out ? p1 : 1.0 - p1;
+        prob[b] = out ? p1 : REST ? p0 : 1.0 - p1;
         if (!is_reset) record_outcome(out, clbit, readout, p01, p10, &cur, u + b * ustride, clbits + b * words);
         set_last(last + b, q, is_reset ? 0 : out);
         cursor[b] = cur;
@@ -836,7 +845,7 @@ int run_steps(lsg_traj_s* t, lsg_state_s* s, const Ctl& c, const double* u, int6
                 double* const rest = sp.settle ? part + B * (int64_t)gx : nullptr;
                 if (!p1_ready)
                     k_t_p1<R><<<dim3(gx, (unsigned)B), kT, 0, st>>>(state, elems, sp.q, c.pred, sp.slot, part, rest);
-                launch_chained(true, k_t_decide, t_grid(B * 32), kT, 0, st, part, rest, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.q, sp.clbit,
+                launch_chained(true, rest ? k_t_decide<true> : k_t_decide<false>, t_grid(B * 32), kT, 0, st, part, rest, (int)gx, c.cursor, u, ustride, c.pred, sp.slot, sp.q, sp.clbit,
                                                          sp.readout, sp.p01, sp.p10, sp.is_reset, c.clbits, t->words, c.last,
                                                          c.outcome, c.prob, c.near, B);
                 // a measurement right after this one: its p(1) partials come out of this collapse
