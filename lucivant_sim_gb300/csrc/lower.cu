@@ -97,16 +97,17 @@ bool nearest(const Mat& m, Unitary* out) {
 
 Mat matrix(const Unitary& u) { return Mat{u.a, -(u.w * conj(u.c)), u.c, u.w * conj(u.a)}; }
 
-// The phase ph of u = diag(1, ph) * N with N's first column in a real ratio. Of its two signs the one that
-// leaves N's e (Rotation) the positive real part: a rotation's e is then one for either sign of its
-// cosine and sine, and whether it needs a diagonal does not depend on its angle.
+// The phase ph of u = diag(1, ph) * N with N's first column in a real ratio. Of its two signs, one where it
+// is real (a gate without phases, h), else the one that leaves N's e (Rotation) the positive real part:
+// whether a rotation needs a diagonal then does not depend on the sign of its cosine or sine.
 Cpx outer_phase(const Unitary& u) {
     if (zero(u.a) || zero(u.c)) return 1.0;
     Cpx ph = u.c * conj(u.a);
     ph = ph / root(norm(ph));
+    if (settled(ph).one() || settled(-ph).one()) return 1.0;
     const cd a = u.a.value(), c = u.c.value(), w = u.w.value(), p = ph.value();
     const cd e = std::norm(c) > std::norm(a) ? w * p * std::conj(c * c) : w * std::conj(p * a * a);
-    return settled(e.real() < 0.0 ? -ph : ph);
+    return e.real() < 0.0 ? -ph : ph;
 }
 Unitary without_phase(const Unitary& u, Cpx ph) {
     return ph.one() ? u : Unitary{u.a, u.c * conj(ph), u.w * conj(ph)};
@@ -385,10 +386,13 @@ bool lower_block(const Plan& plan, const PassDesc& pd, const BlockDesc& blk, con
             const int x = bit((code - kT_SWAP) / 4), y = bit((code - kT_SWAP) % 4);
             return ((e & x) != 0) != ((e & y) != 0) ? e ^ x ^ y : e;
         };
-        std::vector<Cpx> v(pend.v.size());
-        for (int64_t b = 0; b < members; ++b)
-            for (int e = 0; e < D; ++e) v[(size_t)(b * D + e)] = pend.v[(size_t)(b * D + src(e))];
-        pend.v.swap(v);
+        if (!pend.dep) return;  // ones
+        Cpx v[16];
+        for (int64_t b = 0; b < members; ++b) {
+            Cpx* now = pend.v.data() + b * D;
+            std::copy(now, now + D, v);
+            for (int e = 0; e < D; ++e) now[e] = v[src(e)];
+        }
     };
 
     for (int o = first; o < last; ++o) {
