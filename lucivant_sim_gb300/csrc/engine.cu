@@ -923,6 +923,15 @@ static bool pass_fits_swizzle(const PassDesc& pd, const Plan& plan, size_t eb, i
     return fits;
 }
 
+// SMs of the current device (a GB300's where there is none: plans made on the host alone).
+static int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
+        return sms;
+    cudaGetLastError();
+    return 152;
+}
+
 // Copy a program's content to device memory of its own.
 static int program_upload(lsg_program_s* p, const std::vector<unsigned char>& content, cudaStream_t stream) {
     LSG_CHECK(ensure(p->dev, content.size()));
@@ -953,7 +962,7 @@ static int program_build(int nbits, int precision, int64_t batch, const lsg_op* 
     const int full_bits = p->K;
     const bool trajectory = pred || draw || count;
     if (trajectory && precision == LSG_C128 && !t_choice.tile_bits && !getenv("LSG_TILE_BITS") && p->K > 10 &&
-        nbits - p->K < 16 && (batch << (nbits - p->K + 1)) <= 152)
+        nbits - p->K < 16 && (batch << (nbits - p->K + 1)) <= sm_count())
         --p->K;
     const int L = std::min(p->K, low_bits_for(nbits, precision));
     if (nops > 0) {
