@@ -39,10 +39,11 @@ using cd = std::complex<double>;
 
 // How far an operator may be from a rotation between phases, relative to its largest entry. Gate
 // matrices are unitary to a few units in the last place, products of n of them to some sqrt(n) times
-// 1e-16: this holds for any run of gates on a qubit, so that whether an operator is lowered depends
-// on what it is and not on a member's rounding (2e-15 left a tenth of the products of 50 gates dense,
-// for every member of the batch). Anything less unitary stays dense.
-constexpr double kUnitary = 1e-13;
+// 1e-16: this holds for runs of some 10,000 gates on a qubit, so that whether an operator is lowered
+// depends on what it is and not on a member's rounding (2e-15 left a tenth of the products of 50 gates
+// dense, for every member of the batch). Anything less unitary, a matrix known to fewer digits among
+// it, stays dense and is applied as given.
+constexpr double kUnitary = 3e-14;
 // A phase this close to one is the rounding of one (gate matrices are products of a few rounded
 // factors): taken as one, so the diagonal that would hold it is left out.
 constexpr double kResidue = 1e-15;
