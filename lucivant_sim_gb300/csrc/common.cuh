@@ -275,7 +275,7 @@ __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.l
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 #ifndef __CUDACC_RTC__
-// The launch. Measured: 40 serial shots of 13 qubits (174 launches each) 29.2 -> 26.3 ms, 17 qubits x 16
+// The launch. Measured: 40 serial shots of 13 qubits (174 launches each) 29.2 -> 26.3 ms, 17 qubits x 8
 // members x 8 passes 249 -> 232 us. Kernels that walk the whole state are launched plainly: started early
 // their blocks crowd the SMs that happen to be free (18 qubits serial 16.0 -> 19.1 ms). So are passes of
 // more than 16 tiles a block (`early` false): a start counts little there, and 512 members of 18 qubits
